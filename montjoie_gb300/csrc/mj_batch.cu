@@ -815,6 +815,8 @@ int mj_op_set_element_scale(mj_op* op, const double* scale) {
                                                                     op->fac_e.as<float>(), op->n_elt_pad, per_elt);
   count_launch();
   MJ_CUDA(cudaGetLastError());
+  if (op->fac_fx.ptr)
+    if (int rc = k1_fixed_factors(op, op->stream)) return rc;
   MJ_CUDA(cudaStreamSynchronize(op->stream));
   op->fac_version++;
   return MJ_OK;

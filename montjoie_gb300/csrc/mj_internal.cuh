@@ -17,11 +17,14 @@ struct mj_op {
   bool warp = false;                    // warp-per-element layout (FP32, order 4; autotuned)
   bool packed = false;                  // that layout with packed connectivity (nodle_pk; autotuned)
   bool fs = false;                      // compact layout with one factor stage (FP32; autotuned)
+  bool fx = false;                      // fixed-point kernel (FP64, mj_k1_fx.cuh)
+  bool fx_sym = false;                  // its form for matrices antisymmetric under the mirror
   size_t r_len = 0;                     // element-major slots (n_elt_pad * Qp)
   size_t n_inc = 0;                     // incidences (n_elt * Q); R has n_inc + 1 entries
   mj::DevBuf nodle_e, fac_e, slot_e, R, ptr;
   mj::DevBuf nodle_pk;                  // packed connectivity: dof | rank << 27 (FP32 order 4), or empty
   mj::DevBuf err;                       // device error flag (bounded-wait timeouts)
+  mj::DevBuf fac_fx, fac_exp;           // FP64: fac_e as scaled limbs and the scale of every element (fixed-point kernel)
   mj::DevBuf fac_orig;                  // factors before mj_op_set_element_scale (kept on first use)
   int fac_version = 0;                  // bumped whenever fac_e changes after creation
   mj::DevBuf verts;                     // n_elt x 8 x 3 vertices (operators built from geometry)
@@ -33,7 +36,7 @@ struct mj_op {
   std::vector<int> tune_E, tune_vec;
   size_t device_bytes() const {
     return nodle_e.bytes + fac_e.bytes + fac_orig.bytes + slot_e.bytes + R.bytes + ptr.bytes + xbuf.bytes +
-           ybuf.bytes + verts.bytes + nodle_pk.bytes;
+           ybuf.bytes + verts.bytes + nodle_pk.bytes + fac_fx.bytes + fac_exp.bytes;
   }
 };
 
@@ -167,6 +170,20 @@ void k1_launch_fs_f32(int n, int E, int grid, const void* x, const int* nodle_e,
 int k1_prepare_w_f32(int n, int E, bool packed, int* ctas_per_sm);
 void k1_launch_w_f32(int n, int E, bool packed, int grid, const void* x, const int* nodle_e, const void* fac_e,
                      void* R, const int* slot_e, int n_tiles, int* err, cudaStream_t s);
+
+// Fixed-point kernel of FP64 operators (mj_k1_fx.cuh), the same tile sizes,
+// in two forms: the derivative matrix exactly antisymmetric under the mirror
+// (_sym, mj_k1_fx.cu) or any (_gen, mj_k1_fxg.cu).  supports: the matrix is
+// within its range; fixed_factors: fac_e into fac_fx / fac_exp (after every
+// change of fac_e).
+bool k1_fx_supports(int n, const double* g, bool* sym);
+int k1_set_gmat_fx(int n, const double* g, bool sym);
+int k1_set_gmat_fx_gen(int n, const double* g);
+int k1_fixed_factors(mj_op* op, cudaStream_t s);
+int k1_prepare_fx(const mj_op* op, int E, int* ctas_per_sm);
+int k1_prepare_fx_gen(int n, int E, int* ctas_per_sm);
+void k1_launch_fx(mj_op* op, const void* x, cudaStream_t s);
+void k1_launch_fx_gen(mj_op* op, const void* x, cudaStream_t s);
 
 // Test instances of two variants compiled with a bulk-copy wait limit of 0
 // (the test hook of mj_debug_set_wait_limits): FP32 one element per warp with

@@ -1,0 +1,584 @@
+// FP64 element kernel in two-limb fixed point: the same element product as
+// k_local_stiffness<double> (mj_k1.cuh), its contractions and factor products
+// carried out with 32 x 32 -> 64 bit integer multiply-adds.
+//
+// Why: a GB300 SM issues 2 FP64 multiply-adds per clock and 32 wide integer
+// ones (IMAD.WIDE; both measured), and one 61 x 62 bit product takes three of
+// the latter and a short one, so products run several times faster in
+// integers.  The FP64 kernel is bound by its FP64 pipe (91% busy).
+//
+// Numbers.  Every quantity of an element is an integer with one power-of-two
+// scale per element, used as two signed 32-bit limbs v = hi 2^32 + lo
+// (|lo| <= 2^31), so that every partial product is a signed 32 x 32 one:
+//   u : scaled by the element's largest |u| to |u| < 2^60
+//   G : the derivative matrix, sums of |G| over a (of the gradient's
+//       coefficients G[a][l] and of the divergence's G'[l][a]) < 2^62
+//   B': the factors, row sums |B'_a.| < 2^62 over the element, converted when
+//       the factors are set (k_fixed_factors)
+//   v : the fluxes, shifted by the element's largest |g| to |v| < 2^60
+// Point (i, j, k) carries the factor 2^(c_i + c_j + c_k), c from fx_c: B' = 2^c B,
+// G'[l][a] = 2^(c_l - c_a) G[l][a], result = 2^-c y.  c roughly undoes the
+// quadrature weights, which fall by up to 2^4 per axis towards the faces and
+// would otherwise leave few bits there.
+// A sum of products keeps hi*hi in one 64-bit accumulator (h) and hi*lo + lo*hi
+// in another (m); lo*lo enters m with its upper bits.  Bounds, n = 9 worst:
+//   g = sum G u     <= 2^61    h < 2^60, m < 2^62.8
+//   v = sum B' g    <= 2^60    h < 2^59, m < 2^62.4
+//   y = 3 sums G' v <= 2^62.6  h < 2^60, m < 2^62.8
+// so no accumulator overflows for any input in range.  Measured against
+// extended precision, the products are closer than the FP64 kernel's for
+// smooth, random and steep fields at every order (1e-17 to 1e-15 relative L2).
+//
+// Measured (us per launch, FP64-pipe kernel at its best tile -> this kernel):
+// Q4 16^3 60 -> 20, 64^3 2300 -> 598; Q8 15x13x11-sized 359 -> 94, 32^3 3150
+// -> 763; Q6 40^3 2575 -> 590; Q1 64^3 94 -> 45.  What bounds it now (ncu, Q4
+// 40^3): the integer multiply pipe (about 60% busy) behind 16 to 20 warps per
+// SM, which shared memory (the factor stage) and registers allow; DRAM is at
+// half of its rate.  Without the lo*lo term it takes 15% less and errs up to
+// 3 times more than the FP64 kernel on steep fields; with the mirror symmetry
+// it takes 25% less than in the general form.
+//
+// A tile with an element out of range (a NaN or infinity in u or B, or scales
+// whose result would leave the normal range) takes the FP64 arithmetic of
+// k_local_stiffness instead (fx_tile_fp64), so such values propagate as there.
+//
+// Layout: E elements per CTA, E*n*n threads.  A thread owns a z-line in the
+// gather, the z-contractions, the factor products and the result, and an
+// x-line and a y-line in the other contractions, whose n results it computes
+// from n values held in registers.  So each value crosses shared memory once
+// per contraction instead of n times, and no matrix entries are kept in
+// registers.  Factors arrive by bulk copy in one stage (free after the factor
+// products, refilled during the divergence), Nodle in two; the next tile's u
+// is gathered during the divergence and its largest exponent found there too.
+//
+// SYM: G is antisymmetric under the mirror (a, l) -> (n-1-a, n-1-l), as the
+// Gauss-Lobatto matrix is.  Then with e_a = r_a + r_(n-1-a), o_a = r_a - r_(n-1-a)
+//   y_l = Q_l + P_l, y_(n-1-l) = Q_l - P_l,  P_l = sum Me e_a, Q_l = sum Mo o_a
+// and a line takes n^2/2 products instead of n^2.  A matrix handed in with
+// other rounding takes the general form (SYM false, n^2 products).
+#pragma once
+
+#include <climits>
+#include <cmath>
+#include <vector>
+
+#include "mj_internal.cuh"
+#include "mj_k1.cuh"
+
+namespace mj {
+namespace {
+
+constexpr int kFxBad = INT_MIN;  // fac_exp of an element whose factors are not finite
+
+// Coefficients of the line transforms of every order as (lo, hi, lo >> 17),
+// and their scales.  [n][0]: gradient, y_l = sum_a G[a][l] r_a; [n][1]:
+// divergence, y_l = sum_a G'[l][a] r_a.  SYM: row l < (n+1)/2 holds Me at
+// a < n/2, the middle coefficient at a = n/2 (n odd) and Mo_a at n-1-a;
+// general: the matrix.
+__constant__ int4 c_fx[kMaxNK + 1][2][kMaxNK * kMaxNK];
+__constant__ int c_fx_exp[kMaxNK + 1];  // sum of both scales
+
+// Exponent of the similarity scaling at node i of n (see above).
+__host__ __device__ constexpr int fx_c(int n, int i) {
+  const int d = i < n - 1 - i ? i : n - 1 - i;  // distance from the nearer end
+  return d == 0 ? (n == 2 ? 0 : n == 3 ? 1 : 2) : d == 1 && n >= 6 ? 1 : 0;
+}
+
+__device__ __forceinline__ int2 fx_limbs(long long v) {
+  const int lo = (int)v;
+  return make_int2(lo, (int)(v >> 32) + (int)((unsigned)lo >> 31));
+}
+
+// One sum of products, value = h 2^64 + m 2^32, lo*lo to its upper bits in q
+// (units of 2^35; at most 9 terms of 2^27).  The wide multiply-adds are
+// written out: from 64-bit C++ products the compiler makes about three times
+// as many instructions.
+struct FxSum {
+  long long h, m;
+  int q;
+  __device__ __forceinline__ FxSum(int2 a, int ahi, int2 b, int bhi) {
+    asm("mul.wide.s32 %0, %1, %2;" : "=l"(h) : "r"(a.y), "r"(b.y));
+    asm("mul.wide.s32 %0, %1, %2;" : "=l"(m) : "r"(a.y), "r"(b.x));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(m) : "r"(a.x), "r"(b.y));
+    q = ahi * bhi;
+  }
+  __device__ __forceinline__ void mad(int2 a, int ahi, int2 b, int bhi) {
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(h) : "r"(a.y), "r"(b.y));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(m) : "r"(a.y), "r"(b.x));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(m) : "r"(a.x), "r"(b.y));
+    q += ahi * bhi;
+  }
+  // value / 2^(64 - sh), rounded
+  __device__ __forceinline__ long long norm(int sh) const {
+    long long t;
+    asm("mad.wide.s32 %0, %1, 8, %2;" : "=l"(t) : "r"(q), "l"(m));
+    return (h << sh) + ((t + (1LL << (31 - sh))) >> (32 - sh));
+  }
+};
+constexpr int kFxLoData = 18, kFxLoCoef = 17;  // lo*lo: (lo >> 18) (lo >> 17) in units of 2^35
+
+constexpr int kFxShG = 3, kFxShY = 3;
+constexpr int kFxBitsU = 59, kFxBitsB = 61, kFxBitsG = 61;  // the largest value (sum) in [2^bits, 2^(bits+1))
+// y_int = y 2^(c + ku + kb + kg - kFxYBias + sv), sv the shift of the fluxes
+constexpr int kFxYBias = (64 - kFxShG) + 64 + (64 - kFxShY);
+
+// One line transform (KIND 0: gradient, 1: divergence).
+template <int N, int KIND, bool SYM>
+__device__ __forceinline__ void fx_line(const long long (&r)[N], long long (&y)[N]) {
+  constexpr int SH = KIND ? kFxShY : kFxShG;
+  const int4* c = c_fx[N][KIND];
+  auto coef = [&](int at, int2& v, int& hi) {
+    const int4 q = c[at];
+    v = make_int2(q.x, q.y);
+    hi = q.z;
+  };
+  int2 v;
+  int vh;
+  if constexpr (SYM) {
+    constexpr int H = N / 2, C = N & 1;
+    int2 e[H + C], o[H];
+    int eh[H + C], oh[H];
+#pragma unroll
+    for (int a = 0; a < H; a++) {
+      e[a] = fx_limbs(r[a] + r[N - 1 - a]);
+      o[a] = fx_limbs(r[a] - r[N - 1 - a]);
+      eh[a] = e[a].x >> kFxLoData;
+      oh[a] = o[a].x >> kFxLoData;
+    }
+    if (C) {
+      e[H] = fx_limbs(r[H]);
+      eh[H] = e[H].x >> kFxLoData;
+    }
+#pragma unroll
+    for (int l = 0; l < H + C; l++) {
+      coef(l * N + N - 1, v, vh);
+      FxSum q(o[0], oh[0], v, vh);
+#pragma unroll
+      for (int a = 1; a < H; a++) {
+        coef(l * N + N - 1 - a, v, vh);
+        q.mad(o[a], oh[a], v, vh);
+      }
+      if (l == H) {  // the middle of an odd line
+        y[l] = q.norm(SH);
+      } else {
+        coef(l * N, v, vh);
+        FxSum p(e[0], eh[0], v, vh);
+#pragma unroll
+        for (int a = 1; a < H + C; a++) {
+          coef(l * N + a, v, vh);
+          p.mad(e[a], eh[a], v, vh);
+        }
+        const long long pn = p.norm(SH), qn = q.norm(SH);
+        y[l] = qn + pn;
+        y[N - 1 - l] = qn - pn;
+      }
+    }
+  } else {
+    int2 e[N];
+    int eh[N];
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      e[a] = fx_limbs(r[a]);
+      eh[a] = e[a].x >> kFxLoData;
+    }
+#pragma unroll
+    for (int l = 0; l < N; l++) {
+      coef(l * N, v, vh);
+      FxSum q(e[0], eh[0], v, vh);
+#pragma unroll
+      for (int a = 1; a < N; a++) {
+        coef(l * N + a, v, vh);
+        q.mad(e[a], eh[a], v, vh);
+      }
+      y[l] = q.norm(SH);
+    }
+  }
+}
+
+template <int N, int E>
+struct FxPlan {
+  static constexpr int NN = N * N;
+  static constexpr int Qp = elem_slots(N);
+  static constexpr int RS = N | 1;  // x-lines start an odd number of 8-byte words apart: no bank conflicts
+  static constexpr int W = NN * RS;  // work entries per element and array
+  static constexpr size_t fac_bytes = sizeof(int2) * 6 * E * Qp;
+  static constexpr size_t nod_bytes = sizeof(int) * E * Qp;
+  static constexpr size_t work_bytes = ((sizeof(long long) * 3 * E * W + 15) / 16) * 16;
+  static constexpr size_t max_bytes = ((sizeof(unsigned) * 3 * E + 15) / 16) * 16;
+  static constexpr size_t max_at = fac_bytes + 2 * nod_bytes + work_bytes;
+  static constexpr size_t total = max_at + max_bytes + 3 * sizeof(uint64_t);
+  static constexpr int threads = E * NN;
+  // CTAs per SM that shared memory admits (228 KB per SM, 1 KB of it per CTA): the register budget follows it
+  static constexpr int ctas = (int)(228 * 1024 / (total + 1024));
+  static_assert(fac_bytes % 16 == 0 && nod_bytes % 16 == 0, "bulk copies");
+};
+
+// The tile in FP64: the arithmetic of k_local_stiffness<double> (compact).
+// Every thread of the CTA calls it; work arrays are free on entry and exit.
+template <int N, int E>
+__device__ __noinline__ void fx_tile_fp64(const double* __restrict__ x, const int* nod, const double* __restrict__ fac,
+                                          double* __restrict__ R, const int* __restrict__ slot, double* su, double* sa,
+                                          double* sb) {
+  using P = FxPlan<N, E>;
+  constexpr int NN = P::NN, Qp = P::Qp, RS = P::RS;
+  const double* __restrict__ G = c_gmat64[N];
+  const int el = threadIdx.x / NN, ij = threadIdx.x - el * NN, j = ij / N, i = ij - j * N;
+  const int base = el * P::W, lx = base + j * RS, ly = base + i;
+  double u[N], vz[N];
+  for (int k = 0; k < N; k++) {
+    u[k] = x[nod[el * Qp + k * NN + ij]];
+    su[lx + k * N * RS + i] = u[k];
+  }
+  __syncthreads();
+  const double* f = fac + (size_t)el * 6 * Qp + ij;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    double gx = 0, gy = 0, gz = 0;
+#pragma unroll 1
+    for (int a = 0; a < N; a++) {
+      gx += G[a * N + i] * su[lx + k * N * RS + a];
+      gy += G[a * N + j] * su[ly + k * N * RS + a * RS];
+    }
+#pragma unroll
+    for (int a = 0; a < N; a++) gz += G[a * N + k] * u[a];
+    const double* fk = f + k * NN;
+    const double bxx = fk[0], bxy = fk[Qp], bxz = fk[2 * Qp], byy = fk[3 * Qp], byz = fk[4 * Qp], bzz = fk[5 * Qp];
+    sa[lx + k * N * RS + i] = fac_dot(bxx, gx, bxy, gy, bxz, gz);
+    sb[lx + k * N * RS + i] = fac_dot(bxy, gx, byy, gy, byz, gz);
+    vz[k] = fac_dot(bxz, gx, byz, gy, bzz, gz);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    double y = 0;
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      y += G[i * N + a] * sa[lx + k * N * RS + a];
+      y += G[j * N + a] * sb[ly + k * N * RS + a * RS];
+      y += G[k * N + a] * vz[a];
+    }
+    R[slot[el * Qp + k * NN + ij]] = y;
+  }
+}
+
+template <int N, int E, bool SYM>
+__global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
+    k_local_stiffness_fx(const double* __restrict__ x, const int* __restrict__ nodle_e,
+                         const int2* __restrict__ fac_fx, const int* __restrict__ fac_exp,
+                         const double* __restrict__ fac_e, double* __restrict__ R, const int* __restrict__ slot_e,
+                         int n_tiles, int* __restrict__ err) {
+  using P = FxPlan<N, E>;
+  constexpr int NN = P::NN, Qp = P::Qp, RS = P::RS, W = P::W;
+  extern __shared__ __align__(128) unsigned char smem[];
+  int2* s_fac = reinterpret_cast<int2*>(smem);
+  auto s_nod = [&](int st) { return reinterpret_cast<int*>(smem + P::fac_bytes + st * P::nod_bytes); };
+  long long* s_u = reinterpret_cast<long long*>(smem + P::fac_bytes + 2 * P::nod_bytes);  // [el][k][j][i], rows of RS
+  long long* s_a = s_u + E * W;
+  long long* s_b = s_a + E * W;
+  unsigned* s_max = reinterpret_cast<unsigned*>(smem + P::max_at);  // [2][E]: largest |u| (high word) of the tile's and
+  unsigned* s_gmax = s_max + 2 * E;                                 // the next tile's elements; [E]: largest |g|
+  // bar[0], bar[1]: the Nodle stages; bar[2]: the factor stage
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + P::max_at + P::max_bytes);
+
+  const int t = threadIdx.x;
+  const int el = t / NN;
+  const int ij = t - el * NN;
+  const int j = ij / N;
+  const int i = ij - j * N;
+  const int lz = el * W + j * RS + i;          // + k*N*RS: the points of z-line (i, j)
+  const int lx = el * W + ij * RS;             // + a: x-line (k, j) = (ij / N, ij % N)
+  const int ly = el * W + j * N * RS + i;      // + a*RS: y-line (k, i) = (ij / N, ij % N)
+  const int pe = el * Qp + ij;
+
+  if (t == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init(&bar[2], 1);
+    fence_mbar_init();
+  }
+  for (int q = t; q < 3 * E; q += P::threads) s_max[q] = 0u;
+  __syncthreads();
+  auto issue_nod = [&](int st, int tile) {
+    if (t == 0 && tile < n_tiles) {
+      mbar_expect_tx(&bar[st], (uint32_t)P::nod_bytes);
+      bulk_g2s_hint(s_nod(st), nodle_e + (size_t)tile * E * Qp, (uint32_t)P::nod_bytes, &bar[st],
+                    l2_evict_first_policy());
+    }
+  };
+  auto issue_fac = [&](int tile) {
+    if (t == 0 && tile < n_tiles) {
+      mbar_expect_tx(&bar[2], (uint32_t)P::fac_bytes);
+      bulk_g2s_hint(s_fac, fac_fx + (size_t)tile * E * 6 * Qp, (uint32_t)P::fac_bytes, &bar[2],
+                    l2_evict_first_policy());
+    }
+  };
+  const int g = gridDim.x;
+  int tile = blockIdx.x;
+  issue_nod(0, tile);
+  issue_fac(tile);
+  issue_nod(1, tile + g);
+  uint32_t ph = 0u;  // bits 0, 1: parity of the next completion of Nodle stage 0, 1; bit 2: of the factor stage
+  double u[N];
+  // largest high word of |u| over the thread's line (nonzero for any nonzero u), into the element's maximum
+  auto line_max = [&](int par) {
+    unsigned m = 0u;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      m = max(m, ((unsigned)__double2hiint(u[k]) & 0x7fffffffu) | (__double2loint(u[k]) != 0 ? 1u : 0u));
+    atomicMax(&s_max[par * E + el], m);
+  };
+  if (tile < n_tiles) {
+    const bool ok = mbar_wait_bounded(&bar[0], 0u);
+    if (__syncthreads_or(!ok)) {
+      if (t == 0) {  // report; every copy issued above may still be in flight
+        atomicExch(err, 1);
+        mbar_wait_drain(&bar[0], 0u);
+        mbar_wait_drain(&bar[2], 0u);
+        if (tile + g < n_tiles) mbar_wait_drain(&bar[1], 0u);
+      }
+      return;
+    }
+    ph ^= 1u;
+    const int* nd = s_nod(0) + pe;
+#pragma unroll
+    for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+    line_max(0);
+  }
+  __syncthreads();
+  const int kg = c_fx_exp[N];
+  for (int it = 0; tile < n_tiles; tile += g, ++it) {
+    const int s = it & 1;
+    // the element's scales: u 2^ku, B 2^kb, result 2^eo
+    const unsigned um = s_max[s * E + el];
+    const int kb = __ldg(fac_exp + (size_t)tile * E + el);
+    const int eu = (int)(um >> 20) - 1023;
+    const int ku = um ? kFxBitsU - eu : 0;
+    const int eo = kFxYBias - ku - (kb == kFxBad ? 0 : kb) - kg;
+    const bool bad = kb == kFxBad || (um && (eu > 1023 || eu < -900 || eo < -950 || eo > 1000));
+    long long uz[N];
+    {
+      const double sc = __hiloint2double((1023 + (bad ? 0 : ku)) << 20, 0);
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        uz[k] = __double2ll_rn(u[k] * sc);
+        s_u[lz + k * N * RS] = uz[k];
+      }
+    }
+    const bool fp64 = __syncthreads_or(bad);  // also: u staged, the maxima read
+    if (t < E) s_max[s * E + t] = 0u;
+    long long gz[N];
+    if (!fp64) {
+      long long r[N], y[N];
+#pragma unroll
+      for (int a = 0; a < N; a++) r[a] = s_u[lx + a];
+      unsigned gm = 0u;  // largest high word of |g|, one unit low for negative values
+      auto top = [&](const long long (&v)[N]) {
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          const int hi = (int)(v[a] >> 32);
+          gm = max(gm, (unsigned)(hi ^ (hi >> 31)));
+        }
+      };
+      fx_line<N, 0, SYM>(r, y);
+      top(y);
+#pragma unroll
+      for (int a = 0; a < N; a++) s_a[lx + a] = y[a];
+#pragma unroll
+      for (int a = 0; a < N; a++) r[a] = s_u[ly + a * RS];
+      fx_line<N, 0, SYM>(r, y);
+      top(y);
+#pragma unroll
+      for (int a = 0; a < N; a++) s_b[ly + a * RS] = y[a];
+      fx_line<N, 0, SYM>(uz, gz);
+      top(gz);
+      atomicMax(&s_gmax[el], gm);
+    }
+    {  // this tile's factors (the vote is also the barrier after the gradients)
+      const bool ok = mbar_wait_bounded(&bar[2], (ph >> 2) & 1u);
+      if (__syncthreads_or(!ok)) {
+        if (t == 0) {  // report; this tile's factors and the next tile's Nodle may be in flight
+          atomicExch(err, 1);
+          mbar_wait_drain(&bar[2], (ph >> 2) & 1u);
+          if (tile + g < n_tiles) mbar_wait_drain(&bar[s ^ 1], (ph >> (s ^ 1)) & 1u);
+        }
+        return;
+      }
+      ph ^= 4u;
+    }
+    long long vz[N];
+    // |g| < 2^(64 - lz) with lz >= 2 leading zeros: |v| < 2^62 2^(64 - lz) / 2^(64 - sv) <= 2^60
+    const int sv = min(31, __clz((int)s_gmax[el]) - 2);
+    if (!fp64) {
+      const int2* f = s_fac + el * 6 * Qp + ij;
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        const int2 gx = fx_limbs(s_a[lz + k * N * RS]), gy = fx_limbs(s_b[lz + k * N * RS]), gk = fx_limbs(gz[k]);
+        const int gxh = gx.x >> kFxLoData, gyh = gy.x >> kFxLoData, gkh = gk.x >> kFxLoData;
+        const int2* fk = f + k * NN;
+        const int2 bxx = fk[0], bxy = fk[Qp], bxz = fk[2 * Qp];
+        const int2 byy = fk[3 * Qp], byz = fk[4 * Qp], bzz = fk[5 * Qp];
+        const int xyh = bxy.x >> kFxLoCoef, xzh = bxz.x >> kFxLoCoef, yzh = byz.x >> kFxLoCoef;
+        FxSum a(gx, gxh, bxx, bxx.x >> kFxLoCoef), b(gx, gxh, bxy, xyh), c(gx, gxh, bxz, xzh);
+        a.mad(gy, gyh, bxy, xyh); a.mad(gk, gkh, bxz, xzh);
+        b.mad(gy, gyh, byy, byy.x >> kFxLoCoef); b.mad(gk, gkh, byz, yzh);
+        c.mad(gy, gyh, byz, yzh); c.mad(gk, gkh, bzz, bzz.x >> kFxLoCoef);
+        s_a[lz + k * N * RS] = a.norm(sv);
+        s_b[lz + k * N * RS] = b.norm(sv);
+        vz[k] = c.norm(sv);
+      }
+    } else {
+      fx_tile_fp64<N, E>(x, s_nod(s), fac_e + (size_t)tile * E * 6 * Qp, R, slot_e + (size_t)tile * E * Qp,
+                         reinterpret_cast<double*>(s_u), reinterpret_cast<double*>(s_a),
+                         reinterpret_cast<double*>(s_b));
+    }
+    __syncthreads();  // the factor stage is free, the fluxes are staged
+    if (t < E) s_gmax[t] = 0u;
+    if (t == 0) fence_proxy_async();
+    issue_fac(tile + g);  // the next tile's factors, during this divergence
+
+    // gather of the next tile's u, in flight during the divergence
+    const int nt = tile + g;
+    bool lost = false;
+    if (nt < n_tiles) {
+      const int so = s ^ 1;
+      lost = !mbar_wait_bounded(&bar[so], (ph >> so) & 1u);
+      ph ^= 1u << so;
+      if (!lost) {
+        const int* nd = s_nod(so) + pe;
+#pragma unroll
+        for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+      }
+    }
+    long long wz[N];
+    if (!fp64) {
+      long long r[N], y[N];
+#pragma unroll
+      for (int a = 0; a < N; a++) r[a] = s_a[lx + a];
+      fx_line<N, 1, SYM>(r, y);
+#pragma unroll
+      for (int a = 0; a < N; a++) s_a[lx + a] = y[a];
+#pragma unroll
+      for (int a = 0; a < N; a++) r[a] = s_b[ly + a * RS];
+      fx_line<N, 1, SYM>(r, y);
+#pragma unroll
+      for (int a = 0; a < N; a++) s_b[ly + a * RS] = y[a];
+      fx_line<N, 1, SYM>(vz, wz);
+    }
+    if (nt < n_tiles && !lost) line_max(s ^ 1);
+    if (__syncthreads_or(lost)) {
+      if (t == 0) {  // report; Nodle stage s^1 and the factors just issued may be in flight
+        atomicExch(err, 1);
+        mbar_wait_drain(&bar[s ^ 1], ((ph >> (s ^ 1)) & 1u) ^ 1u);
+        mbar_wait_drain(&bar[2], (ph >> 2) & 1u);
+      }
+      return;
+    }
+    if (t == 0) fence_proxy_async();
+    issue_nod(s, tile + 2 * g);
+    if (!fp64) {
+      const int ex = 1023 + (um ? eo - sv : 9) - fx_c(N, i) - fx_c(N, j);
+      const int* st = slot_e + ((size_t)tile * E + el) * Qp + ij;
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        const long long y = wz[k] + s_a[lz + k * N * RS] + s_b[lz + k * N * RS];
+        R[__ldg(st + k * NN)] = __ll2double_rn(y) * __hiloint2double((ex - fx_c(N, k)) << 20, 0);
+      }
+    }
+  }
+}
+
+// (n, E): the tile sizes of k1_tile_candidates
+#define MJ_FX_VARIANTS(X) \
+  X(2, 30) X(2, 60) X(3, 12) X(3, 24) X(4, 8) X(4, 16) X(5, 4) X(5, 5) X(5, 8) X(5, 10) \
+  X(6, 3) X(6, 4) X(6, 6) X(7, 2) X(7, 3) X(7, 4) X(7, 5) X(8, 2) X(8, 3) X(8, 4) X(9, 1) X(9, 2) X(9, 3)
+
+template <int N, int E, bool SYM>
+int prepare_fx_one(int* ctas) {
+  using P = FxPlan<N, E>;
+  int dev = 0, optin = 0;
+  MJ_CUDA(cudaGetDevice(&dev));
+  MJ_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  if ((int)P::total > optin) {
+    set_error("element kernel variant does not fit in shared memory");
+    return MJ_ERR_ARG;
+  }
+  MJ_CUDA(cudaFuncSetAttribute(k_local_stiffness_fx<N, E, SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)P::total));
+  MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, k_local_stiffness_fx<N, E, SYM>, P::threads, P::total));
+  if (*ctas < 1) {
+    set_error("element kernel variant cannot be resident");
+    return MJ_ERR_ARG;
+  }
+  return MJ_OK;
+}
+
+template <bool SYM>
+int prepare_fx(int n, int E, int* ctas) {
+#define MJ_X(NV, EV) \
+  if (n == NV && E == EV) return prepare_fx_one<NV, EV, SYM>(ctas);
+  MJ_FX_VARIANTS(MJ_X)
+#undef MJ_X
+  set_error("no fixed-point element kernel variant for this order and tile size");
+  return MJ_ERR_ARG;
+}
+
+template <bool SYM>
+void launch_fx(mj_op* op, const void* x, cudaStream_t s) {
+#define MJ_X(NV, EV)                                                                                          \
+  if (op->n == NV && op->E == EV) {                                                                           \
+    k_local_stiffness_fx<NV, EV, SYM><<<op->grid_k1, FxPlan<NV, EV>::threads, FxPlan<NV, EV>::total, s>>>(    \
+        static_cast<const double*>(x), op->nodle_e.as<int>(), op->fac_fx.as<int2>(), op->fac_exp.as<int>(),   \
+        op->fac_e.as<double>(), op->R.as<double>(), op->slot_e.as<int>(), op->n_tiles, op->err.as<int>());    \
+    return;                                                                                                   \
+  }
+  MJ_FX_VARIANTS(MJ_X)
+#undef MJ_X
+}
+#undef MJ_FX_VARIANTS
+
+// Coefficients of order n into this unit's constant memory.
+template <bool SYM>
+int set_gmat_fx(int n, const double* g) {
+  // gradient y_l = sum_a G[a][l] r_a and divergence y_l = sum_a 2^(c_l - c_a) G[l][a] r_a
+  auto coef = [&](int kind, int a, int l) {
+    return kind ? std::ldexp(g[l * n + a], fx_c(n, l) - fx_c(n, a)) : g[a * n + l];
+  };
+  int4 v[2][kMaxNK * kMaxNK] = {};
+  int ksum = 0;
+  for (int kind = 0; kind < 2; kind++) {
+    double m = 0.0;  // largest sum of |coefficients|
+    for (int l = 0; l < n; l++) {
+      double t = 0.0;
+      for (int a = 0; a < n; a++) t += std::fabs(coef(kind, a, l));
+      m = std::max(m, t);
+    }
+    const int kg = kFxBitsG - std::ilogb(m);
+    ksum += kg;
+    auto M = [&](int a, int l) { return std::llrint(std::ldexp(coef(kind, a, l), kg)); };
+    auto put = [&](int at, long long x) {
+      const int lo = (int)(x & 0xffffffffLL);
+      v[kind][at] = make_int4(lo, (int)((x - lo) / 4294967296LL), lo >> kFxLoCoef, 0);
+    };
+    if (!SYM) {
+      for (int l = 0; l < n; l++)
+        for (int a = 0; a < n; a++) put(l * n + a, M(a, l));
+      continue;
+    }
+    for (int l = 0; l < (n + 1) / 2; l++) {
+      for (int a = 0; a < n / 2; a++) {
+        const long long p = M(a, l), q = M(n - 1 - a, l);  // r_a = (e + o) / 2, r_(n-1-a) = (e - o) / 2
+        put(l * n + a, (p + q) / 2);
+        put(l * n + n - 1 - a, (p - q) / 2);
+      }
+      if ((n & 1) && l != n / 2) put(l * n + n / 2, M(n / 2, l));
+    }
+  }
+  const size_t per = sizeof(v);
+  MJ_CUDA(cudaMemcpyToSymbol(c_fx, v, per, per * n));
+  MJ_CUDA(cudaMemcpyToSymbol(c_fx_exp, &ksum, sizeof(int), sizeof(int) * n));
+  MJ_CUDA(cudaMemcpyToSymbol(c_gmat64, g, sizeof(double) * n * n, sizeof(double) * kMaxNK * kMaxNK * n));
+  return MJ_OK;
+}
+
+}  // namespace
+}  // namespace mj

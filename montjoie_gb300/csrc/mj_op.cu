@@ -82,7 +82,7 @@ void launch_k1(mj_op* op, const void* x, cudaStream_t s) {
     const bool done =
         op->warp ? k1_launch_w_f32_waits_out(op->n, op->E, op->grid_k1, x, op->nodle_e.as<int>(), op->fac_e.ptr,
                                             op->R.ptr, op->slot_e.as<int>(), op->n_tiles, op->err.as<int>(), s)
-        : op->precision == MJ_FP64 && !op->vec
+        : op->precision == MJ_FP64 && !op->vec && !op->fx
             ? k1_launch_f64_waits_out(op->n, op->E, op->grid_k1, x, op->nodle_e.as<int>(), op->fac_e.ptr, op->R.ptr,
                                       op->slot_e.as<int>(), op->n_tiles, op->err.as<int>(), s)
             : false;
@@ -90,6 +90,11 @@ void launch_k1(mj_op* op, const void* x, cudaStream_t s) {
       count_launch();
       return;
     }
+  }
+  if (op->fx) {
+    k1_launch_fx(op, x, s);
+    count_launch();
+    return;
   }
   if (op->warp) {
     k1_launch_w_f32(op->n, op->E, op->packed, op->grid_k1, x, (op->packed ? op->nodle_pk : op->nodle_e).as<int>(),
@@ -135,11 +140,13 @@ int autotune_k1(mj_op* op) {
   MJ_CUDA(cudaEventCreate(&e1));
   double best = 1e300;
   int bestE = -1, bestGrid = 1;
-  bool bestVec = false, bestWarp = false, bestPacked = false, bestFs = false;
+  bool bestVec = false, bestWarp = false, bestPacked = false, bestFs = false, bestFx = false;
   const bool time_it = (long long)op->n_elt * op->Q >= 2000000;
   // layouts: 0 compact, 1 vector lines, 2 one element per warp, 3 the same
-  // with packed connectivity, 4 compact with one factor stage (2-4: FP32)
-  std::vector<int> layouts = {0};
+  // with packed connectivity, 4 compact with one factor stage (2-4: FP32), 5 fixed point (FP64: always where the
+  // derivative matrix is in its range; the FP64-pipe kernel took 2.1 (Q1) to 4.4 (Q6) times as long on large meshes,
+  // 1.4 to 3 times on meshes of 5,000 to 275,000 dofs, and as long on 125 dofs)
+  std::vector<int> layouts = {op->fac_fx.ptr ? 5 : 0};
   if (op->precision == MJ_FP32) {
     layouts = {0, 1, 2};
     if (op->nodle_pk.ptr) layouts.push_back(3);
@@ -148,8 +155,10 @@ int autotune_k1(mj_op* op) {
   for (int lay : layouts)
     for (int E : ((lay == 2 || lay == 3) ? k1_warp_tile_candidates(op->n) : cands)) {
       const bool vec = lay == 1, warp = lay == 2 || lay == 3, packed = lay == 3, fs = lay == 4;
+      const bool fx = lay == 5;
       int ctas = 0;
-      const int rc = warp ? k1_prepare_w_f32(op->n, E, packed, &ctas)
+      const int rc = fx ? k1_prepare_fx(op, E, &ctas)
+                     : warp ? k1_prepare_w_f32(op->n, E, packed, &ctas)
                      : fs ? k1_prepare_fs_f32(op->n, E, &ctas)
                           : op->precision == MJ_FP64 ? k1_prepare_f64(op->n, E, vec, &ctas)
                                                      : k1_prepare_f32(op->n, E, vec, &ctas);
@@ -158,7 +167,8 @@ int autotune_k1(mj_op* op) {
       const int grid = std::max(1, std::min(tiles, ctas * sms));
       double ms = 0.0;
       if (time_it) {
-        op->E = E; op->vec = vec; op->warp = warp; op->packed = packed; op->fs = fs; op->grid_k1 = grid;
+        op->E = E; op->vec = vec; op->warp = warp; op->packed = packed; op->fs = fs; op->fx = fx;
+        op->grid_k1 = grid;
         op->n_tiles = tiles;
         launch_k1(op, x.ptr, op->stream);
         MJ_CUDA(cudaEventRecord(e0, op->stream));
@@ -177,6 +187,7 @@ int autotune_k1(mj_op* op) {
       op->tune_ms.push_back(ms);
       if (ms < best) {
         best = ms; bestE = E; bestGrid = grid; bestVec = vec; bestWarp = warp; bestPacked = packed; bestFs = fs;
+        bestFx = fx;
       }
     }
   cudaEventDestroy(e0);
@@ -190,11 +201,13 @@ int autotune_k1(mj_op* op) {
   op->warp = bestWarp;
   op->packed = bestPacked;
   op->fs = bestFs;
+  op->fx = bestFx;
   op->grid_k1 = bestGrid;
   // the chosen variant's shared-memory attribute must be the one set last
   {
     int ctas = 0;
-    const int rc = bestWarp ? k1_prepare_w_f32(op->n, bestE, bestPacked, &ctas)
+    const int rc = bestFx ? k1_prepare_fx(op, bestE, &ctas)
+                   : bestWarp ? k1_prepare_w_f32(op->n, bestE, bestPacked, &ctas)
                    : bestFs ? k1_prepare_fs_f32(op->n, bestE, &ctas)
                             : op->precision == MJ_FP64 ? k1_prepare_f64(op->n, bestE, bestVec, &ctas)
                                                        : k1_prepare_f32(op->n, bestE, bestVec, &ctas);
@@ -403,6 +416,14 @@ int op_layout(mj_op* op, const mj_mesh_desc* mesh, const double* gradphi, int pr
 int op_finish(mj_op* op) {
   int rc = op->precision == MJ_FP64 ? k1_set_gmat_f64(op->n, op->gradphi) : k1_set_gmat_f32(op->n, op->gradphi);
   if (rc) return rc;
+  if (op->precision == MJ_FP64 && k1_fx_supports(op->n, op->gradphi, &op->fx_sym)) {
+    rc = k1_set_gmat_fx(op->n, op->gradphi, op->fx_sym);
+    if (rc) return rc;
+    MJ_CUDA(op->fac_fx.alloc(op->fac_e.bytes));
+    MJ_CUDA(op->fac_exp.alloc(sizeof(int) * op->n_elt_pad));
+    rc = k1_fixed_factors(op, op->stream);
+    if (rc) return rc;
+  }
   return autotune_k1(op);
 }
 
@@ -639,7 +660,7 @@ int mj_op_tuning(const mj_op* op, int* tile_elems, int* vector_lines, int* grid,
                  double* candidate_ms) {
   MJ_CHECK_ARG(op, "mj_op_tuning: null operator");
   if (tile_elems) *tile_elems = op->E;
-  if (vector_lines) *vector_lines = op->fs ? 4 : op->packed ? 3 : op->warp ? 2 : op->vec ? 1 : 0;
+  if (vector_lines) *vector_lines = op->fx ? 5 : op->fs ? 4 : op->packed ? 3 : op->warp ? 2 : op->vec ? 1 : 0;
   if (grid) *grid = op->grid_k1;
   if (n_candidates) *n_candidates = (int)op->tune_ms.size();
   if (candidate_ms)
@@ -669,6 +690,7 @@ int mj_op_set_variant(mj_op* op, int tile_elems, int vector_lines) {
   op->warp = warp;
   op->packed = packed;
   op->fs = fs;
+  op->fx = false;
   op->n_tiles = op->n_elt_pad / tile_elems;
   op->grid_k1 = std::max(1, std::min(op->n_tiles, ctas * sm_count()));
   return MJ_OK;

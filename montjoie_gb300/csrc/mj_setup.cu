@@ -98,6 +98,12 @@ void gl_derivative_matrix(int r, const double* pts, double* g) {
     g[b * n + b] = -sum;
     if (std::fabs(g[b * n + b]) <= 1e3 * 2.220446049250313e-16) g[b * n + b] = 0.0;
   }
+  // the matrix is antisymmetric under the mirror (a, b) -> (r-a, r-b); keep it so to the last bit
+  for (int q = 0; q < n * n / 2; q++) {
+    g[q] = 0.5 * (g[q] - g[n * n - 1 - q]);
+    g[n * n - 1 - q] = -g[q];
+  }
+  if (n & 1) g[n * n / 2] = 0.0;
 }
 
 // ------------------------------------------------------------ geometry kernel
