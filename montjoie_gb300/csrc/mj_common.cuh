@@ -73,6 +73,27 @@ struct DevBuf {
   T* as() const { return static_cast<T*>(ptr); }
 };
 
+// Page-locked host buffer owned by the library: device-to-host copies into it
+// are queued, where a copy into pageable memory makes the host wait for each.
+struct PinBuf {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  PinBuf() = default;
+  PinBuf(const PinBuf&) = delete;
+  PinBuf& operator=(const PinBuf&) = delete;
+  ~PinBuf() {
+    if (ptr) cudaFreeHost(ptr);
+  }
+  cudaError_t alloc(size_t b) {
+    if (ptr) cudaFreeHost(ptr);
+    ptr = nullptr;
+    bytes = b;
+    return cudaMallocHost(&ptr, b);
+  }
+  template <class T>
+  T* as() const { return static_cast<T*>(ptr); }
+};
+
 // Local numbering NumDofs3D of a Q_r hexahedron, num[(i*n+j)*n+k] = local
 // index of the node (i,j,k) (i along x): vertices, the 12 edges, the faces
 // x=0, y=0, z=0, z=1, y=1, x=1, then the interior
@@ -88,7 +109,8 @@ int sm_count();
 
 // Reads a kernel's device error flag after the work on `s`; when it is set,
 // clears it (so the next call starts clean), records "<what>: <message>" and
-// returns MJ_ERR_CUDA.  Synchronises `s`.
-int take_kernel_error(void* dev_flag, cudaStream_t s, const char* what);
+// returns MJ_ERR_CUDA.  Synchronises `s`.  host: a page-locked int to read it
+// through.
+int take_kernel_error(void* dev_flag, cudaStream_t s, const char* what, int* host);
 
 }  // namespace mj

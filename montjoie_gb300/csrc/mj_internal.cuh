@@ -30,13 +30,14 @@ struct mj_op {
   mj::DevBuf verts;                     // n_elt x 8 x 3 vertices (operators built from geometry)
   std::vector<int> h_ptr;               // CSR of incidences per dof (host copy)
   double gradphi[mj::kMaxN * mj::kMaxN];
-  mj::DevBuf xbuf, ybuf;                // staging for host-vector MltAdd
+  mj::DevBuf xbuf, ybuf, stage;         // staging for host-vector MltAdd
+  mj::PinBuf h_status;                  // where kernel error flags are read (page-locked)
   cudaStream_t stream = nullptr;
   std::vector<double> tune_ms;          // autotuner timings of the candidates (diagnostic)
   std::vector<int> tune_E, tune_vec;
   size_t device_bytes() const {
     return nodle_e.bytes + fac_e.bytes + fac_orig.bytes + slot_e.bytes + R.bytes + ptr.bytes + xbuf.bytes +
-           ybuf.bytes + verts.bytes + nodle_pk.bytes + fac_fx.bytes + fac_exp.bytes;
+           ybuf.bytes + stage.bytes + verts.bytes + nodle_pk.bytes + fac_fx.bytes + fac_exp.bytes;
   }
 };
 
@@ -54,8 +55,9 @@ struct mj_lf {
                              // them as dt^2 / (dt^2/D), from the dt^2/D it stages anyway
   mj::DevBuf rec_idx, rec_w; // receivers
   mj::DevBuf ua, ub;         // state: U^n (cur) and U^{n+1} (next)
-  mj::DevBuf du0, tmp;       // staging
-  mj::DevBuf partial, norms_d, traces_d, flag;
+  mj::DevBuf du0, stage;     // staging
+  mj::DevBuf partial, diag_d, flag;  // diag_d: norms, then the receivers' rows
+  mj::PinBuf h_diag;         // page-locked copy of small diagnostics, and the flag
   mj::DevBuf diag_done, diag_where;  // fused diagnostics: finished-block counter, DiagDev of graph replays
   mj::DevBuf stream_partial;         // per-CTA norm partials of the streaming gather's diagnostics
   mj::DevBuf pulse_d, ctr;   // pulse of every step and the two step counters
@@ -221,6 +223,7 @@ int assemble_points(int order, int n_elt, int Qp, const double* jw, const double
 // variant choice at creation, and the advance used by mj_lfb_advance.
 int lfb_fused_setup(mj_lfb* b);
 int lfb_fused_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, bool use_graph);
+int lfb_copy_traces(mj_lfb* b, int nsteps, double* traces, int trace_stride, cudaStream_t s);
 void lfb_receivers(mj_lfb* b, const float* u, int stride, int col, cudaStream_t s);
 int lfb_phase_ms(const mj_lfb* b, double* out);
 int lfb_fused_step_on(mj_lfb* b, float* u0, float* u1, float* out, bool sources, cudaStream_t s);

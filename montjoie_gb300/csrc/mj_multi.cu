@@ -403,9 +403,9 @@ int mb_check_err(mj_mb* mb, cudaStream_t s) {
     else if (rc) return rc;
     if (g->seq)  // runs stepped with their own kernels report through their operators
       for (mj_lf* lf : g->runs)
-        if (take_kernel_error(lf->op->err.ptr, s, "mj_mb_advance")) herr = 1;
+        if (take_kernel_error(lf->op->err.ptr, s, "mj_mb_advance", lf->op->h_status.as<int>())) herr = 1;
   }
-  if (mb->uni && take_kernel_error(mb->uni->op->err.ptr, s, "mj_mb_advance")) herr = 1;
+  if (mb->uni && take_kernel_error(mb->uni->op->err.ptr, s, "mj_mb_advance", mb->uni->op->h_status.as<int>())) herr = 1;
   int own = 0;
   MJ_CUDA(cudaMemcpyAsync(&own, mb->err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
   MJ_CUDA(cudaStreamSynchronize(s));

@@ -221,11 +221,10 @@ int autotune_k1(mj_op* op) {
 
 }  // namespace
 
-int mj::take_kernel_error(void* dev_flag, cudaStream_t s, const char* what) {
-  int herr = 0;
-  MJ_CUDA(cudaMemcpyAsync(&herr, dev_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+int mj::take_kernel_error(void* dev_flag, cudaStream_t s, const char* what, int* host) {
+  MJ_CUDA(cudaMemcpyAsync(host, dev_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
   MJ_CUDA(cudaStreamSynchronize(s));
-  if (!herr) return MJ_OK;
+  if (!*host) return MJ_OK;
   MJ_CUDA(cudaMemsetAsync(dev_flag, 0, sizeof(int), s));
   MJ_CUDA(cudaStreamSynchronize(s));
   set_error(std::string(what) + ": a bounded wait of a kernel on its bulk copies timed out (results invalid)");
@@ -414,6 +413,7 @@ int op_layout(mj_op* op, const mj_mesh_desc* mesh, const double* gradphi, int pr
 
 // Derivative matrix into constant memory and the element-kernel autotuner.
 int op_finish(mj_op* op) {
+  MJ_CUDA(op->h_status.alloc(64));
   int rc = op->precision == MJ_FP64 ? k1_set_gmat_f64(op->n, op->gradphi) : k1_set_gmat_f32(op->n, op->gradphi);
   if (rc) return rc;
   if (op->precision == MJ_FP64 && k1_fx_supports(op->n, op->gradphi, &op->fx_sym)) {
@@ -638,7 +638,7 @@ int mj_op_power_iteration(mj_op* op, const double* inv_mass, const double* x0, i
   }
   MJ_CUDA(cudaGetLastError());
   *lambda_max = lam;
-  return take_kernel_error(op->err.ptr, s, "mj_op_power_iteration");
+  return take_kernel_error(op->err.ptr, s, "mj_op_power_iteration", op->h_status.as<int>());
 }
 
 int mj_op_destroy(mj_op* op) {
@@ -709,7 +709,7 @@ int mj_op_mltadd(mj_op* op, double alpha, const double* x, double beta, double* 
   const int n = op->n_dof;
   if (op->xbuf.bytes < esz * n) MJ_CUDA(op->xbuf.alloc(esz * n));
   if (op->ybuf.bytes < esz * n) MJ_CUDA(op->ybuf.alloc(esz * n));
-  DevBuf stage;
+  DevBuf& stage = op->stage;  // FP32: kept, an allocation per call cost more than a small product
   cudaStream_t s = op->stream;
   int rc = upload_vec(op, x, op->xbuf.ptr, stage, s);
   if (rc) return rc;
@@ -721,7 +721,7 @@ int mj_op_mltadd(mj_op* op, double alpha, const double* x, double beta, double* 
   if (rc) return rc;
   rc = download_vec(op, op->ybuf.ptr, y, stage, s);
   if (rc) return rc;
-  return take_kernel_error(op->err.ptr, s, "mj_op_mltadd");
+  return take_kernel_error(op->err.ptr, s, "mj_op_mltadd", op->h_status.as<int>());
 }
 
 int mj_debug_set_wait_limits(long long mbar_polls, long long barrier_polls, long long barrier_ns) {
@@ -824,6 +824,9 @@ int lf_stream_setup(mj_lf* lf) {
 
 }  // namespace
 
+// Page-locked bytes of an integrator for its flag and small diagnostics.
+constexpr size_t kDiagPinned = 32768;
+
 extern "C" {
 
 // ------------------------------------------------------------------ leap-frog
@@ -917,6 +920,7 @@ int mj_lf_create(mj_op* op, const mj_lf_desc* desc, mj_lf** out) {
   MJ_CUDA(lf->diag_done.alloc(sizeof(unsigned)));
   MJ_CUDA(cudaMemset(lf->diag_done.ptr, 0, sizeof(unsigned)));
   MJ_CUDA(lf->diag_where.alloc(sizeof(DiagDev)));
+  MJ_CUDA(lf->h_diag.alloc(kDiagPinned));
   MJ_CUDA(cudaMemset(lf->flag.ptr, 0, sizeof(int)));
   if (op->precision == MJ_FP32) {
     int rc = lf_sorted_sources(lf.get());
@@ -948,7 +952,7 @@ int lf_init_impl(mj_lf* lf, const double* u0, const double* du0) {
   mj_op* op = lf->op;
   cudaStream_t s = lf->stream;
   const int n = lf->n_dof;
-  DevBuf stage;
+  DevBuf& stage = lf->stage;
   int rc = upload_vec(op, u0, lf->ua.ptr, stage, s);
   if (rc) return rc;
   const Real* du0_d = nullptr;
@@ -1213,16 +1217,13 @@ int lf_advance_impl(mj_lf* lf, int nsteps, double* norms, double* traces, int st
   const int cols = nsteps + (final_diag ? 1 : 0);
   double* nd = nullptr;
   double* td = nullptr;
-  if (norms && lf->norm_w.ptr) {
-    if (lf->norms_d.bytes < sizeof(double) * cols) MJ_CUDA(lf->norms_d.alloc(sizeof(double) * cols));
-    nd = lf->norms_d.as<double>();
-  }
-  if (traces && lf->n_rec) {
-    MJ_CHECK_ARG(stride >= cols, "mj_lf_advance: trace_stride smaller than the number of recorded iterates");
-    const size_t b = sizeof(double) * (size_t)lf->n_rec * cols;
-    if (lf->traces_d.bytes < b) MJ_CUDA(lf->traces_d.alloc(b));
-    td = lf->traces_d.as<double>();
-  }
+  const bool want_n = norms && lf->norm_w.ptr, want_t = traces && lf->n_rec;
+  MJ_CHECK_ARG(!want_t || stride >= cols, "mj_lf_advance: trace_stride smaller than the number of recorded iterates");
+  // norms, then the receivers' rows, in one buffer
+  const size_t diag_bytes = sizeof(double) * (size_t)cols * ((want_n ? 1 : 0) + (want_t ? lf->n_rec : 0));
+  if (lf->diag_d.bytes < diag_bytes) MJ_CUDA(lf->diag_d.alloc(diag_bytes));
+  if (want_n) nd = lf->diag_d.as<double>();
+  if (want_t) td = lf->diag_d.as<double>() + (want_n ? cols : 0);
   int s0 = 0;
   bool replayed_prof = false;
   if (!nd && !td && !lf->profile && lf->use_graph && nsteps >= kGraphSteps + 1) {
@@ -1302,17 +1303,31 @@ int lf_advance_impl(mj_lf* lf, int nsteps, double* norms, double* traces, int st
     if (rc) return rc;
   }
   cudaStream_t s = lf->stream;
-  if (nd) MJ_CUDA(cudaMemcpyAsync(norms, nd, sizeof(double) * cols, cudaMemcpyDeviceToHost, s));
-  if (td)
-    for (int k = 0; k < lf->n_rec; k++)
-      MJ_CUDA(cudaMemcpyAsync(traces + (size_t)k * stride, td + (size_t)k * cols, sizeof(double) * cols,
-                              cudaMemcpyDeviceToHost, s));
-  int flag = 0;
-  MJ_CUDA(cudaMemcpyAsync(&flag, lf->flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
-  {
-    const int rc = take_kernel_error(lf->op->err.ptr, s, "mj_lf_advance");
-    if (rc) return rc;
+  // Small diagnostics come back in one queued copy through the page-locked
+  // buffer (a copy into pageable memory per receiver and flag made the host
+  // wait 8 us each: a one-step call with 8 receivers took 137 us); large ones
+  // in one copy each.
+  const bool small = diag_bytes && diag_bytes + 8 <= kDiagPinned;
+  int* hflag = lf->h_diag.as<int>();
+  double* hdata = lf->h_diag.as<double>() + 1;
+  MJ_CUDA(cudaMemcpyAsync(hflag, lf->flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (small) {
+    MJ_CUDA(cudaMemcpyAsync(hdata, lf->diag_d.ptr, diag_bytes, cudaMemcpyDeviceToHost, s));
+  } else if (cols) {
+    if (nd) MJ_CUDA(cudaMemcpyAsync(norms, nd, sizeof(double) * cols, cudaMemcpyDeviceToHost, s));
+    if (td)
+      MJ_CUDA(cudaMemcpy2DAsync(traces, sizeof(double) * stride, td, sizeof(double) * cols, sizeof(double) * cols,
+                                lf->n_rec, cudaMemcpyDeviceToHost, s));
   }
+  const int kernel_rc = take_kernel_error(lf->op->err.ptr, s, "mj_lf_advance", lf->op->h_status.as<int>());
+  if (small) {
+    if (nd) std::copy(hdata, hdata + cols, norms);
+    const double* rows = hdata + (nd ? cols : 0);
+    for (int k = 0; td && k < lf->n_rec; k++)
+      std::copy(rows + (size_t)k * cols, rows + (size_t)(k + 1) * cols, traces + (size_t)k * stride);
+  }
+  const int flag = *hflag;
+  if (kernel_rc) return kernel_rc;
   if (replayed_prof) {  // per-kernel times of the last replay
     const int base = (int)lf->ev.size() - 3 * kGraphSteps;
     for (int k = 0; k < kGraphSteps; k++) {
@@ -1379,7 +1394,7 @@ int mj_lf_get_state(mj_lf* lf, double* u_n, double* u_np1) {
     set_error("mj_lf_get_state: mj_lf_init must be called first");
     return MJ_ERR_STATE;
   }
-  DevBuf stage;
+  DevBuf& stage = lf->stage;
   int rc;
   if (u_n && (rc = download_vec(lf->op, lf->cur(), u_n, stage, lf->stream))) return rc;
   if (u_np1 && (rc = download_vec(lf->op, lf->next(), u_np1, stage, lf->stream))) return rc;

@@ -189,10 +189,10 @@ std::vector<RsChunk> rs_chunks(const mj_lfb* b, int half, const std::vector<char
 }
 
 int rs_check_err(mj_lfb* b, cudaStream_t s) {
-  int herr = 0;
-  MJ_CUDA(cudaMemcpyAsync(&herr, b->rs_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int* herr = b->op->h_status.as<int>();
+  MJ_CUDA(cudaMemcpyAsync(herr, b->rs_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
   MJ_CUDA(cudaStreamSynchronize(s));
-  if (herr) {
+  if (*herr) {
     cudaMemset(b->rs_err.ptr, 0, sizeof(int));
     cudaMemset(b->rs_sync.ptr, 0, sizeof(SyncState));
     set_error("mj_lfb_advance: a bounded wait of the step kernel timed out (state is invalid)");
@@ -420,9 +420,7 @@ int lfb_fused_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, b
     b->step++;
   }
   if (diag)
-    for (int r = 0; r < b->n_rec * b->S; r++)
-      MJ_CUDA(cudaMemcpyAsync(traces + (size_t)r * trace_stride, b->traces_d.as<double>() + (size_t)r * nsteps,
-                              sizeof(double) * nsteps, cudaMemcpyDeviceToHost, s));
+    if (int rc = lfb_copy_traces(b, nsteps, traces, trace_stride, s)) return rc;
   return rs_check_err(b, s);
 }
 
