@@ -168,16 +168,17 @@ __global__ void k_source_rhs(const int* __restrict__ idx, const int* __restrict_
   }
 }
 
-// Adjoint source: lam[d][s] += invD[d] * sum_{(k,w) at d} w * res[k][s][col]
-// over the dofs touched by receivers (rdof, CSR rptr/rk/rw).
+// Adjoint source: lam[d][s] += invD[d] * sum_{(k,w) at d} w * res[k][s]
+// over the dofs touched by receivers (rdof, CSR rptr/rk/rw); res: the
+// residual of one column.
 __global__ void k_inject_rhs(const int* __restrict__ rdof, const int* __restrict__ rptr, const int* __restrict__ rk,
-                             const double* __restrict__ rw, int n_rd, const double* __restrict__ res, int res_stride,
-                             int col, const double* __restrict__ inv_mass, float* __restrict__ lam, int S) {
+                             const double* __restrict__ rw, int n_rd, const double* __restrict__ res,
+                             const double* __restrict__ inv_mass, float* __restrict__ lam, int S) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_rd * S) return;
   const int i = t / S, s = t - i * S;
   double acc = 0.0;
-  for (int e = rptr[i]; e < rptr[i + 1]; e++) acc += rw[e] * res[((size_t)rk[e] * S + s) * res_stride + col];
+  for (int e = rptr[i]; e < rptr[i + 1]; e++) acc += rw[e] * res[(size_t)rk[e] * S + s];
   const int d = rdof[i];
   lam[(size_t)d * S + s] += (float)(inv_mass[d] * acc);
 }
@@ -213,16 +214,53 @@ __global__ void k_gather_init_rhs(const float* __restrict__ R, const int* __rest
 }
 
 // Receiver k, right-hand side s: sum_t W[k][t] U[idx[k][t]][s], FP64 sum;
-// written to out[(k*S + s)*stride + col].
-__global__ void k_receivers_rhs(const float* __restrict__ u, const int* __restrict__ idx,
-                                const double* __restrict__ w, int n_rec, int n_w, int S,
-                                double* __restrict__ out, int stride, int col) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_rec * S) return;
-  const int k = t / S, s = t - k * S;
+// written to out[(k*S + s)*stride + col].  A block takes one receiver and L
+// right-hand sides: its kRecThreads / L thread rows each sum every
+// (kRecThreads / L)-th weight, the row sums are added in row order.  Bound by
+// the latency of the gathered rows: one thread per (receiver, right-hand side)
+// walking all 125 (Q4) weights took 34 us per step for 64 receivers and 64 or
+// 16 right-hand sides, this split 8 us.
+constexpr int kRecThreads = 256;
+__global__ void __launch_bounds__(kRecThreads)
+    k_receivers_rhs(const float* __restrict__ u, const int* __restrict__ idx, const double* __restrict__ w, int n_w,
+                    int S, int L, double* __restrict__ out, int stride, int col) {
+  __shared__ double part[kRecThreads];
+  const int lane = threadIdx.x % L, row = threadIdx.x / L, rows = kRecThreads / L;
+  const int per = S / L, k = blockIdx.x / per, s = (blockIdx.x - k * per) * L + lane;
+  const int* ik = idx + (size_t)k * n_w;
+  const double* wk = w + (size_t)k * n_w;
   double acc = 0.0;
-  for (int a = 0; a < n_w; a++) acc += w[(size_t)k * n_w + a] * double(u[(size_t)idx[(size_t)k * n_w + a] * S + s]);
-  out[(size_t)t * stride + col] = acc;
+  int a = row;
+  for (; a + 3 * rows < n_w; a += 4 * rows) {
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) v[q] = __ldg(u + (size_t)__ldg(ik + a + q * rows) * S + s);
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc += __ldg(wk + a + q * rows) * double(v[q]);
+  }
+  for (; a < n_w; a += rows) acc += __ldg(wk + a) * double(__ldg(u + (size_t)__ldg(ik + a) * S + s));
+  part[threadIdx.x] = acc;
+  __syncthreads();
+  if (row == 0) {
+    for (int q = 1; q < rows; q++) acc += part[q * L + lane];
+    out[((size_t)k * S + s) * stride + col] = acc;
+  }
+}
+
+// out[c][r] = in[r][c] (FP64): the residual by column, so that the adjoint
+// source of a step reads contiguous rows.
+__global__ void __launch_bounds__(256)
+    k_transpose(const double* __restrict__ in, double* __restrict__ out, int rows, int cols) {
+  __shared__ double tile[32][33];
+  const int c0 = blockIdx.x * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int r0 = blockIdx.y * 32; r0 < rows; r0 += gridDim.y * 32) {
+    for (int q = y; q < 32; q += 8)
+      if (r0 + q < rows && c0 + x < cols) tile[q][x] = in[(size_t)(r0 + q) * cols + c0 + x];
+    __syncthreads();
+    for (int q = y; q < 32; q += 8)
+      if (c0 + q < cols && r0 + x < rows) out[(size_t)(c0 + q) * rows + r0 + x] = tile[x][q];
+    __syncthreads();
+  }
 }
 
 __global__ void k_cast_f64_to_f32(const double* __restrict__ a, float* __restrict__ b, long long n) {
@@ -240,13 +278,19 @@ int grid_for(long long n) {
 
 }  // namespace
 
+namespace {
+void receivers_launch(mj_lfb* b, const float* u, double* out, int stride, int col, cudaStream_t s) {
+  const int L = b->S % 32 == 0 ? 32 : b->S % 16 == 0 ? 16 : 8;  // S is a multiple of 8
+  k_receivers_rhs<<<b->n_rec * (b->S / L), kRecThreads, 0, s>>>(u, b->rec_idx.as<int>(), b->rec_w.as<double>(),
+                                                                b->n_rec_w, b->S, L, out, stride, col);
+  count_launch();
+}
+}  // namespace
+
 // Receiver values of every run before a step: out column `col` of
 // b->traces_d (stride = steps of the call).
 void lfb_receivers(mj_lfb* b, const float* u, int stride, int col, cudaStream_t s) {
-  const int threads = 128, blocks = (b->n_rec * b->S + threads - 1) / threads;
-  k_receivers_rhs<<<blocks, threads, 0, s>>>(u, b->rec_idx.as<int>(), b->rec_w.as<double>(), b->n_rec, b->n_rec_w,
-                                             b->S, b->traces_d.as<double>(), stride, col);
-  count_launch();
+  receivers_launch(b, u, b->traces_d.as<double>(), stride, col, s);
 }
 
 // Recorded traces to the host: one copy (one per run and receiver took 8 us
@@ -534,12 +578,7 @@ int mj_lfb_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, int 
     }
   }
   for (; done < nsteps; done++) {
-    if (diag) {
-      const int threads = 128, blocks = (b->n_rec * b->S + threads - 1) / threads;
-      k_receivers_rhs<<<blocks, threads, 0, s>>>(b->cur(), b->rec_idx.as<int>(), b->rec_w.as<double>(), b->n_rec,
-                                                 b->n_rec_w, b->S, b->traces_d.as<double>(), nsteps, done);
-      count_launch();
-    }
+    if (diag) lfb_receivers(b, b->cur(), nsteps, done, s);
     lfb_step_launch(b, b->cur(), b->next(), b->step & 1, s);
     b->cur_is_a = !b->cur_is_a;
     b->step++;
@@ -637,6 +676,7 @@ struct mj_adj {
   DevBuf seg;                        // K states of the segment being replayed
   DevBuf la, lb;                     // adjoint states
   DevBuf traces, res;                // n_rec x S x (N+1), FP64
+  DevBuf res_t;                      // the residual by column: (N+1) x n_rec x S
   DevBuf grad, coef;                 // per element (padded), FP64
   DevBuf rdof, rptr, rk, rw;         // receiver injection CSR
   int n_rd = 0;
@@ -657,20 +697,16 @@ struct mj_adj {
 namespace {
 
 void adj_receivers(mj_adj* a, const float* u, int col, cudaStream_t s) {
-  mj_lfb* b = a->b;
-  const int threads = 128, blocks = (b->n_rec * b->S + threads - 1) / threads;
-  k_receivers_rhs<<<blocks, threads, 0, s>>>(u, b->rec_idx.as<int>(), b->rec_w.as<double>(), b->n_rec, b->n_rec_w,
-                                             b->S, a->traces.as<double>(), a->N + 1, col);
-  count_launch();
+  receivers_launch(a->b, u, a->traces.as<double>(), a->N + 1, col, s);
 }
 
 // out = 2*u1 - u0 + dt^2 D^-1 (-A u1 + pulse[step] F): the forward update with
-// an explicit step index (pulse counter set on the host first).
+// an explicit step index.
 int adj_forward_step(mj_adj* a, const float* u0, const float* u1, float* out, int step, cudaStream_t s) {
   mj_lfb* b = a->b;
+  if (b->fused)  // the one-kernel step (bitwise the same arithmetic), the step index by value
+    return lfb_fused_step_on(b, const_cast<float*>(u0), const_cast<float*>(u1), out, step, s);
   MJ_CUDA(cudaMemcpyAsync(b->ctr.as<int>(), &step, sizeof(int), cudaMemcpyHostToDevice, s));
-  if (b->fused)  // the one-kernel step (bitwise the same arithmetic)
-    return lfb_fused_step_on(b, const_cast<float*>(u0), const_cast<float*>(u1), out, true, s);
   lfb_k1(b, u1, s);
   const long long total = (long long)b->n_dof * b->S;
   k_gather_leapfrog_rhs<<<grid_for(total), 256, 0, s>>>(b->R.as<float>(), b->op->ptr.as<int>(), b->ctr.as<int>(), 0,
@@ -777,7 +813,7 @@ int adj_visit(mj_adj* a, const float* um, int m, float*& lam1, float*& lam2, cud
     }
     if (!done) {
       if (um) adj_term(a, lam1, um, s);
-      const int rc = lfb_fused_step_on(b, lam2, lam1, lam2, false, s);
+      const int rc = lfb_fused_step_on(b, lam2, lam1, lam2, -1, s);
       if (rc) return rc;
     }
   } else {
@@ -790,8 +826,8 @@ int adj_visit(mj_adj* a, const float* um, int m, float*& lam1, float*& lam2, cud
   }
   const int inj_blocks = (a->n_rd * S + 127) / 128;
   k_inject_rhs<<<inj_blocks, 128, 0, s>>>(a->rdof.as<int>(), a->rptr.as<int>(), a->rk.as<int>(), a->rw.as<double>(),
-                                          a->n_rd, a->res.as<double>(), N + 1, m, b->inv_mass64.as<double>(), lam2,
-                                          S);
+                                          a->n_rd, a->res_t.as<double>() + (size_t)m * b->n_rec * S,
+                                          b->inv_mass64.as<double>(), lam2, S);
   count_launch();
   std::swap(lam1, lam2);  // lam1 = lambda^m, lam2 = lambda^{m+1}
   MJ_CUDA(cudaGetLastError());
@@ -846,6 +882,7 @@ int adj_common_init(mj_adj* a) {
   const size_t tr = (size_t)b->n_rec * b->S * (nsteps + 1);
   MJ_CUDA(a->traces.alloc(sizeof(double) * tr));
   MJ_CUDA(a->res.alloc(sizeof(double) * tr));
+  MJ_CUDA(a->res_t.alloc(sizeof(double) * tr));
   mj_op* op = b->op;
   MJ_CUDA(a->grad.alloc(sizeof(double) * op->n_elt_pad));
   MJ_CUDA(a->coef.alloc(sizeof(double) * op->n_elt_pad));
@@ -1068,6 +1105,10 @@ int mj_adj_backward(mj_adj* a, const double* residual, const double* coef, doubl
   const int N = a->N, K = a->K, S = b->S;
   const size_t rows = a->rows, bytes = sizeof(float) * rows;
   MJ_CUDA(cudaMemcpyAsync(a->res.ptr, residual, sizeof(double) * b->n_rec * S * (N + 1), cudaMemcpyHostToDevice, s));
+  const int rr = b->n_rec * S;
+  k_transpose<<<dim3((N + 1 + 31) / 32, std::min((rr + 31) / 32, 1024)), 256, 0, s>>>(a->res.as<double>(),
+                                                                                      a->res_t.as<double>(), rr, N + 1);
+  count_launch();
   std::vector<double> cf(op->n_elt_pad, 0.0);
   for (int e = 0; e < op->n_elt; e++) cf[e] = coef[e];
   MJ_CUDA(cudaMemcpyAsync(a->coef.ptr, cf.data(), sizeof(double) * cf.size(), cudaMemcpyHostToDevice, s));

@@ -122,8 +122,9 @@ struct mj_lfb {
   // shape, dof chunks, sources grouped by dof, barrier state, graphs by parity
   bool fused = true;
   int rs_variant = -1, rs_grid = 0, rs_threads = 0, rs_n_chunks = 0;
-  mj::DevBuf rs_chunks, rs_src_dof, rs_src_ptr, rs_src_rhs, rs_src_val, rs_sync, rs_err;
-  int rs_n_src_dof = 0;
+  mj::DevBuf rs_chunks, rs_src_ptr, rs_src_rhs, rs_src_val, rs_sync, rs_err;
+  int rs_zmap_key[3] = {0, 0, 0};  // (n, E, LB) that rs_zmap, the z-line order of a step's threads, was made for
+  unsigned char rs_zmap[mj::kMaxN * mj::kMaxN] = {};
   int rs_en_variant = -1, rs_en_grid = 0;  // the step's EN form (adjoint gradient term): for which variant, its grid
   cudaGraphExec_t rs_graph[2] = {nullptr, nullptr};
   std::vector<double> rs_tune_ms;
@@ -226,7 +227,7 @@ int lfb_fused_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, b
 int lfb_copy_traces(mj_lfb* b, int nsteps, double* traces, int trace_stride, cudaStream_t s);
 void lfb_receivers(mj_lfb* b, const float* u, int stride, int col, cudaStream_t s);
 int lfb_phase_ms(const mj_lfb* b, double* out);
-int lfb_fused_step_on(mj_lfb* b, float* u0, float* u1, float* out, bool sources, cudaStream_t s);
+int lfb_fused_step_on(mj_lfb* b, float* u0, float* u1, float* out, int step, cudaStream_t s);
 int lfb_fused_step(mj_lfb* b, cudaStream_t s, float* copy = nullptr);
 int lfb_fused_step_en(mj_lfb* b, float* u0, float* u1, float* out, const float* ue, double* gacc,
                       const double* gcoef, cudaStream_t s, bool* done);

@@ -154,7 +154,6 @@ RsParams rs_params(mj_lfb* b, const RsVariant& v) {
   p.m = b->m.as<float>();
   p.pulse = b->pulse.as<double>();
   p.ctr = b->ctr.as<int>();
-  p.src_dof = b->rs_src_dof.as<int>();
   p.src_ptr = b->rs_src_ptr.as<int>();
   p.src_rhs = b->rs_src_rhs.as<int>();
   p.src_val = b->rs_src_val.as<float>();
@@ -163,11 +162,17 @@ RsParams rs_params(mj_lfb* b, const RsVariant& v) {
   p.ue = nullptr;
   p.gacc = nullptr;
   p.gcoef = nullptr;
-  p.n_src_dof = b->rs_n_src_dof;
   p.n_pulse = b->n_pulse;
   p.S = b->S;
   p.n_tiles = op->n_elt_pad / v.E;
-  rs_zline_order(v.n, v.E, v.LB, p.zmap);
+  p.step = -1;
+  if (b->rs_zmap_key[0] != v.n || b->rs_zmap_key[1] != v.E || b->rs_zmap_key[2] != v.LB) {
+    rs_zline_order(v.n, v.E, v.LB, b->rs_zmap);
+    b->rs_zmap_key[0] = v.n;
+    b->rs_zmap_key[1] = v.E;
+    b->rs_zmap_key[2] = v.LB;
+  }
+  std::copy(b->rs_zmap, b->rs_zmap + kMaxNK * kMaxNK, p.zmap);
   return p;
 }
 
@@ -227,27 +232,21 @@ int lfb_fused_setup(mj_lfb* b) {
   std::vector<int> order(b->n_src);
   for (int t = 0; t < b->n_src; t++) order[t] = t;
   std::sort(order.begin(), order.end(), [&](int x, int y) { return si[x] != si[y] ? si[x] < si[y] : sr[x] < sr[y]; });
-  std::vector<int> dofs, dptr, rhs;
+  std::vector<int> dptr((size_t)op->n_dof + 1, 0), rhs;
   std::vector<float> val;
   std::vector<char> is_src(op->n_dof, 0);
   for (int t = 0; t < b->n_src; t++) {
     const int e = order[t];
-    if (dofs.empty() || dofs.back() != si[e]) {
-      dofs.push_back(si[e]);
-      dptr.push_back((int)rhs.size());
-    }
     rhs.push_back(sr[e]);
     val.push_back(sv[e]);
     is_src[si[e]] = 1;
+    dptr[si[e] + 1]++;
   }
-  dptr.push_back((int)rhs.size());
-  b->rs_n_src_dof = (int)dofs.size();
-  MJ_CUDA(b->rs_src_dof.alloc(sizeof(int) * std::max<size_t>(1, dofs.size())));
+  for (int d = 0; d < op->n_dof; d++) dptr[d + 1] += dptr[d];
   MJ_CUDA(b->rs_src_ptr.alloc(sizeof(int) * dptr.size()));
   MJ_CUDA(b->rs_src_rhs.alloc(sizeof(int) * std::max<size_t>(1, rhs.size())));
   MJ_CUDA(b->rs_src_val.alloc(sizeof(float) * std::max<size_t>(1, val.size())));
-  if (!dofs.empty()) {
-    MJ_CUDA(cudaMemcpy(b->rs_src_dof.ptr, dofs.data(), sizeof(int) * dofs.size(), cudaMemcpyHostToDevice));
+  if (!rhs.empty()) {
     MJ_CUDA(cudaMemcpy(b->rs_src_rhs.ptr, rhs.data(), sizeof(int) * rhs.size(), cudaMemcpyHostToDevice));
     MJ_CUDA(cudaMemcpy(b->rs_src_val.ptr, val.data(), sizeof(float) * val.size(), cudaMemcpyHostToDevice));
   }
@@ -425,17 +424,18 @@ int lfb_fused_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, b
 }
 
 // One step of the one-kernel form on caller-given states: U^n = u0,
-// U^{n+1} = u1, U^{n+2} written to out (out may be u0); the pulse index is
-// ctr[0] (set by the caller), sources only when `sources`.  Used by the
-// adjoint's checkpoint replays and its adjoint steps.
-int lfb_fused_step_on(mj_lfb* b, float* u0, float* u1, float* out, bool sources, cudaStream_t s) {
+// U^{n+1} = u1, U^{n+2} written to out (out may be u0); step: the pulse
+// index, or -1 for a step without sources.  The integrator's own counter
+// stays as it is.  Used by the adjoint's checkpoint replays and its adjoint
+// steps.
+int lfb_fused_step_on(mj_lfb* b, float* u0, float* u1, float* out, int step, cudaStream_t s) {
   const RsVariant& v = rs_variants()[b->rs_variant];
   RsParams prm = rs_params(b, v);
   prm.ua = u0;
   prm.ub = u1;
   prm.uout = out;
-  if (!sources) {
-    prm.n_src_dof = 0;
+  prm.step = std::max(step, 0);
+  if (step < 0) {
     prm.n_pulse = 0;
   }
   return rs_launch(v, b->rs_grid, prm, b->rs_chunks.as<RsChunk>(), b->rs_n_chunks, b->rs_sync.as<SyncState>(), 0,
@@ -462,8 +462,8 @@ int lfb_fused_step_en(mj_lfb* b, float* u0, float* u1, float* out, const float* 
   prm.ua = u0;
   prm.ub = u1;
   prm.uout = out;
-  prm.n_src_dof = 0;
   prm.n_pulse = 0;
+  prm.step = 0;
   prm.ue = ue;
   prm.gacc = gacc;
   prm.gcoef = gcoef;

@@ -24,8 +24,7 @@ struct RsParams {
   const float* m;     // dt^2 / D (padded)
   const double* pulse;
   int* ctr;
-  const int* src_dof;  // dofs carrying sources, sorted
-  const int* src_ptr;  // their entries [src_ptr[i], src_ptr[i+1]) in
+  const int* src_ptr;  // source entries of dof d: [src_ptr[d], src_ptr[d+1]) in
   const int* src_rhs;  //   (right-hand side, value) pairs
   const float* src_val;
   float* uout;         // where U^{n+2} goes (nullptr: over U^n)
@@ -35,7 +34,8 @@ struct RsParams {
   const float* ue;
   double* gacc;
   const double* gcoef;
-  int n_src_dof, n_pulse, S, n_tiles;
+  int n_pulse, S, n_tiles;
+  int step;            // the step's pulse index, or -1: ctr[par], and ctr[1-par] = ctr[par] + 1 after it
   unsigned char zmap[kMaxNK * kMaxNK];  // z-line (j*n + i) of each thread slot of an element (rs_zline_order)
 };
 
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(RsPlan<N, E, LB, V>::T, rs_min_ctas(RsPlan<N, 
   float* __restrict__ cur = par == 0 ? p.ua : p.ub;        // U^n, overwritten by U^{n+2}
   const float* __restrict__ nxt = par == 0 ? p.ub : p.ua;  // U^{n+1}
   // step counters: ctr[1-par] = ctr[par] + 1 (phase 2 reads ctr[par] only)
-  if (blockIdx.x == 0 && t == 0) p.ctr[1 - par] = p.ctr[par] + 1;
+  if (p.step < 0 && blockIdx.x == 0 && t == 0) p.ctr[1 - par] = p.ctr[par] + 1;
   // optional phase time stamps of this CTA: start, phase 1 done, barrier passed, end
   if (stamps && t == 0) stamps[4 * blockIdx.x] = global_ns();
 
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(RsPlan<N, E, LB, V>::T, rs_min_ctas(RsPlan<N, 
 
   // ---- phase 2
   float* __restrict__ dst = p.uout ? p.uout : cur;
-  const int step = p.ctr[par];
+  const int step = p.step >= 0 ? p.step : p.ctr[par];
   const bool pulse_on = step < p.n_pulse;
   const float pf = pulse_on ? (float)p.pulse[step] : 0.f;
   const int S4 = S >> 2;
@@ -430,17 +430,13 @@ __global__ void __launch_bounds__(RsPlan<N, E, LB, V>::T, rs_min_ctas(RsPlan<N, 
       un[2] = 2.f * a1.z - a0.z + md * (-y.z);
       un[3] = 2.f * a1.w - a0.w + md * (-y.w);
       if (ch.has_src && pulse_on) {
-        int lo = 0, hi = p.n_src_dof - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (__ldg(p.src_dof + mid) < d) lo = mid + 1;
-          else hi = mid;
+        // offsets per dof: a binary search over the source dofs took 16
+        // dependent loads per item (13 us of a 64 us step at 16^3 Q4 with 16 sources)
+        const int e1 = __ldg(p.src_ptr + d + 1);
+        for (int e = __ldg(p.src_ptr + d); e < e1; e++) {
+          const int r = __ldg(p.src_rhs + e);
+          if ((r >> 2) == c4) un[r & 3] += md * pf * __ldg(p.src_val + e);
         }
-        if (__ldg(p.src_dof + lo) == d)
-          for (int e = __ldg(p.src_ptr + lo); e < __ldg(p.src_ptr + lo + 1); e++) {
-            const int r = __ldg(p.src_rhs + e);
-            if ((r >> 2) == c4) un[r & 3] += md * pf * __ldg(p.src_val + e);
-          }
       }
       const float4 o = make_float4(un[0], un[1], un[2], un[3]);
       *reinterpret_cast<float4*>(dst + (size_t)d * S + 4 * c4) = o;
