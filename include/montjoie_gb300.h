@@ -260,11 +260,13 @@ int mj_lf_set_graph(mj_lf* lf, int enable);
  * for order 2. */
 int mj_lf_set_scheme(mj_lf* lf, int order, int n_pulse_d2, const double* pulse_d2);
 
-/* FP32 order-2 step: with enable != 0 (the default for MJ_FP32) the gather,
- * update and source run as one streaming kernel that stages each chunk of
- * dofs (states, dt^2/D, CSR offsets, contributions) in shared memory by bulk
- * copy; enable = 0 uses a gather kernel and a separate source kernel.  Both
- * give the same states bit for bit. */
+/* Order-2 step: the gather, update and source run as one streaming kernel that
+ * stages each chunk of dofs (states, masses, CSR offsets, contributions) in
+ * shared memory by bulk copy, with the norm and the receivers of the new
+ * iterate when they are asked for; enable = 0 uses a gather kernel and
+ * separate source and diagnostics kernels.  FP32: both give the same states
+ * bit for bit, and enable != 0 (the default) selects the first again.  FP64:
+ * equal up to rounding; enable != 0 is refused (MJ_ERR_ARG). */
 int mj_lf_set_stream_gather(mj_lf* lf, int enable);
 
 /* Divergence guard: mj_lf_advance / mj_lf_run return MJ_ERR_NONFINITE (with

@@ -86,9 +86,11 @@ struct mj_lf {
   mj::DevBuf w4, z4, d3_4;
   mj::DevBuf src_mask, src_sidx, src_sval;
   int n_src_sorted = 0;
-  // FP32 order-2 step: streaming gather (k_gather_leapfrog_stream) over dof chunks
-  bool stream_gather = false;
+  // order-2 step: streaming gather (k_gather_leapfrog_stream, FP64: ..._stream64) over dof chunks
+  bool stream_gather = false;  // FP32
+  bool stream64 = false;       // FP64
   mj::DevBuf stream_chunks;
+  mj::DevBuf m64, stream_lists;  // FP64: dt^2/D, and each chunk's dofs with several contributions
   int n_stream_chunks = 0, stream_grid_ = 0;
   ~mj_lf() {
     for (cudaEvent_t e : ev) cudaEventDestroy(e);

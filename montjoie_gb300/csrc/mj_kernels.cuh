@@ -336,14 +336,15 @@ struct DiagDev {
   int stride, col, ncols;
 };
 
-// Norm and receivers of the new iterate, fused into the streaming gather
-// (FP32): weights rounded to FP32, one partial per CTA, the finished-CTA
+// Norm and receivers of the new iterate, fused into the streaming gathers
+// (FP32: weights rounded to FP32), one partial per CTA, the finished-CTA
 // counter (zero between launches), the non-finite flag, the receivers, and
 // where to write: (dd ? *dd : direct), column where.col + col.
 struct StreamDiag {
   const float* w32;    // the FP32 norm weights, or NULL: weights = wdt2 / m (norm weights equal to the mass)
   const float* m;      // dt^2/D (k_stream_diag, with w32 == NULL)
   float wdt2;          // dt^2 in FP32 (w32 == NULL), else 0; 0 with w32 == NULL: no norm
+  const double* w64;   // FP64 integrators: the norm weights, or NULL
   double* partial;
   unsigned* done;
   int* flag;
@@ -357,7 +358,9 @@ struct StreamDiag {
 
 struct StreamChunk {
   int d0, d1, q0, q1;  // dofs [d0, d1); R range [q0, q1) rounded to multiples of 4
-  int has_src, pad0, pad1, pad2;
+  int has_src;
+  int n_multi;         // FP64: dofs with two or more contributions (the chunk's list)
+  int pad1, pad2;
 };
 
 // One dof's term of the fused norm, rounded the same way wherever it is
@@ -370,7 +373,8 @@ __device__ __forceinline__ float stream_norm_term(float w, float u, float acc) {
 // block tree of the threads' sums, one partial per CTA; the last CTA to
 // finish adds the partials in a fixed order and samples the receivers from
 // the finished state u.
-__device__ __forceinline__ void stream_diag_finish(double nacc, const StreamDiag& dg, const float* u, int G) {
+template <typename Real>
+__device__ __forceinline__ void stream_diag_finish(double nacc, const StreamDiag& dg, const Real* u, int G) {
   __shared__ double sh[kStreamThreads / 32];
   __shared__ bool last;
   const int t = threadIdx.x;
@@ -421,7 +425,7 @@ __device__ __forceinline__ void stream_diag_finish(double nacc, const StreamDiag
         int q = lane;
         for (; q + 32 < dg.n_w; q += 2 * 32) {
           const int i0 = idx[q], i1 = idx[q + 32];
-          const float u0v = __ldcg(u + i0), u1v = __ldcg(u + i1);
+          const Real u0v = __ldcg(u + i0), u1v = __ldcg(u + i1);
           acc += wr[q] * double(u0v);
           acc += wr[q + 32] * double(u1v);
         }
@@ -530,6 +534,165 @@ __global__ void __launch_bounds__(kStreamThreads, 8)  // 8 CTAs per SM: 32 regis
     }
   }
   if constexpr (DIAG) stream_diag_finish(nacc, dg, u0, G);
+}
+
+// K2s in FP64: the streaming gather + update + source,
+//   u^{n+2} = 2 u^{n+1} - u^n + m Ah,  m = dt^2 / D,
+// for integrators whose 1/D is the reciprocal of D (others keep the reference's
+// order of operations in k_gather_leapfrog: the two agree up to rounding, and
+// this one is closer to the exact update, which D * (1/D) != 1 disturbs there).
+// A chunk's u^{n+1}, u^n, m, CSR offsets, contributions and its dofs with two
+// or more contributions, sorted by their number, are staged; one dof per
+// thread.  What bounds it is HBM (52 B per dof) and the FP64 pipe, which takes
+// 16 clocks per warp instruction and SM whatever the active lanes: the sums
+// run over the sorted list, so that a warp's dofs have equal numbers of
+// additions (a warp of neighbouring dofs runs as many as its largest, 3 to 7,
+// for 0.93 on average), and the update takes two operations.  64^3 Q4
+// (17.0 M dofs): gather and source kernels 355 us, this form with the
+// reference's order and unsorted sums 343, as it is 138 (0.94 of the measured
+// copy bandwidth). With the source kernel and, in the DIAG form, the norm and
+// receivers inside, a step is two launches.
+constexpr int kStream64Dofs = 256;
+constexpr int kStream64U0 = kStream64Dofs * 8, kStream64M = 2 * kStream64U0;
+constexpr int kStream64P = 3 * kStream64U0;
+constexpr int kStream64L = kStream64P + (kStream64Dofs + 8) * 4;
+constexpr int kStream64R = kStream64L + kStream64Dofs;
+constexpr int kStream64Buf = 12544;
+constexpr int kStream64RCap = (kStream64Buf - kStream64R) / 8;
+constexpr int kStream64Smem = kStreamNB * kStream64Buf + 8 * kStreamNB;
+static_assert(kStream64P % 16 == 0 && kStream64L % 16 == 0 && kStream64R % 16 == 0 && kStream64Buf % 16 == 0,
+              "aligned buffer segments");
+static_assert(kStream64Dofs == kStreamThreads, "one dof per thread");
+
+template <bool DIAG>
+__global__ void __launch_bounds__(kStreamThreads, 7)
+    k_gather_leapfrog_stream64(const double* __restrict__ R, const int* __restrict__ ptr, int* __restrict__ ctr,
+                               int qc, double* __restrict__ u0, const double* __restrict__ u1,
+                               const double* __restrict__ m, const StreamChunk* __restrict__ chunks, int n_chunks,
+                               const unsigned char* __restrict__ lists, const unsigned* __restrict__ mask,
+                               const int* __restrict__ sidx, const double* __restrict__ sval, int nsrc,
+                               const double* __restrict__ pulse, int n_pulse, int* __restrict__ err, StreamDiag dg) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kStreamNB * kStream64Buf);
+  const int t = threadIdx.x, G = gridDim.x;
+  if (blockIdx.x == 0 && t == 0) ctr[1 - qc] = ctr[qc] + 1;
+  const int step = ctr[qc];
+  const bool src_on = nsrc > 0 && step < n_pulse;
+  const double p = src_on ? pulse[step] : 0.0;
+  auto issue = [&](int c, int b) {
+    if (c >= n_chunks) return;
+    const StreamChunk ch = chunks[c];
+    unsigned char* dst = smem + b * kStream64Buf;
+    const uint32_t sb = (uint32_t)(((ch.d1 - ch.d0 + 3) & ~3) * 8);
+    const uint32_t pb = (uint32_t)(((ch.d1 - ch.d0 + 1 + 3) & ~3) * 4);
+    const uint32_t rb = (uint32_t)((ch.q1 - ch.q0) * 8);
+    mbar_expect_tx(&bar[b], 3u * sb + pb + rb + kStream64Dofs);
+    const uint64_t pol = l2_evict_first_policy();
+    bulk_g2s_hint(dst, u1 + ch.d0, sb, &bar[b], pol);
+    bulk_g2s_hint(dst + kStream64U0, u0 + ch.d0, sb, &bar[b], pol);
+    bulk_g2s_hint(dst + kStream64M, m + ch.d0, sb, &bar[b], pol);
+    bulk_g2s_hint(dst + kStream64P, ptr + ch.d0, pb, &bar[b], pol);
+    bulk_g2s_hint(dst + kStream64L, lists + (size_t)c * kStream64Dofs, kStream64Dofs, &bar[b], pol);
+    bulk_g2s_hint(dst + kStream64R, R + ch.q0, rb, &bar[b], pol);
+  };
+  if (t == 0) {
+    for (int b = 0; b < kStreamNB; b++) mbar_init(&bar[b], 1);
+    fence_mbar_init();
+    for (int b = 0; b < kStreamNB; b++) issue(blockIdx.x + b * G, b);
+  }
+  __syncthreads();
+  uint32_t ph = 0u;  // bit b: parity of buffer b's next completion
+  int b = 0;
+  double nacc = 0.0;  // DIAG: this thread's sum of w u^2
+  for (int c = blockIdx.x; c < n_chunks; c += G, b = (b + 1 == kStreamNB ? 0 : b + 1)) {
+    const StreamChunk ch = chunks[c];
+    const bool ok = mbar_wait_bounded(&bar[b], (ph >> b) & 1u);
+    if (__syncthreads_or(!ok)) {
+      // report, wait (bounded) for this CTA's copies still in flight, and
+      // still take part in the diagnostics' finished-CTA count
+      if (t == 0) atomicExch(err, 1);
+      for (int i = 0, cb = b; i < kStreamNB; i++, cb = (cb + 1 == kStreamNB ? 0 : cb + 1))
+        if (c + i * G < n_chunks) mbar_wait_drain(&bar[cb], (ph >> cb) & 1u);
+      break;
+    }
+    ph ^= 1u << b;
+    unsigned char* buf = smem + b * kStream64Buf;
+    const double* su1 = reinterpret_cast<const double*>(buf);
+    const int* sp = reinterpret_cast<const int*>(buf + kStream64P);
+    double* sR = reinterpret_cast<double*>(buf + kStream64R) - ch.q0;
+    if (t < ch.n_multi) {  // this thread's listed dof: its sum in CSR order, over its first contribution
+      const int dl = buf[kStream64L + t];
+      const int qa = sp[dl], qb = sp[dl + 1];
+      double s = sR[qa];
+      for (int q = qa + 1; q < qb; q++) s += sR[q];
+      sR[qa] = s;
+    }
+    __syncthreads();
+    const int d = ch.d0 + t;
+    if (d < ch.d1) {
+      const double md = su1[2 * kStream64Dofs + t];
+      double un = fma(-md, sR[sp[t]], fma(2.0, su1[t], -su1[kStream64Dofs + t]));
+      if (src_on && ch.has_src) {
+        const double f = source_at(mask, sidx, sval, nsrc, d);
+        if (f != 0.0) un = un + md * p * f;
+      }
+      u0[d] = un;
+      if (DIAG && dg.w64) nacc = fma(__ldg(dg.w64 + d) * un, un, nacc);
+    }
+    __syncthreads();  // buffer b is free
+    if (t == 0) {
+      fence_proxy_async();
+      issue(c + kStreamNB * G, b);
+    }
+  }
+  if constexpr (DIAG) stream_diag_finish(nacc, dg, u0, G);
+}
+
+// Set-up of the FP64 streaming gather: every chunk's list (one CTA per chunk,
+// one dof per thread: its place is the number of dofs with more contributions,
+// or as many and a lower number) and its length.
+__global__ void __launch_bounds__(kStream64Dofs)
+    k_chunk_lists(StreamChunk* __restrict__ chunks, const int* __restrict__ ptr, unsigned char* __restrict__ lists) {
+  __shared__ int deg[kStream64Dofs];
+  StreamChunk& ch = chunks[blockIdx.x];
+  const int t = threadIdx.x, n = ch.d1 - ch.d0;
+  const int mine = t < n ? ptr[ch.d0 + t + 1] - ptr[ch.d0 + t] : 0;
+  deg[t] = mine;
+  const int multi = __syncthreads_count(mine >= 2);
+  unsigned char* l = lists + (size_t)blockIdx.x * kStream64Dofs;
+  int at = 0;
+  for (int q = 0; q < n; q++) at += deg[q] > mine || (deg[q] == mine && q < t);
+  if (mine >= 2) l[at] = (unsigned char)t;
+  if (t == 0) ch.n_multi = multi;
+}
+
+// m = dt^2 inv; *other is set when inv is not the reciprocal of D somewhere.
+__global__ void k_dt2_over_mass(const double* __restrict__ inv, const double* __restrict__ mass, double dt2,
+                                double* __restrict__ m, int n, int* __restrict__ other) {
+  for (int d = blockIdx.x * blockDim.x + threadIdx.x; d < n; d += gridDim.x * blockDim.x) {
+    const double v = dt2 * inv[d];
+    m[d] = v;
+    if (!(fabs(inv[d] * mass[d] - 1.0) <= 1e-15) || !isfinite(v)) *other = 1;
+  }
+}
+
+// k_stream_diag (below) for FP64 states: the chunks, grid and arithmetic of
+// k_gather_leapfrog_stream64<true>.
+__global__ void __launch_bounds__(kStreamThreads)
+    k_stream_diag64(const double* __restrict__ u, const StreamChunk* __restrict__ chunks, int n_chunks,
+                    StreamDiag dg) {
+  const int G = gridDim.x;
+  double nacc = 0.0;
+  if (dg.w64)
+    for (int c = blockIdx.x; c < n_chunks; c += G) {
+      const StreamChunk ch = chunks[c];
+      const int d = ch.d0 + threadIdx.x;
+      if (d < ch.d1) {
+        const double v = __ldg(u + d);
+        nacc = fma(__ldg(dg.w64 + d) * v, v, nacc);
+      }
+    }
+  stream_diag_finish(nacc, dg, u, G);
 }
 
 // The order-4 gathers of the FP32 form as streaming kernels, on the chunks,

@@ -779,10 +779,15 @@ int lf_sorted_sources(mj_lf* lf) {
 }
 
 // Dof chunks of the streaming gather: start on a multiple of 4, at most
-// kStreamDofs dofs, the 16-byte rounded range of their contributions within
-// kStreamRCap; then the launch shape.
-int lf_stream_setup(mj_lf* lf) {
+// kStreamDofs (FP64: kStream64Dofs) dofs, the 16-byte rounded range of their
+// contributions within kStreamRCap (kStream64RCap); then the launch shape.
+// FP64: false in *fits when some dof has too many contributions for a chunk.
+int lf_stream_setup(mj_lf* lf, bool* fits = nullptr) {
   const mj_op* op = lf->op;
+  const bool f64 = op->precision == MJ_FP64;
+  const int max_dofs = f64 ? kStream64Dofs : kStreamDofs, cap = f64 ? kStream64RCap : kStreamRCap;
+  const int smem = f64 ? kStream64Smem : kStreamSmem;
+  if (fits) *fits = true;
   const std::vector<int>& ptr = op->h_ptr;
   std::vector<char> is_src(op->n_dof, 0);
   {
@@ -793,10 +798,14 @@ int lf_stream_setup(mj_lf* lf) {
   }
   std::vector<StreamChunk> chunks;
   for (int d = 0; d < op->n_dof;) {
-    int e = std::min(op->n_dof, d + kStreamDofs);
+    int e = std::min(op->n_dof, d + max_dofs);
     auto range = [&](int e2) { return ((ptr[e2] + 3) & ~3) - (ptr[d] & ~3); };
-    while (range(e) > kStreamRCap) e = d + std::max(4, ((e - d) / 2) & ~3);
-    if (range(e) > kStreamRCap) {
+    while (range(e) > cap && e - d > 4) e = d + std::max(4, ((e - d) / 2) & ~3);
+    if (range(e) > cap && fits) {
+      *fits = false;
+      return MJ_OK;
+    }
+    if (range(e) > cap) {
       set_error("streaming gather: a dof has too many contributions for one chunk buffer");
       return MJ_ERR_ARG;
     }
@@ -809,13 +818,26 @@ int lf_stream_setup(mj_lf* lf) {
   MJ_CUDA(cudaMemcpy(lf->stream_chunks.ptr, chunks.data(), sizeof(StreamChunk) * chunks.size(),
                      cudaMemcpyHostToDevice));
   lf->n_stream_chunks = (int)chunks.size();
-  MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kStreamSmem));
-  MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kStreamSmem));
+  if (f64) {
+    MJ_CUDA(lf->stream_lists.alloc(chunks.size() * kStream64Dofs));
+    MJ_CUDA(cudaMemsetAsync(lf->stream_lists.ptr, 0, lf->stream_lists.bytes, op->stream));
+    k_chunk_lists<<<(int)chunks.size(), kStream64Dofs, 0, op->stream>>>(
+        lf->stream_chunks.as<StreamChunk>(), op->ptr.as<int>(), lf->stream_lists.as<unsigned char>());
+    count_launch();
+    MJ_CUDA(cudaGetLastError());
+  }
   int ctas = 0;
-  MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_gather_leapfrog_stream<false>, kStreamThreads,
-                                                        kStreamSmem));
+  if (f64) {
+    MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_gather_leapfrog_stream64<true>, kStreamThreads,
+                                                          smem));
+  } else {
+    MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_gather_leapfrog_stream<false>, kStreamThreads,
+                                                          smem));
+  }
   MJ_CHECK_ARG(ctas >= 1, "streaming gather cannot be resident");
   lf->stream_grid_ = std::max(1, std::min(lf->n_stream_chunks, ctas * sm_count()));
   MJ_CUDA(lf->stream_partial.alloc(sizeof(double) * lf->stream_grid_));
@@ -872,7 +894,7 @@ int mj_lf_create(mj_op* op, const mj_lf_desc* desc, mj_lf** out) {
     MJ_CUDA(lf->mass.alloc(sizeof(double) * n));
     MJ_CUDA(lf->minv.alloc(sizeof(double) * n));
     MJ_CUDA(cudaMemcpy(lf->mass.ptr, desc->mass, sizeof(double) * n, cudaMemcpyHostToDevice));
-    MJ_CUDA(cudaMemcpy(lf->minv.ptr, invD.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+    MJ_CUDA(cudaMemcpy(lf->minv.ptr, lf->inv_mass64.ptr, sizeof(double) * n, cudaMemcpyDeviceToDevice));
   } else {
     std::vector<float> sv(std::max(1, desc->n_src)), m(n);
     for (int s = 0; s < desc->n_src; s++) sv[s] = (float)desc->src_val[s];
@@ -927,6 +949,24 @@ int mj_lf_create(mj_op* op, const mj_lf_desc* desc, mj_lf** out) {
     if (!rc) rc = lf_stream_setup(lf.get());
     if (rc) return rc;
     lf->stream_gather = true;
+  } else {
+    // the streaming form when 1/D is the reciprocal of D (a caller's own array may be something else);
+    // m64 padded by 4 entries like the states (16-byte rounded bulk copies)
+    DevBuf other;
+    int h_other = 0;
+    MJ_CUDA(other.alloc(sizeof(int)));
+    MJ_CUDA(cudaMemset(other.ptr, 0, sizeof(int)));
+    MJ_CUDA(lf->m64.alloc(sizeof(double) * (n + 4)));
+    MJ_CUDA(cudaMemset(lf->m64.ptr, 0, sizeof(double) * (n + 4)));
+    k_dt2_over_mass<<<stream_grid(n), 256>>>(lf->inv_mass64.as<double>(), lf->mass.as<double>(), desc->dt * desc->dt,
+                                             lf->m64.as<double>(), n, other.as<int>());
+    count_launch();
+    MJ_CUDA(cudaMemcpy(&h_other, other.ptr, sizeof(int), cudaMemcpyDeviceToHost));
+    if (!h_other) {
+      int rc = lf_sorted_sources(lf.get());
+      if (!rc) rc = lf_stream_setup(lf.get(), &lf->stream64);
+      if (rc) return rc;
+    }
   }
   *out = lf.release();
   return MJ_OK;
@@ -1034,7 +1074,7 @@ constexpr int kGraphSteps = 20;
 // Kernels one step launches (launch accounting of graph replays).
 int lf_kernels_per_step(const mj_lf* lf) {
   if (lf->time_order == 4) return 4;
-  if (lf->stream_gather && lf->op->precision == MJ_FP32) return 2;
+  if (lf->op->precision == MJ_FP32 ? lf->stream_gather : lf->stream64) return 2;
   return 2 + (lf->n_src > 0);
 }
 
@@ -1081,10 +1121,10 @@ void lf_step4_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_
   }
 }
 
-// Diagnostics fused into the step: the FP32 order-2 step with the streaming
+// Diagnostics fused into the step: the order-2 step with the streaming
 // gather computes the norm and the receivers of the iterate it produces.
 bool lf_fused_diag(const mj_lf* lf) {
-  return lf->stream_gather && lf->op->precision == MJ_FP32 && lf->time_order == 2;
+  return (lf->op->precision == MJ_FP32 ? lf->stream_gather : lf->stream64) && lf->time_order == 2;
 }
 
 // dg: the step's fused diagnostics (streaming gather only), or nullptr.
@@ -1108,6 +1148,21 @@ void lf_step_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_t
         static_cast<const float*>(next), lf->minv.as<float>(), lf->stream_chunks.as<StreamChunk>(),
         lf->n_stream_chunks, lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<float>(),
         lf->n_src_sorted, lf->pulse_d.as<double>(), lf->n_pulse, lf->inv_mass64.as<double>(), dt2,
+        op->err.as<int>(), dg ? *dg : StreamDiag{});
+    count_launch();
+    if (prof) {
+      cudaEventRecord(lf->ev[lf->ev_used + 2], s);
+      lf->ev_used += 3;
+    }
+    return;
+  }
+  if (op->precision == MJ_FP64 && lf->stream64) {
+    auto k2 = dg ? k_gather_leapfrog_stream64<true> : k_gather_leapfrog_stream64<false>;
+    k2<<<lf->stream_grid_, kStreamThreads, kStream64Smem, s>>>(
+        op->R.as<double>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, static_cast<double*>(cur),
+        static_cast<const double*>(next), lf->m64.as<double>(), lf->stream_chunks.as<StreamChunk>(),
+        lf->n_stream_chunks, lf->stream_lists.as<unsigned char>(), lf->src_mask.as<unsigned>(),
+        lf->src_sidx.as<int>(), lf->src_sval.as<double>(), lf->n_src_sorted, lf->pulse_d.as<double>(), lf->n_pulse,
         op->err.as<int>(), dg ? *dg : StreamDiag{});
     count_launch();
     if (prof) {
@@ -1147,6 +1202,7 @@ StreamDiag lf_stream_diag(mj_lf* lf, const DiagDev* dd, DiagDev direct, int col)
   g.w32 = from_m ? nullptr : lf->norm_w32.as<float>();
   g.m = lf->minv.as<float>();
   g.wdt2 = from_m ? (float)(lf->dt * lf->dt) : 0.f;
+  g.w64 = lf->norm_w.as<double>();
   g.partial = lf->stream_partial.as<double>();
   g.done = lf->diag_done.as<unsigned>();
   g.flag = lf->flag.as<int>();
@@ -1266,9 +1322,13 @@ int lf_advance_impl(mj_lf* lf, int nsteps, double* norms, double* traces, int st
   if (fused)  // iterates 0 and 1 with the same arithmetic as the fused steps
     for (int c = 0; c < std::min(cols, 2); c++) {
       const StreamDiag dg = lf_stream_diag(lf, nullptr, direct, c);
-      k_stream_diag<<<lf->stream_grid_, kStreamThreads, 0, lf->stream>>>(
-          static_cast<const float*>(c == 0 ? lf->cur() : lf->next()), lf->stream_chunks.as<StreamChunk>(),
-          lf->n_stream_chunks, dg);
+      const void* u = c == 0 ? lf->cur() : lf->next();
+      if (sizeof(Real) == 8)
+        k_stream_diag64<<<lf->stream_grid_, kStreamThreads, 0, lf->stream>>>(
+            static_cast<const double*>(u), lf->stream_chunks.as<StreamChunk>(), lf->n_stream_chunks, dg);
+      else
+        k_stream_diag<<<lf->stream_grid_, kStreamThreads, 0, lf->stream>>>(
+            static_cast<const float*>(u), lf->stream_chunks.as<StreamChunk>(), lf->n_stream_chunks, dg);
       count_launch();
     }
   if ((nd || td) && !lf->profile && lf->use_graph && nsteps >= kGraphSteps + 1) {
@@ -1459,7 +1519,8 @@ int mj_lf_set_stream_gather(mj_lf* lf, int enable) {
       cudaGraphExecDestroy(*g);
       *g = nullptr;
     }
-  lf->stream_gather = enable != 0;
+  if (lf->op->precision == MJ_FP32) lf->stream_gather = enable != 0;
+  else lf->stream64 = false;
   return MJ_OK;
 }
 
