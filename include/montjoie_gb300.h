@@ -142,7 +142,9 @@ int mj_op_info(const mj_op* op, int* order, int* n_elt, int* n_dof, int* precisi
  * plus the rank and no slot array is read; 4 compact with one factor stage:
  * the next tile's factors are copied during the current tile's divergence,
  * so a CTA holds one factor block instead of two; 5 fixed point, the kernel of
- * MJ_FP64 operators: two-limb integer products instead of the FP64 pipe), grid; and the timings (ms per launch,
+ * MJ_FP64 operators: two-limb integer products instead of the FP64 pipe; 6
+ * line owner, FP32 orders 7 and 8: a thread computes whole lines of the
+ * gradient), grid; and the timings (ms per launch,
  * or a negative occupancy score on meshes too small to time) of the
  * candidates tried (candidate_ms may be NULL, else room for 64 values). */
 int mj_op_tuning(const mj_op* op, int* tile_elems, int* vector_lines, int* grid, int* n_candidates,

@@ -17,6 +17,7 @@ struct mj_op {
   bool warp = false;                    // warp-per-element layout (FP32, order 4; autotuned)
   bool packed = false;                  // that layout with packed connectivity (nodle_pk; autotuned)
   bool fs = false;                      // compact layout with one factor stage (FP32; autotuned)
+  bool ln = false;                      // line-owner layout (FP32, mj_k1_ln.cu; autotuned)
   bool fx = false;                      // fixed-point kernel (FP64, mj_k1_fx.cuh)
   bool fx_sym = false;                  // its form for matrices antisymmetric under the mirror
   size_t r_len = 0;                     // element-major slots (n_elt_pad * Qp)
@@ -171,6 +172,12 @@ std::vector<int> k1_warp_tile_candidates(int n);
 int k1_set_gmat_fs(int n, const double* g);  // called by k1_set_gmat_f32
 int k1_prepare_fs_f32(int n, int E, int* ctas_per_sm);
 void k1_launch_fs_f32(int n, int E, int grid, const void* x, const int* nodle_e, const void* fac_e, void* R,
+                      const int* slot_e, int n_tiles, int* err, cudaStream_t s);
+// Line-owner layout (FP32, mj_k1_ln.cu), its own tile sizes.
+std::vector<int> k1_ln_tile_candidates(int n);
+int k1_set_gmat_ln(int n, const double* g);  // called by k1_set_gmat_f32
+int k1_prepare_ln_f32(int n, int E, int* ctas_per_sm);
+void k1_launch_ln_f32(int n, int E, int grid, const void* x, const int* nodle_e, const void* fac_e, void* R,
                       const int* slot_e, int n_tiles, int* err, cudaStream_t s);
 int k1_prepare_w_f32(int n, int E, bool packed, int* ctas_per_sm);
 void k1_launch_w_f32(int n, int E, bool packed, int grid, const void* x, const int* nodle_e, const void* fac_e,

@@ -96,6 +96,12 @@ void launch_k1(mj_op* op, const void* x, cudaStream_t s) {
     count_launch();
     return;
   }
+  if (op->ln) {
+    k1_launch_ln_f32(op->n, op->E, op->grid_k1, x, op->nodle_e.as<int>(), op->fac_e.ptr, op->R.ptr,
+                     op->slot_e.as<int>(), op->n_tiles, op->err.as<int>(), s);
+    count_launch();
+    return;
+  }
   if (op->warp) {
     k1_launch_w_f32(op->n, op->E, op->packed, op->grid_k1, x, (op->packed ? op->nodle_pk : op->nodle_e).as<int>(),
                     op->fac_e.ptr, op->R.ptr, (op->packed ? op->ptr : op->slot_e).as<int>(), op->n_tiles,
@@ -140,7 +146,7 @@ int autotune_k1(mj_op* op) {
   MJ_CUDA(cudaEventCreate(&e1));
   double best = 1e300;
   int bestE = -1, bestGrid = 1;
-  bool bestVec = false, bestWarp = false, bestPacked = false, bestFs = false, bestFx = false;
+  bool bestVec = false, bestWarp = false, bestPacked = false, bestFs = false, bestFx = false, bestLn = false;
   const bool time_it = (long long)op->n_elt * op->Q >= 2000000;
   // layouts: 0 compact, 1 vector lines, 2 one element per warp, 3 the same
   // with packed connectivity, 4 compact with one factor stage (2-4: FP32), 5 fixed point (FP64: always where the
@@ -151,13 +157,17 @@ int autotune_k1(mj_op* op) {
     layouts = {0, 1, 2};
     if (op->nodle_pk.ptr) layouts.push_back(3);
     layouts.push_back(4);
+    layouts.push_back(6);
   }
   for (int lay : layouts)
-    for (int E : ((lay == 2 || lay == 3) ? k1_warp_tile_candidates(op->n) : cands)) {
+    for (int E : (lay == 6                ? k1_ln_tile_candidates(op->n)
+                  : lay == 2 || lay == 3 ? k1_warp_tile_candidates(op->n)
+                                         : cands)) {
       const bool vec = lay == 1, warp = lay == 2 || lay == 3, packed = lay == 3, fs = lay == 4;
-      const bool fx = lay == 5;
+      const bool fx = lay == 5, ln = lay == 6;
       int ctas = 0;
       const int rc = fx ? k1_prepare_fx(op, E, &ctas)
+                     : ln ? k1_prepare_ln_f32(op->n, E, &ctas)
                      : warp ? k1_prepare_w_f32(op->n, E, packed, &ctas)
                      : fs ? k1_prepare_fs_f32(op->n, E, &ctas)
                           : op->precision == MJ_FP64 ? k1_prepare_f64(op->n, E, vec, &ctas)
@@ -167,7 +177,7 @@ int autotune_k1(mj_op* op) {
       const int grid = std::max(1, std::min(tiles, ctas * sms));
       double ms = 0.0;
       if (time_it) {
-        op->E = E; op->vec = vec; op->warp = warp; op->packed = packed; op->fs = fs; op->fx = fx;
+        op->E = E; op->vec = vec; op->warp = warp; op->packed = packed; op->fs = fs; op->fx = fx; op->ln = ln;
         op->grid_k1 = grid;
         op->n_tiles = tiles;
         launch_k1(op, x.ptr, op->stream);
@@ -180,7 +190,8 @@ int autotune_k1(mj_op* op) {
         ms = f / 3.0;
       } else {
         ms = -double(ctas) * E * op->n * op->n + (vec ? 0.5 : 0.0) + (warp ? 0.75 : 0.0) +
-             (packed ? 0.1 : 0.0) + (fs ? 0.25 : 0.0);  // most resident threads first
+             (packed ? 0.1 : 0.0) + (fs ? 0.25 : 0.0) -
+             (ln ? 1e4 : 0.0);  // the line-owner layout where it exists (orders 7, 8), else most resident threads
       }
       op->tune_E.push_back(E);
       op->tune_vec.push_back(lay);
@@ -188,6 +199,7 @@ int autotune_k1(mj_op* op) {
       if (ms < best) {
         best = ms; bestE = E; bestGrid = grid; bestVec = vec; bestWarp = warp; bestPacked = packed; bestFs = fs;
         bestFx = fx;
+        bestLn = ln;
       }
     }
   cudaEventDestroy(e0);
@@ -202,11 +214,13 @@ int autotune_k1(mj_op* op) {
   op->packed = bestPacked;
   op->fs = bestFs;
   op->fx = bestFx;
+  op->ln = bestLn;
   op->grid_k1 = bestGrid;
   // the chosen variant's shared-memory attribute must be the one set last
   {
     int ctas = 0;
     const int rc = bestFx ? k1_prepare_fx(op, bestE, &ctas)
+                   : bestLn ? k1_prepare_ln_f32(op->n, bestE, &ctas)
                    : bestWarp ? k1_prepare_w_f32(op->n, bestE, bestPacked, &ctas)
                    : bestFs ? k1_prepare_fs_f32(op->n, bestE, &ctas)
                             : op->precision == MJ_FP64 ? k1_prepare_f64(op->n, bestE, bestVec, &ctas)
@@ -660,7 +674,7 @@ int mj_op_tuning(const mj_op* op, int* tile_elems, int* vector_lines, int* grid,
                  double* candidate_ms) {
   MJ_CHECK_ARG(op, "mj_op_tuning: null operator");
   if (tile_elems) *tile_elems = op->E;
-  if (vector_lines) *vector_lines = op->fx ? 5 : op->fs ? 4 : op->packed ? 3 : op->warp ? 2 : op->vec ? 1 : 0;
+  if (vector_lines) *vector_lines = op->ln ? 6 : op->fx ? 5 : op->fs ? 4 : op->packed ? 3 : op->warp ? 2 : op->vec ? 1 : 0;
   if (grid) *grid = op->grid_k1;
   if (n_candidates) *n_candidates = (int)op->tune_ms.size();
   if (candidate_ms)
@@ -690,7 +704,7 @@ int mj_op_set_variant(mj_op* op, int tile_elems, int vector_lines) {
   op->warp = warp;
   op->packed = packed;
   op->fs = fs;
-  op->fx = false;
+  op->fx = op->ln = false;
   op->n_tiles = op->n_elt_pad / tile_elems;
   op->grid_k1 = std::max(1, std::min(op->n_tiles, ctas * sm_count()));
   return MJ_OK;

@@ -125,7 +125,7 @@ class FemMatrixFreeOperator:
         E, lay, grid, nc = (v.value for v in vals)
         return {"tile_elems": E,
                 "layout": ["compact", "vector_lines", "warp_per_element", "warp_per_element_packed",
-                           "compact_one_factor_stage", "fixed_point"][lay],
+                           "compact_one_factor_stage", "fixed_point", "line_owner"][lay],
                 "grid": grid, "candidate_ms": ms[:nc].tolist()}
 
     def set_variant(self, tile_elems: int, layout) -> None:
