@@ -213,38 +213,34 @@ __global__ void k_gather_init_rhs(const float* __restrict__ R, const int* __rest
   }
 }
 
-// Receiver k, right-hand side s: sum_t W[k][t] U[idx[k][t]][s], FP64 sum;
-// written to out[(k*S + s)*stride + col].  A block takes one receiver and L
-// right-hand sides: its kRecThreads / L thread rows each sum every
-// (kRecThreads / L)-th weight, the row sums are added in row order.  Bound by
-// the latency of the gathered rows: one thread per (receiver, right-hand side)
-// walking all 125 (Q4) weights took 34 us per step for 64 receivers and 64 or
-// 16 right-hand sides, this split 8 us.
-constexpr int kRecThreads = 256;
+// Receiver k, right-hand side s: sum_t W[k][t] U[idx[k][t]][s], an FP64 sum in
+// the order of t; written to out[(k*S + s)*stride + col].  A block takes one
+// receiver and L right-hand sides: all its threads gather a chunk of the
+// weights' rows into shared memory, then one thread per right-hand side adds
+// them in order (the order is fixed: an adjoint's residuals, and so its FP32
+// sources, hang on the last bit).  The gathers' latency is what it costs: one thread per
+// (receiver, right-hand side) gathering its 125 (Q4) rows as it went took
+// 34 us per step for 64 receivers and 64 or 16 right-hand sides, this 12 us.
+constexpr int kRecThreads = 256, kRecChunk = 128;
 __global__ void __launch_bounds__(kRecThreads)
     k_receivers_rhs(const float* __restrict__ u, const int* __restrict__ idx, const double* __restrict__ w, int n_w,
                     int S, int L, double* __restrict__ out, int stride, int col) {
-  __shared__ double part[kRecThreads];
+  __shared__ double sv[kRecChunk * 32];
+  __shared__ double sw[kRecChunk];
   const int lane = threadIdx.x % L, row = threadIdx.x / L, rows = kRecThreads / L;
   const int per = S / L, k = blockIdx.x / per, s = (blockIdx.x - k * per) * L + lane;
-  const int* ik = idx + (size_t)k * n_w;
-  const double* wk = w + (size_t)k * n_w;
   double acc = 0.0;
-  int a = row;
-  for (; a + 3 * rows < n_w; a += 4 * rows) {
-    float v[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) v[q] = __ldg(u + (size_t)__ldg(ik + a + q * rows) * S + s);
-#pragma unroll
-    for (int q = 0; q < 4; q++) acc += __ldg(wk + a + q * rows) * double(v[q]);
+  for (int t0 = 0; t0 < n_w; t0 += kRecChunk) {
+    const int m = min(kRecChunk, n_w - t0);
+    const size_t at = (size_t)k * n_w + t0;
+    if (t0) __syncthreads();  // the previous chunk has been added
+    for (int a = row; a < m; a += rows) sv[a * L + lane] = double(__ldg(u + (size_t)__ldg(idx + at + a) * S + s));
+    for (int a = threadIdx.x; a < m; a += kRecThreads) sw[a] = __ldg(w + at + a);
+    __syncthreads();
+    if (row == 0)
+      for (int a = 0; a < m; a++) acc += sw[a] * sv[a * L + lane];
   }
-  for (; a < n_w; a += rows) acc += __ldg(wk + a) * double(__ldg(u + (size_t)__ldg(ik + a) * S + s));
-  part[threadIdx.x] = acc;
-  __syncthreads();
-  if (row == 0) {
-    for (int q = 1; q < rows; q++) acc += part[q * L + lane];
-    out[((size_t)k * S + s) * stride + col] = acc;
-  }
+  if (row == 0) out[((size_t)k * S + s) * stride + col] = acc;
 }
 
 // out[c][r] = in[r][c] (FP64): the residual by column, so that the adjoint
