@@ -126,6 +126,12 @@ struct mj_lfb {
   bool fused = true;
   int rs_variant = -1, rs_grid = 0, rs_threads = 0, rs_n_chunks = 0;
   mj::DevBuf rs_chunks, rs_src_ptr, rs_src_rhs, rs_src_val, rs_sync, rs_err;
+  // the plane form's dof phase: its chunks' segments, the dofs it updates, and
+  // the sources at the others (RpParams)
+  mj::DevBuf rs_segs, rs_mi, rs_mk, rs_pk, rs_dk, rs_fix, rs_fix_val;
+  std::vector<int> rs_h_dk, rs_h_pk;
+  int rs_n_fix = 0;
+  bool rs_interior = false;
   int rs_zmap_key[3] = {0, 0, 0};  // (n, E, LB) that rs_zmap, the z-line order of a step's threads, was made for
   unsigned char rs_zmap[mj::kMaxN * mj::kMaxN] = {};
   int rs_en_variant = -1, rs_en_grid = 0;  // the step's EN form (adjoint gradient term): for which variant, its grid

@@ -10,6 +10,8 @@
 //            once (8- or 16-byte loads) and the factors are read once per V.
 //            The operation order per right-hand side is that of
 //            k_local_stiffness_rhs; results go to the dof-ordered R.
+//            (The plane form of the step, mj_rhs_plane.cuh, splits this phase
+//            by planes instead.)
 //   barrier  grid-wide, bounded (cooperative launch; mj_sync.cuh);
 //   phase 2  dof chunks: u^{n+1}, u^n rows, the chunk's contiguous block of
 //            R rows, dt^2/D and the CSR offsets arrive by bulk copy (two
@@ -89,19 +91,26 @@ void rs_zline_order(int n, int E, int LB, unsigned char* out) {
 
 struct RsVariant {
   int n, E, LB, V, threads, smem, half;
+  bool plane;  // the plane form (mj_rhs_plane.cuh)
 };
 
 const std::vector<RsVariant>& rs_variants() {
-  static const std::vector<RsVariant> v = {
-#define MJ_X(N_, E_, LB_, V_)                                                                          \
-  {N_, E_, LB_, V_, RsPlan<N_, E_, LB_, V_>::T, RsPlan<N_, E_, LB_, V_>::kSmem, RsPlan<N_, E_, LB_, V_>::kHalf},
-      MJ_RS_VARIANTS(MJ_X)
+  static const std::vector<RsVariant> v = [] {
+    std::vector<RsVariant> all = {
+#define MJ_X(N_, E_, LB_, V_)                                                                                    \
+  {N_, E_, LB_, V_, RsPlan<N_, E_, LB_, V_>::T, RsPlan<N_, E_, LB_, V_>::kSmem, RsPlan<N_, E_, LB_, V_>::kHalf, \
+   false},
+        MJ_RS_VARIANTS(MJ_X)
 #undef MJ_X
-  };
+    };
+    for (const RpVariant& r : rp_variants()) all.push_back({r.n, r.E, r.LB, r.V, r.threads, 0, r.half, true});
+    return all;
+  }();
   return v;
 }
 
-int rs_prepare(const RsVariant& v, int* ctas) {
+int rs_prepare(const RsVariant& v, int S, int* ctas) {
+  if (v.plane) return rp_prepare(v.n, v.E, v.LB, v.V, false, S, ctas);
 #define MJ_X(N_, E_, LB_, V_)                                                                               \
   if (v.n == N_ && v.E == E_ && v.LB == LB_ && v.V == V_) {                                                 \
     MJ_CUDA(cudaFuncSetAttribute(k_rhs_step<N_, E_, LB_, V_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
@@ -116,8 +125,27 @@ int rs_prepare(const RsVariant& v, int* ctas) {
   return MJ_ERR_ARG;
 }
 
-int rs_launch(const RsVariant& v, int grid, const RsParams& prm, const RsChunk* chunks, int n_chunks,
-              SyncState* sync, int par, int* err, cudaStream_t s, unsigned long long* stamps = nullptr) {
+// A candidate's chunk lists (segs: the plane form's).
+struct RsLists {
+  DevBuf chunks, segs;
+  int n_chunks = 0;
+};
+
+RpParams rp_params(const mj_lfb* b, const DevBuf& chunks, const DevBuf& segs, int n_chunks) {
+  return {chunks.as<RpChunk>(),  segs.as<RpSeg>(),    b->rs_mi.as<float>(),
+          b->rs_mk.as<float>(),  b->rs_pk.as<int>(),  b->rs_dk.as<int>(),
+          b->rs_fix.as<int>(),   b->rs_fix_val.as<float>(), n_chunks,
+          b->rs_n_fix,           b->op->n_elt,        b->rs_interior ? 1 : 0};
+}
+
+int rs_launch(const mj_lfb* b, const RsVariant& v, int grid, const RsParams& prm, const DevBuf& chunk_list,
+              const DevBuf& segs, int n_chunks, int par, cudaStream_t s, unsigned long long* stamps = nullptr) {
+  SyncState* sync = b->rs_sync.as<SyncState>();
+  int* err = b->rs_err.as<int>();
+  const RsChunk* chunks = chunk_list.as<RsChunk>();
+  if (v.plane)
+    return rp_launch(v.n, v.E, v.LB, v.V, false, grid, prm, rp_params(b, chunk_list, segs, n_chunks), sync, par, err,
+                     s, stamps);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(v.threads);
@@ -166,6 +194,7 @@ RsParams rs_params(mj_lfb* b, const RsVariant& v) {
   p.S = b->S;
   p.n_tiles = op->n_elt_pad / v.E;
   p.step = -1;
+  if (v.plane) return p;  // reads no z-line order
   if (b->rs_zmap_key[0] != v.n || b->rs_zmap_key[1] != v.E || b->rs_zmap_key[2] != v.LB) {
     rs_zline_order(v.n, v.E, v.LB, b->rs_zmap);
     b->rs_zmap_key[0] = v.n;
@@ -193,6 +222,134 @@ std::vector<RsChunk> rs_chunks(const mj_lfb* b, int half, const std::vector<char
   return out;
 }
 
+// The dofs the plane form's dof phase updates (rs_h_dk, their first
+// contribution rows rs_h_pk, device copies): all but the elements' interior
+// ones, or all of them where an interior point shares its dof or the interior
+// dofs are numbered in runs too short for the segments; and the sources at
+// the dofs left out.  Order 3 and up: an order-2 element has one interior
+// dof in eight of its own.
+int rp_kept(mj_lfb* b, const std::vector<int>& dptr, const std::vector<int>& rhs, const std::vector<float>& val) {
+  mj_op* op = b->op;
+  const int n_dof = op->n_dof;
+  std::vector<char> in(n_dof, 0);
+  b->rs_interior = false;
+  if (op->n >= 4) {
+    DevBuf flag;
+    MJ_CUDA(flag.alloc(sizeof(int) + n_dof));
+    MJ_CUDA(cudaMemsetAsync(flag.ptr, 0, sizeof(int) + n_dof, b->stream));
+    if (int rc = rp_mark_interior(op->nodle_e.as<int>(), op->ptr.as<int>(), op->n_elt, op->n,
+                                  flag.as<char>() + sizeof(int), flag.as<int>(), b->stream))
+      return rc;
+    int bad = 0;
+    MJ_CUDA(cudaMemcpyAsync(&bad, flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+    MJ_CUDA(cudaMemcpyAsync(in.data(), flag.as<char>() + sizeof(int), n_dof, cudaMemcpyDeviceToHost, b->stream));
+    MJ_CUDA(cudaStreamSynchronize(b->stream));
+    long long kept = 0, runs = 0;
+    for (int d = 0; d < n_dof; d++)
+      if (!in[d]) {
+        kept++;
+        runs += d == 0 || in[d - 1];
+      }
+    b->rs_interior = !bad && kept >= 4 * runs;
+    if (b->rs_interior) {
+      const int I = op->n - 2;
+      MJ_CUDA(b->rs_mi.alloc(sizeof(float) * (size_t)op->n_elt_pad * ((I * I * I + 3) / 4 * 4)));
+      if (int rc = rp_interior_mass(op->nodle_e.as<int>(), b->m.as<float>(), op->n_elt, op->n_elt_pad, op->n,
+                                    b->rs_mi.as<float>(), b->stream))
+        return rc;
+    } else {
+      std::fill(in.begin(), in.end(), 0);
+    }
+  }
+  std::vector<int>&dk = b->rs_h_dk, &pk = b->rs_h_pk;
+  dk.clear();
+  pk.assign(1, 0);
+  std::vector<int> fix;
+  std::vector<float> fix_val, mk, m(n_dof);
+  MJ_CUDA(cudaMemcpy(m.data(), b->m.ptr, sizeof(float) * n_dof, cudaMemcpyDeviceToHost));
+  for (int d = 0; d < n_dof; d++) {
+    if (!in[d]) {
+      dk.push_back(d);
+      mk.push_back(m[d]);
+      pk.push_back(pk.back() + op->h_ptr[d + 1] - op->h_ptr[d]);
+      continue;
+    }
+    for (int e = dptr[d]; e < dptr[d + 1]; e++) {
+      fix.push_back(d);
+      fix.push_back(rhs[e]);
+      fix_val.push_back(val[e]);
+    }
+  }
+  b->rs_n_fix = (int)fix_val.size();
+  auto upload = [](DevBuf& dst, const void* src, size_t bytes, size_t pad) {
+    MJ_CUDA(dst.alloc(bytes + pad));
+    MJ_CUDA(cudaMemset(dst.ptr, 0, bytes + pad));
+    if (bytes) MJ_CUDA(cudaMemcpy(dst.ptr, src, bytes, cudaMemcpyHostToDevice));
+    return MJ_OK;
+  };
+  if (int rc = upload(b->rs_mk, mk.data(), sizeof(float) * mk.size(), 32)) return rc;
+  if (int rc = upload(b->rs_pk, pk.data(), sizeof(int) * pk.size(), 32)) return rc;
+  if (int rc = upload(b->rs_dk, dk.data(), sizeof(int) * dk.size(), 32)) return rc;
+  if (int rc = upload(b->rs_fix, fix.data(), sizeof(int) * fix.size(), 32)) return rc;
+  return upload(b->rs_fix_val, fix_val.data(), sizeof(float) * fix_val.size(), 32);
+}
+
+// Chunks and segments of a plane variant: as many kept dofs as fit a buffer
+// of half bytes (<= 512, <= kRpMaxSegs runs of consecutive dofs).
+bool rp_chunks(const mj_lfb* b, int half, const std::vector<char>& is_src, std::vector<RpChunk>& out,
+               std::vector<RpSeg>& segs) {
+  const std::vector<int>&dk = b->rs_h_dk, &pk = b->rs_h_pk;
+  const int n = (int)dk.size();
+  for (int i0 = 0; i0 < n;) {
+    if (rp_buf(i0, i0 + 1, pk[i0 + 1] - pk[i0], b->S).end > half) return false;
+    RpChunk ch = {i0, i0, (int)segs.size(), 0, 0, 0, 0, 0};
+    for (int i = i0; i < n && i - i0 < 512 && rp_buf(i0, i + 1, pk[i + 1] - pk[i0], b->S).end <= half; i++) {
+      const int nq = pk[i + 1] - pk[i];
+      if (i == i0 || dk[i] != dk[i - 1] + 1) {
+        if ((int)segs.size() - ch.s0 == kRpMaxSegs) break;
+        segs.push_back({dk[i], 0, b->op->h_ptr[dk[i]], 0, i - i0, pk[i] - pk[i0], 0, 0});
+      }
+      segs.back().nd++;
+      segs.back().nq += nq;
+      ch.i1 = i + 1;
+      ch.has_src |= is_src[dk[i]];
+    }
+    ch.s1 = (int)segs.size();
+    ch.rows = pk[ch.i1] - pk[i0];
+    out.push_back(ch);
+    i0 = ch.i1;
+  }
+  return true;
+}
+
+// The chunk lists of variant v on the device; L.n_chunks = 0 when a dof has
+// too many contributions for one buffer.
+int rs_lists(const mj_lfb* b, const RsVariant& v, const std::vector<char>& is_src, RsLists& L) {
+  std::vector<RsChunk> ch;
+  std::vector<RpChunk> pch;
+  std::vector<RpSeg> segs;
+  L.n_chunks = 0;
+  if (v.plane ? !rp_chunks(b, v.half, is_src, pch, segs) : (ch = rs_chunks(b, v.half, is_src)).empty()) return MJ_OK;
+  const void* src = v.plane ? (const void*)pch.data() : ch.data();
+  const size_t bytes = v.plane ? sizeof(RpChunk) * pch.size() : sizeof(RsChunk) * ch.size();
+  MJ_CUDA(L.chunks.alloc(bytes));
+  MJ_CUDA(cudaMemcpy(L.chunks.ptr, src, bytes, cudaMemcpyHostToDevice));
+  if (v.plane) {
+    MJ_CUDA(L.segs.alloc(sizeof(RpSeg) * segs.size()));
+    MJ_CUDA(cudaMemcpy(L.segs.ptr, segs.data(), sizeof(RpSeg) * segs.size(), cudaMemcpyHostToDevice));
+  }
+  L.n_chunks = (int)(v.plane ? pch.size() : ch.size());
+  return MJ_OK;
+}
+
+void rs_use_lists(mj_lfb* b, RsLists& L) {
+  std::swap(b->rs_chunks.ptr, L.chunks.ptr);
+  std::swap(b->rs_chunks.bytes, L.chunks.bytes);
+  std::swap(b->rs_segs.ptr, L.segs.ptr);
+  std::swap(b->rs_segs.bytes, L.segs.bytes);
+  b->rs_n_chunks = L.n_chunks;
+}
+
 int rs_check_err(mj_lfb* b, cudaStream_t s) {
   int* herr = b->op->h_status.as<int>();
   MJ_CUDA(cudaMemcpyAsync(herr, b->rs_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -210,7 +367,9 @@ int rs_check_err(mj_lfb* b, cudaStream_t s) {
 
 // Sources grouped by dof, chunk lists per candidate, and the variant choice:
 // each candidate of the order runs 3 steps (after one warm-up) on the
-// integrator's state, which mj_lfb_init resets afterwards.  Leaves
+// integrator's state, which mj_lfb_init resets afterwards.  The z-line
+// variants are tried only where no plane variant runs (the plane form's list
+// holds only variants faster than the best of them, mj_rhs_plane.cuh).  Leaves
 // b->fused = false when no variant fits (S too large for a chunk buffer).
 int lfb_fused_setup(mj_lfb* b) {
   mj_op* op = b->op;
@@ -220,6 +379,7 @@ int lfb_fused_setup(mj_lfb* b) {
     for (int a = 0; a < op->n * op->n; a++) v[a] = (float)op->gradphi[a];
     MJ_CUDA(cudaMemcpyToSymbol(c_gmat32, v, sizeof(float) * op->n * op->n, sizeof(float) * kMaxNK * kMaxNK * op->n));
     if (int rc = rs_en_set_gmat(op->n, v)) return rc;
+    if (int rc = rp_set_gmat(op->n, v)) return rc;
   }
   // sources grouped by dof: sorted (dof, rhs) pairs from the device copies
   std::vector<int> si(b->n_src), sr(b->n_src);
@@ -268,27 +428,32 @@ int lfb_fused_setup(mj_lfb* b) {
   const uint64_t before = launch_counter().load();
   double best = 1e300;
   int bi = -1;
-  std::vector<DevBuf> lists(all.size());
-  std::vector<int> counts(all.size(), 0), grids(all.size(), 0);
-  for (size_t c = 0; c < all.size(); c++) {
+  std::vector<RsLists> lists(all.size());
+  std::vector<int> grids(all.size(), 0);
+  bool planes = false;  // a plane variant runs
+  std::vector<size_t> tried(all.size());
+  for (size_t c = 0; c < all.size(); c++) tried[c] = c;
+  std::stable_partition(tried.begin(), tried.end(), [&](size_t c) { return all[c].plane; });
+  for (size_t c : tried) {
     const RsVariant& v = all[c];
+    if (!v.plane && planes) continue;
     if (v.n != op->n || b->S % (v.LB * v.V) != 0) continue;
     if (rs_buf(3, 4, 0, 8, b->S).end > v.half) continue;  // one dof (up to 8 contributions) must fit
     int ctas = 0;
-    if (rs_prepare(v, &ctas) != MJ_OK || ctas < 1) continue;
-    const std::vector<RsChunk> ch = rs_chunks(b, v.half, is_src);
-    if (ch.empty()) continue;  // a dof with too many contributions for one buffer
-    MJ_CUDA(lists[c].alloc(sizeof(RsChunk) * ch.size()));
-    MJ_CUDA(cudaMemcpy(lists[c].ptr, ch.data(), sizeof(RsChunk) * ch.size(), cudaMemcpyHostToDevice));
-    counts[c] = (int)ch.size();
-    grids[c] = ctas * sm_count();
+    if (rs_prepare(v, b->S, &ctas) != MJ_OK || ctas < 1) continue;
+    if (v.plane && b->rs_h_dk.empty())
+      if (int rc = rp_kept(b, dptr, rhs, val)) return rc;
+    if (int rc = rs_lists(b, v, is_src, lists[c])) return rc;
+    if (!lists[c].n_chunks) continue;
+    planes |= v.plane;
     const RsParams prm = rs_params(b, v);
-    int rc = rs_launch(v, grids[c], prm, lists[c].as<RsChunk>(), counts[c], b->rs_sync.as<SyncState>(), 0,
-                       b->rs_err.as<int>(), b->stream);
+    grids[c] = ctas * sm_count();
+    auto run = [&](int k) {
+      return rs_launch(b, v, grids[c], prm, lists[c].chunks, lists[c].segs, lists[c].n_chunks, k & 1, b->stream);
+    };
+    int rc = run(0);
     if (!rc) rc = cudaEventRecord(e0, b->stream) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
-    for (int k = 1; !rc && k <= 3; k++)
-      rc = rs_launch(v, grids[c], prm, lists[c].as<RsChunk>(), counts[c], b->rs_sync.as<SyncState>(), k & 1,
-                     b->rs_err.as<int>(), b->stream);
+    for (int k = 1; !rc && k <= 3; k++) rc = run(k);
     if (!rc) rc = cudaEventRecord(e1, b->stream) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
     if (!rc) rc = rs_check_err(b, b->stream);
     float ms = 0.f;
@@ -312,10 +477,7 @@ int lfb_fused_setup(mj_lfb* b) {
   b->rs_variant = bi;
   b->rs_threads = all[bi].threads;
   b->rs_grid = grids[bi];
-  b->rs_n_chunks = counts[bi];
-  b->rs_chunks.release();
-  std::swap(b->rs_chunks.ptr, lists[bi].ptr);
-  std::swap(b->rs_chunks.bytes, lists[bi].bytes);
+  rs_use_lists(b, lists[bi]);
   b->fused = true;
   return MJ_OK;
 }
@@ -339,24 +501,24 @@ int lfb_set_step_variant(mj_lfb* b, int E, int LB, int V) {
     return MJ_ERR_ARG;
   }
   int ctas = 0;
-  if (int rc = rs_prepare(v, &ctas)) return rc;
+  if (int rc = rs_prepare(v, b->S, &ctas)) return rc;
   std::vector<char> is_src(op->n_dof, 0);
   if (b->n_src) {
     std::vector<int> si(b->n_src);
     MJ_CUDA(cudaMemcpy(si.data(), b->src_idx.ptr, sizeof(int) * b->n_src, cudaMemcpyDeviceToHost));
     for (int d : si) is_src[d] = 1;
   }
-  const std::vector<RsChunk> ch = rs_chunks(b, v.half, is_src);
-  if (ch.empty() || ctas < 1) {
+  RsLists lists;
+  if (ctas >= 1 && !(v.plane && b->rs_h_dk.empty()))
+    if (int rc = rs_lists(b, v, is_src, lists)) return rc;
+  if (!lists.n_chunks) {
     set_error("mj_lfb_set_step_variant: the variant does not fit this integrator");
     return MJ_ERR_ARG;
   }
-  MJ_CUDA(b->rs_chunks.alloc(sizeof(RsChunk) * ch.size()));
-  MJ_CUDA(cudaMemcpy(b->rs_chunks.ptr, ch.data(), sizeof(RsChunk) * ch.size(), cudaMemcpyHostToDevice));
+  rs_use_lists(b, lists);
   b->rs_variant = c;
   b->rs_threads = v.threads;
   b->rs_grid = ctas * sm_count();
-  b->rs_n_chunks = (int)ch.size();
   for (auto& g : b->rs_graph)
     if (g) {
       cudaGraphExecDestroy(g);
@@ -377,8 +539,7 @@ int lfb_fused_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, b
   if (prof && b->rs_stamps.bytes < sizeof(unsigned long long) * 4 * b->rs_grid)
     MJ_CUDA(b->rs_stamps.alloc(sizeof(unsigned long long) * 4 * b->rs_grid));
   auto launch = [&](int par, cudaStream_t st) {
-    return rs_launch(v, b->rs_grid, prm, b->rs_chunks.as<RsChunk>(), b->rs_n_chunks, b->rs_sync.as<SyncState>(),
-                     par, b->rs_err.as<int>(), st,
+    return rs_launch(b, v, b->rs_grid, prm, b->rs_chunks, b->rs_segs, b->rs_n_chunks, par, st,
                      prof ? b->rs_stamps.as<unsigned long long>() : (unsigned long long*)nullptr);
   };
   int done = 0;
@@ -438,8 +599,7 @@ int lfb_fused_step_on(mj_lfb* b, float* u0, float* u1, float* out, int step, cud
   if (step < 0) {
     prm.n_pulse = 0;
   }
-  return rs_launch(v, b->rs_grid, prm, b->rs_chunks.as<RsChunk>(), b->rs_n_chunks, b->rs_sync.as<SyncState>(), 0,
-                   b->rs_err.as<int>(), s);
+  return rs_launch(b, v, b->rs_grid, prm, b->rs_chunks, b->rs_segs, b->rs_n_chunks, 0, s);
 }
 
 // lfb_fused_step_on without sources, in the EN form: also
@@ -453,7 +613,9 @@ int lfb_fused_step_en(mj_lfb* b, float* u0, float* u1, float* out, const float* 
   const RsVariant& v = rs_variants()[b->rs_variant];
   if (b->rs_en_variant != b->rs_variant) {
     int ctas = 0;
-    if (int rc = rs_en_prepare(v.n, v.E, v.LB, v.V, b->S, &ctas)) return rc;
+    const int rc = v.plane ? rp_prepare(v.n, v.E, v.LB, v.V, true, b->S, &ctas)
+                           : rs_en_prepare(v.n, v.E, v.LB, v.V, b->S, &ctas);
+    if (rc) return rc;
     b->rs_en_variant = b->rs_variant;
     b->rs_en_grid = ctas * sm_count();
   }
@@ -467,8 +629,12 @@ int lfb_fused_step_en(mj_lfb* b, float* u0, float* u1, float* out, const float* 
   prm.ue = ue;
   prm.gacc = gacc;
   prm.gcoef = gcoef;
-  const int rc = rs_en_launch(v.n, v.E, v.LB, v.V, b->S, b->rs_en_grid, prm, b->rs_chunks.as<RsChunk>(),
-                              b->rs_n_chunks, b->rs_sync.as<SyncState>(), 0, b->rs_err.as<int>(), s);
+  SyncState* sync = b->rs_sync.as<SyncState>();
+  int* err = b->rs_err.as<int>();
+  const int rc = v.plane ? rp_launch(v.n, v.E, v.LB, v.V, true, b->rs_en_grid, prm,
+                                     rp_params(b, b->rs_chunks, b->rs_segs, b->rs_n_chunks), sync, 0, err, s, nullptr)
+                         : rs_en_launch(v.n, v.E, v.LB, v.V, b->S, b->rs_en_grid, prm, b->rs_chunks.as<RsChunk>(),
+                                        b->rs_n_chunks, sync, 0, err, s);
   *done = rc == MJ_OK;
   return rc;
 }
@@ -482,8 +648,7 @@ int lfb_fused_step(mj_lfb* b, cudaStream_t s, float* copy) {
   const RsVariant& v = rs_variants()[b->rs_variant];
   RsParams prm = rs_params(b, v);
   prm.ucopy = copy;
-  return rs_launch(v, b->rs_grid, prm, b->rs_chunks.as<RsChunk>(), b->rs_n_chunks, b->rs_sync.as<SyncState>(),
-                   b->step & 1, b->rs_err.as<int>(), s);
+  return rs_launch(b, v, b->rs_grid, prm, b->rs_chunks, b->rs_segs, b->rs_n_chunks, b->step & 1, s);
 }
 
 // Phase times (ms) of the last profiled step: element phase (last CTA,

@@ -7,6 +7,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "mj_internal.cuh"
 #include "mj_k1.cuh"
 #include "mj_sync.cuh"
@@ -83,6 +85,70 @@ int rs_en_prepare(int n, int E, int LB, int V, int S, int* ctas);
 int rs_en_launch(int n, int E, int LB, int V, int S, int grid, const RsParams& prm, const RsChunk* chunks,
                  int n_chunks, SyncState* sync, int par, int* err, cudaStream_t s);
 int rs_en_set_gmat(int n, const float* g);
+
+// Dof phase of the plane form: the dofs that phase 1 does not update itself,
+// in increasing order ("kept" dofs: all, or all but the elements' interior
+// ones), cut into chunks [i0, i1) of that order.  The rows of a chunk's dofs
+// are not one range of the states: each run of consecutive dofs in it is a
+// segment, copied on its own.
+struct RpChunk {
+  int i0, i1, s0, s1;  // kept dofs, segments
+  int rows, has_src;   // contributions; whether a kept dof of it is a source dof
+  int pad0, pad1;
+};
+struct RpSeg {
+  int d0, nd, q0, nq;  // dofs [d0, d0 + nd), contributions [q0, q0 + nq)
+  int ud, rd;          // its first dof row and contribution row within the chunk
+  int pad0, pad1;
+};
+constexpr int kRpMaxSegs = 32;  // per chunk: a lane of warp 0 issues each
+
+// Byte layout of a chunk's buffer: u^{n+1} rows | u^n rows | R rows |
+// dt^2/D, first contribution row and dof of kept dofs i0&~3 onwards.
+struct RpBuf {
+  int u0, r, m, p, d, end;
+};
+__host__ __device__ __forceinline__ RpBuf rp_buf(int i0, int i1, int rows, int S) {
+  RpBuf b;
+  const int D = i1 - i0, w = (((i1 + 1 + 3) & ~3) - (i0 & ~3)) * 4;
+  b.u0 = D * S * 4;
+  b.r = 2 * D * S * 4;
+  b.m = b.r + rows * S * 4;
+  b.p = b.m + w;
+  b.d = b.p + w;
+  b.end = b.d + w;
+  return b;
+}
+
+// Parameters beyond RsParams.
+struct RpParams {
+  const RpChunk* chunks;
+  const RpSeg* segs;
+  const float* mi;    // dt^2 / D of the interior points of every element, their number rounded up to 4 per element
+  const float* mk;    // dt^2 / D of the kept dofs (padded)
+  const int* pk;      // their first contribution row, counted over the kept dofs only (padded)
+  const int* dk;      // the dofs themselves (padded)
+  const int* fix;     // sources at interior dofs: (dof, rhs) pairs, sorted
+  const float* fix_val;
+  int n_chunks, n_fix, n_elt;
+  int interior;       // phase 1 updates the interior dofs of an element
+};
+
+// The plane form (mj_rhs_plane.cu): its variants, and prepare, launch and the
+// derivative matrix as above; en: its EN form.
+struct RpVariant {
+  int n, E, LB, V, threads, half;
+};
+const std::vector<RpVariant>& rp_variants();
+int rp_prepare(int n, int E, int LB, int V, bool en, int S, int* ctas);
+int rp_launch(int n, int E, int LB, int V, bool en, int grid, const RsParams& prm, const RpParams& x,
+              SyncState* sync, int par, int* err, cudaStream_t s, unsigned long long* stamps);
+int rp_set_gmat(int n, const float* g);
+// flag[d] = 1 for the dofs of the interior points of the elements; *bad = 1
+// when one of them has other contributions than that point's.
+int rp_mark_interior(const int* nodle_e, const int* ptr, int n_elt, int n, char* flag, int* bad, cudaStream_t s);
+// mi of RpParams for n_elt_pad elements (0 in the padding) from m per dof.
+int rp_interior_mass(const int* nodle_e, const float* m, int n_elt, int n_elt_pad, int n, float* mi, cudaStream_t s);
 
 namespace {
 
