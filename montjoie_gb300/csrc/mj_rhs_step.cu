@@ -32,6 +32,7 @@ namespace mj {
 namespace {
 
 constexpr int kGraphStepsRs = 20;
+constexpr int kRsSmallMesh = 6144;  // elements
 
 // Order in which the threads of an element take its n*n z-lines.  A warp
 // holds Z = 32/LB consecutive slots; each of its shared-memory line reads
@@ -350,6 +351,13 @@ void rs_use_lists(mj_lfb* b, RsLists& L) {
   b->rs_n_chunks = L.n_chunks;
 }
 
+// CTAs of a step: all that are resident, or as many as have work.  A small
+// mesh's step is launch and grid barrier, and both grow with the CTAs: Q2
+// 8x7x7 with 8 sources took 13 us on 608 CTAs and takes 8.5 on 60.
+int rs_grid(int ctas, const RsParams& prm, int n_chunks) {
+  return std::min(ctas * sm_count(), std::max(prm.n_tiles, n_chunks));
+}
+
 int rs_check_err(mj_lfb* b, cudaStream_t s) {
   int* herr = b->op->h_status.as<int>();
   MJ_CUDA(cudaMemcpyAsync(herr, b->rs_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -369,7 +377,11 @@ int rs_check_err(mj_lfb* b, cudaStream_t s) {
 // each candidate of the order runs 3 steps (after one warm-up) on the
 // integrator's state, which mj_lfb_init resets afterwards.  The z-line
 // variants are tried only where no plane variant runs (the plane form's list
-// holds only variants faster than the best of them, mj_rhs_plane.cuh).  Leaves
+// holds only variants faster than the best of them, mj_rhs_plane.cuh) and on
+// meshes below kRsSmallMesh elements, where their smaller tiles use more of
+// the SMs: 8.5 us against 9.5 at Q2 8x7x7 with 8 sources, 10.9 against 12.4
+// at Q2 5x7x5 with 64, 32.2 against 34.4 at Q3 18^3 with 16; from 16^3 Q4 on
+// the plane form's candidates are always ahead (45.0 against 49.9).  Leaves
 // b->fused = false when no variant fits (S too large for a chunk buffer).
 int lfb_fused_setup(mj_lfb* b) {
   mj_op* op = b->op;
@@ -436,7 +448,7 @@ int lfb_fused_setup(mj_lfb* b) {
   std::stable_partition(tried.begin(), tried.end(), [&](size_t c) { return all[c].plane; });
   for (size_t c : tried) {
     const RsVariant& v = all[c];
-    if (!v.plane && planes) continue;
+    if (!v.plane && planes && op->n_elt >= kRsSmallMesh) continue;
     if (v.n != op->n || b->S % (v.LB * v.V) != 0) continue;
     if (rs_buf(3, 4, 0, 8, b->S).end > v.half) continue;  // one dof (up to 8 contributions) must fit
     int ctas = 0;
@@ -447,7 +459,7 @@ int lfb_fused_setup(mj_lfb* b) {
     if (!lists[c].n_chunks) continue;
     planes |= v.plane;
     const RsParams prm = rs_params(b, v);
-    grids[c] = ctas * sm_count();
+    grids[c] = rs_grid(ctas, prm, lists[c].n_chunks);
     auto run = [&](int k) {
       return rs_launch(b, v, grids[c], prm, lists[c].chunks, lists[c].segs, lists[c].n_chunks, k & 1, b->stream);
     };
@@ -518,7 +530,7 @@ int lfb_set_step_variant(mj_lfb* b, int E, int LB, int V) {
   rs_use_lists(b, lists);
   b->rs_variant = c;
   b->rs_threads = v.threads;
-  b->rs_grid = ctas * sm_count();
+  b->rs_grid = rs_grid(ctas, rs_params(b, v), lists.n_chunks);
   for (auto& g : b->rs_graph)
     if (g) {
       cudaGraphExecDestroy(g);
@@ -617,7 +629,7 @@ int lfb_fused_step_en(mj_lfb* b, float* u0, float* u1, float* out, const float* 
                            : rs_en_prepare(v.n, v.E, v.LB, v.V, b->S, &ctas);
     if (rc) return rc;
     b->rs_en_variant = b->rs_variant;
-    b->rs_en_grid = ctas * sm_count();
+    b->rs_en_grid = rs_grid(ctas, rs_params(b, v), b->rs_n_chunks);
   }
   if (b->rs_en_grid < 1) return MJ_OK;
   RsParams prm = rs_params(b, v);
