@@ -84,6 +84,36 @@ static __global__ void k_union_sources(const __grid_constant__ UnionRuns runs, i
   }
 }
 
+// The runs' states and their places in the union's (kernel parameter).
+struct UnionStates {
+  struct {
+    float* cur;
+    float* next;
+    int off, n;
+  } r[kMaxRuns];
+  int n;
+};
+
+// Copies every run's two states into the union's (in) or back: one launch,
+// where there was one of about 2.5 us per run and state.
+static __global__ void k_union_states(const __grid_constant__ UnionStates runs, float* __restrict__ ucur,
+                                      float* __restrict__ unext, bool in) {
+  for (int r = 0; r < runs.n; r++) {
+    const auto& q = runs.r[r];
+    float* c = ucur + q.off;
+    float* x = unext + q.off;
+    for (int d = blockIdx.x * blockDim.x + threadIdx.x; d < q.n; d += gridDim.x * blockDim.x) {
+      if (in) {
+        c[d] = q.cur[d];
+        x[d] = q.next[d];
+      } else {
+        q.cur[d] = c[d];
+        q.next[d] = x[d];
+      }
+    }
+  }
+}
+
 // A group's runs stepped as one union operator (lf_union_create).
 struct UnionGroup {
   std::unique_ptr<mj_op> op;
@@ -127,7 +157,16 @@ struct mj_mb {
   // at the start of each advance and handed back at its end.
   std::unique_ptr<UnionGroup> uni;
   bool force_union = false;  // mj_mb_set_config(-2)
+  // What an advance of the timed form costs besides its steps: the union
+  // copies in and out (0 in a form without; < 0: forced, not timed).
+  double copy_ms = -1;
+  // Grouped by order: a stream per group beside the batch's own, and the
+  // events that fork and join them.
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> side_ev;  // [0]: fork, [1 + g]: end of group g
   ~mj_mb() {
+    for (auto& e : side_ev) cudaEventDestroy(e);
+    for (auto& st : side) cudaStreamDestroy(st);
     for (auto& g : graph)
       if (g) cudaGraphExecDestroy(g);
   }
@@ -219,6 +258,53 @@ uint64_t mb_launches_per_step(const mj_mb* mb) {
   return n;
 }
 
+// Steps [i0, i0 + n) of an advance that began at launch index off, in the
+// batch's chosen form, on stream s.  The groups of a batch grouped by order
+// have no state in common: each steps on a stream of its own, forked from and
+// joined to s by events (and so branches of a captured graph), because a
+// group's kernels are small (12 meshes of 5 orders: 5 chains of 3 kernels of
+// 5 to 30 us that leave most SMs idle in turn).  Groups in the cooperative
+// batch form stay on s, where no other grid can hold back their CTAs' start.
+// Ensemble of 12 meshes, 40 steps: 3.69 ms one after the other, 2.22 ms so.
+int mb_steps(mj_mb* mb, int off, int i0, int n, cudaStream_t s) {
+  const size_t ng = mb->groups.size();
+  auto own = [&](size_t g) { return mb->groups[g]->seq || mb->groups[g]->use == 3; };
+  size_t forked = 0;
+  if (mb->use == 2 && !mb->profile)
+    for (size_t g = 0; g < ng; g++) forked += own(g);
+  if (forked < 2) {
+    for (int i = i0; i < i0 + n; i++)
+      if (int rc = mb_launch(mb, mb->use, off + i, i, s)) return rc;
+    return MJ_OK;
+  }
+  while (mb->side.size() < ng) {
+    cudaStream_t st;
+    MJ_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    mb->side.push_back(st);
+  }
+  while (mb->side_ev.size() < ng + 1) {
+    cudaEvent_t e;
+    MJ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    mb->side_ev.push_back(e);
+  }
+  MJ_CUDA(cudaEventRecord(mb->side_ev[0], s));
+  for (size_t g = 0; g < ng; g++)
+    if (own(g)) MJ_CUDA(cudaStreamWaitEvent(mb->side[g], mb->side_ev[0], 0));
+  int rc = MJ_OK;
+  for (int i = i0; !rc && i < i0 + n; i++)
+    for (size_t g = 0; !rc && g < ng; g++) {
+      mj_mb* q = mb->groups[g].get();
+      cudaStream_t st = own(g) ? mb->side[g] : s;
+      rc = q->seq ? mb_launch_seq(q, off + i, st) : mb_launch(q, q->use, off + i, i, st);
+    }
+  for (size_t g = 0; g < ng; g++)  // joined also after an error: a capture ends with every branch joined
+    if (own(g)) {
+      MJ_CUDA(cudaEventRecord(mb->side_ev[1 + g], mb->side[g]));
+      MJ_CUDA(cudaStreamWaitEvent(s, mb->side_ev[1 + g], 0));
+    }
+  return rc;
+}
+
 // The union copies of the runs' states: in, before the steps of an advance
 // (U^n, U^{n+1} of every run at its offset); out, after `steps` steps and the
 // runs' role update, back into each run's own buffers.
@@ -226,21 +312,15 @@ int union_copy(mj_mb* mb, bool in, int steps, cudaStream_t s) {
   UnionGroup* u = mb->uni.get();
   float* A = u->lf->ua.as<float>();
   float* B = u->lf->ub.as<float>();
-  float* ucur = (steps & 1) ? B : A;
-  float* unext = (steps & 1) ? A : B;
-  for (size_t r = 0; r < mb->runs.size(); r++) {
+  UnionStates t;
+  t.n = (int)mb->runs.size();
+  for (int r = 0; r < t.n; r++) {
     mj_lf* lf = mb->runs[r];
-    const size_t bytes = sizeof(float) * lf->n_dof;
-    float* c = ucur + u->dof_off[r];
-    float* x = unext + u->dof_off[r];
-    if (in) {
-      MJ_CUDA(cudaMemcpyAsync(c, lf->cur(), bytes, cudaMemcpyDeviceToDevice, s));
-      MJ_CUDA(cudaMemcpyAsync(x, lf->next(), bytes, cudaMemcpyDeviceToDevice, s));
-    } else {
-      MJ_CUDA(cudaMemcpyAsync(lf->cur(), c, bytes, cudaMemcpyDeviceToDevice, s));
-      MJ_CUDA(cudaMemcpyAsync(lf->next(), x, bytes, cudaMemcpyDeviceToDevice, s));
-    }
+    t.r[r] = {static_cast<float*>(lf->cur()), static_cast<float*>(lf->next()), u->dof_off[r], (int)lf->n_dof};
   }
+  const int blocks = std::max(1, std::min((int)((u->lf->n_dof + 1023) / 1024), 4 * sm_count()));
+  k_union_states<<<blocks, 256, 0, s>>>(t, (steps & 1) ? B : A, (steps & 1) ? A : B, in);
+  MJ_CUDA(cudaGetLastError());
   return MJ_OK;
 }
 
@@ -444,6 +524,7 @@ int mb_autotune(mj_mb* mb, int off, cudaStream_t s) {
   MJ_CUDA(cudaEventCreate(&e1));
   const uint64_t before = launch_counter().load();
   int best = 0;
+  double copy_ms[4] = {0, 0, 0, 0};
   std::vector<int> forms = {0, 1};
   if (!mb->groups.empty()) forms.push_back(2);
   if (mb->uni) forms.push_back(3);
@@ -469,14 +550,26 @@ int mb_autotune(mj_mb* mb, int off, cudaStream_t s) {
         if (rc) break;
         g->seq = g->seq_ms < g->batch_ms;
       }
-    if (!rc) rc = mb_launch(mb, c, off, 0, s);
+    mb->use = c;
+    if (!rc) rc = mb_steps(mb, off, 0, 1, s);
     if (!rc) rc = cudaEventRecord(e0, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
-    for (int i = 1; !rc && i <= 3; i++) rc = mb_launch(mb, c, off + i, i, s);
+    if (!rc) rc = mb_steps(mb, off, 1, 3, s);
     if (!rc) rc = cudaEventRecord(e1, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
     if (!rc) rc = mb_check_err(mb, s);
     float ms = 0.f;
     if (!rc) rc = cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+    if (c >= 2) {  // its copies, out and in again
+      if (!rc) rc = cudaEventRecord(e0, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+      if (!rc) rc = mb_union_copy(mb, false, 4, s);
+      if (!rc) rc = mb_union_copy(mb, true, 0, s);
+      if (!rc) rc = cudaEventRecord(e1, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+      if (!rc) rc = cudaStreamSynchronize(s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+      float cms = 0.f;
+      if (!rc) rc = cudaEventElapsedTime(&cms, e0, e1) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+      copy_ms[c] = cms;
+    }
     if (rc) {
+      mb->use = -1;
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       return rc;
@@ -497,6 +590,7 @@ int mb_autotune(mj_mb* mb, int off, cudaStream_t s) {
   }
   MJ_CUDA(cudaStreamSynchronize(s));
   mb->use = best;
+  mb->copy_ms = copy_ms[best];
   return MJ_OK;
 }
 
@@ -680,6 +774,19 @@ int mj_mb_advance(mj_mb* mb, int nsteps, int use_graph) {
         const int rc = mb_autotune(g.get(), off, s);
         if (rc) return rc;
       }
+  // An advance of a few steps does not pay for a union's copies: one kernel
+  // of all its meshes then (the forms' FP32 states agree to rounding, and
+  // timing chooses between them anyway).  10 meshes, one step: 172 us, with
+  // the copies 234.
+  struct Form {  // this call's form; the batch keeps its own
+    mj_mb* mb;
+    int use;
+    ~Form() { mb->use = use; }
+  } kept{mb, mb->use};
+  if (mb->use >= 2 && mb->copy_ms >= 0 && nsteps < kGraphStepsMb && !mb->profile) {
+    const int one = mb->tune_ms[0] <= mb->tune_ms[1] ? 0 : 1;
+    if (nsteps * mb->tune_ms[one] < mb->copy_ms + nsteps * mb->tune_ms[mb->use]) mb->use = one;
+  }
   if (int rc = mb_union_copy(mb, true, 0, s)) return rc;
   mb->last_graph = false;
   int done = 0;
@@ -690,13 +797,10 @@ int mj_mb_advance(mj_mb* mb, int nsteps, int use_graph) {
       cudaGraph_t g;
       const uint64_t before = launch_counter().load();
       MJ_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < kGraphStepsMb; k++) {
-        const int rc = mb_launch(mb, mb->use, off + k, k, cs);
-        if (rc) {
-          cudaStreamEndCapture(cs, &g);
-          cudaStreamDestroy(cs);
-          return rc;
-        }
+      if (const int rc = mb_steps(mb, off, 0, kGraphStepsMb, cs)) {
+        cudaStreamEndCapture(cs, &g);
+        cudaStreamDestroy(cs);
+        return rc;
       }
       MJ_CUDA(cudaStreamEndCapture(cs, &g));
       launch_counter().store(before);  // captured, not launched
@@ -712,10 +816,8 @@ int mj_mb_advance(mj_mb* mb, int nsteps, int use_graph) {
     }
     mb->last_graph = true;
   }
-  for (; done < nsteps; done++) {
-    const int rc = mb_launch(mb, mb->use, off + done, done, s);
-    if (rc) return rc;
-  }
+  if (done < nsteps)
+    if (int rc = mb_steps(mb, off, done, nsteps - done, s)) return rc;
   for (mj_lf* lf : mb->runs) {
     lf->step += nsteps;
     if (nsteps & 1) lf->cur_is_a = !lf->cur_is_a;
@@ -829,9 +931,11 @@ int mj_mb_set_config(mj_mb* mb, int threads) {
     if (mb->groups.empty()) {
       MJ_CHECK_ARG(mb->uni, "mj_mb_set_config: the batch is too large for one union");
       mb->use = 3;
+      mb->copy_ms = -1;
     } else {
       for (auto& g : mb->groups) MJ_CHECK_ARG(g->uni, "mj_mb_set_config: a group is too large for one union");
       mb->use = 2;
+      mb->copy_ms = -1;
       for (auto& g : mb->groups) {
         g->use = 3;
         g->seq = false;
@@ -839,6 +943,7 @@ int mj_mb_set_config(mj_mb* mb, int threads) {
     }
   } else {
     mb->use = threads == 0 ? -1 : threads == 256 ? 0 : threads == 128 ? 1 : 2;
+    mb->copy_ms = -1;
     for (auto& g : mb->groups) g->use = -1;  // groups tune again at the next advance
   }
   for (auto& g : mb->graph)

@@ -203,3 +203,27 @@ def test_batch_rejects_bad_runs():
     mb.close()
     for x in (lf64, lf, lf2, lf3, op64, op):
         x.close()
+
+
+@pytest.mark.parametrize("steps", [(1, 25, 3), (2, 20, 41)])
+def test_short_and_long_advances_mix(steps):
+    """The form an advance takes depends on its length (a few steps do not
+    pay for a union's copies; groups step on streams of their own): any
+    sequence of lengths gives the states of the runs advanced alone."""
+    from montjoie_gb300.leapfrog import MeshBatch
+    gs = [load_golden(c) for c in CASES]
+    batch_runs = [run_fp32(g) for g in gs]
+    single_runs = [run_fp32(g) for g in gs]
+    mb = MeshBatch([lf for _, lf in batch_runs])
+    for config in (0, -1):
+        mb.set_config(config)
+        for n in steps:
+            mb.advance(n)
+            for (_, lf), (_, ls) in zip(batch_runs, single_runs):
+                ls.Advance(n)
+                assert lf.n_time == ls.n_time
+                assert rel_l2(lf.GetIterate(), ls.GetIterate()) < SAME_TOL
+    mb.close()
+    for op, lf in batch_runs + single_runs:
+        lf.close()
+        op.close()
