@@ -1046,7 +1046,8 @@ int mj_adj_forward(mj_adj* a, double* traces) {
   float* ck = a->revolve ? a->slots.as<float>() : a->ckpt.as<float>();
   size_t next_store = 0;  // revolve: the next (k, slot) of sweep_stores (increasing k)
   for (int n = 0; n <= a->N; n++) {
-    adj_receivers(a, b->cur(), n, s);
+    // a one-kernel step takes the receivers of U^{n+1} along; U^0's are taken here
+    if (n == 0 || !b->fused) adj_receivers(a, b->cur(), n, s);
     if (n == a->N) break;
     int slot = -1;
     if (!a->revolve && n % a->K == 0) slot = n / a->K;
@@ -1068,7 +1069,7 @@ int mj_adj_forward(mj_adj* a, double* traces) {
     }
     if (b->fused) {
       float* copy = a->store_all && n + 2 < a->N ? a->seg.as<float>() + (size_t)(n + 2) * a->rows : nullptr;
-      const int rc = lfb_fused_step(b, s, copy);
+      const int rc = lfb_fused_step(b, s, copy, a->traces.as<double>() + n + 1, a->N + 1);
       if (rc) return rc;
     } else {
       lfb_step_launch(b, b->cur(), b->next(), b->step & 1, s);

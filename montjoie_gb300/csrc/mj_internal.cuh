@@ -125,6 +125,7 @@ struct mj_lfb {
   // shape, dof chunks, sources grouped by dof, barrier state, graphs by parity
   bool fused = true;
   int rs_variant = -1, rs_grid = 0, rs_threads = 0, rs_n_chunks = 0;
+  int rs_resident = 0;  // CTAs of the step that the device holds
   mj::DevBuf rs_chunks, rs_src_ptr, rs_src_rhs, rs_src_val, rs_sync, rs_err;
   // the plane form's dof phase: its chunks' segments, the dofs it updates, and
   // the sources at the others (RpParams)
@@ -243,7 +244,7 @@ int lfb_copy_traces(mj_lfb* b, int nsteps, double* traces, int trace_stride, cud
 void lfb_receivers(mj_lfb* b, const float* u, int stride, int col, cudaStream_t s);
 int lfb_phase_ms(const mj_lfb* b, double* out);
 int lfb_fused_step_on(mj_lfb* b, float* u0, float* u1, float* out, int step, cudaStream_t s);
-int lfb_fused_step(mj_lfb* b, cudaStream_t s, float* copy = nullptr);
+int lfb_fused_step(mj_lfb* b, cudaStream_t s, float* copy, double* rec, int rec_stride);
 int lfb_fused_step_en(mj_lfb* b, float* u0, float* u1, float* out, const float* ue, double* gacc,
                       const double* gcoef, cudaStream_t s, bool* done);
 int lfb_fused_check(mj_lfb* b, cudaStream_t s);

@@ -496,6 +496,9 @@ __global__ void __launch_bounds__(RpPlan<N, E, LB, V>::T, RpPlan<N, E, LB, V>::k
     }
   }
 
+  if constexpr (!EN) {
+    if (p.rec_out) rs_receivers<P::T, P::kArea>(p, nxt, smem);
+  }
   fence_proxy_async_global();  // this thread's R stores before the bulk copies of phase 2
   if (stamps && t == 0) stamps[4 * blockIdx.x + 1] = global_ns();
   if (!grid_barrier(sync, err)) return;

@@ -191,6 +191,12 @@ RsParams rs_params(mj_lfb* b, const RsVariant& v) {
   p.ue = nullptr;
   p.gacc = nullptr;
   p.gcoef = nullptr;
+  p.rec_idx = b->rec_idx.as<int>();
+  p.rec_w = b->rec_w.as<double>();
+  p.rec_out = nullptr;
+  p.n_rec = b->n_rec;
+  p.n_rec_w = b->n_rec_w;
+  p.rec_stride = 0;
   p.n_pulse = b->n_pulse;
   p.S = b->S;
   p.n_tiles = op->n_elt_pad / v.E;
@@ -358,6 +364,12 @@ int rs_grid(int ctas, const RsParams& prm, int n_chunks) {
   return std::min(ctas * sm_count(), std::max(prm.n_tiles, n_chunks));
 }
 
+// The grid of a step that also takes the receivers' values.
+int rs_rec_grid(const mj_lfb* b) {
+  const int L = b->S % 32 == 0 ? 32 : b->S % 16 == 0 ? 16 : 8;
+  return std::min(b->rs_resident, std::max(b->rs_grid, b->n_rec * (b->S / L)));
+}
+
 int rs_check_err(mj_lfb* b, cudaStream_t s) {
   int* herr = b->op->h_status.as<int>();
   MJ_CUDA(cudaMemcpyAsync(herr, b->rs_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -441,7 +453,7 @@ int lfb_fused_setup(mj_lfb* b) {
   double best = 1e300;
   int bi = -1;
   std::vector<RsLists> lists(all.size());
-  std::vector<int> grids(all.size(), 0);
+  std::vector<int> grids(all.size(), 0), resident(all.size(), 0);
   bool planes = false;  // a plane variant runs
   std::vector<size_t> tried(all.size());
   for (size_t c = 0; c < all.size(); c++) tried[c] = c;
@@ -460,6 +472,7 @@ int lfb_fused_setup(mj_lfb* b) {
     planes |= v.plane;
     const RsParams prm = rs_params(b, v);
     grids[c] = rs_grid(ctas, prm, lists[c].n_chunks);
+    resident[c] = ctas * sm_count();
     auto run = [&](int k) {
       return rs_launch(b, v, grids[c], prm, lists[c].chunks, lists[c].segs, lists[c].n_chunks, k & 1, b->stream);
     };
@@ -489,6 +502,7 @@ int lfb_fused_setup(mj_lfb* b) {
   b->rs_variant = bi;
   b->rs_threads = all[bi].threads;
   b->rs_grid = grids[bi];
+  b->rs_resident = resident[bi];
   rs_use_lists(b, lists[bi]);
   b->fused = true;
   return MJ_OK;
@@ -531,6 +545,7 @@ int lfb_set_step_variant(mj_lfb* b, int E, int LB, int V) {
   b->rs_variant = c;
   b->rs_threads = v.threads;
   b->rs_grid = rs_grid(ctas, rs_params(b, v), lists.n_chunks);
+  b->rs_resident = ctas * sm_count();
   for (auto& g : b->rs_graph)
     if (g) {
       cudaGraphExecDestroy(g);
@@ -544,15 +559,15 @@ int lfb_set_step_variant(mj_lfb* b, int E, int LB, int V) {
 // runs of 20 steps replay a CUDA graph captured for the current step parity.
 int lfb_fused_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, bool use_graph) {
   const RsVariant& v = rs_variants()[b->rs_variant];
-  const RsParams prm = rs_params(b, v);
+  RsParams prm = rs_params(b, v);
   cudaStream_t s = b->stream;
   const bool diag = traces && b->n_rec;
   const bool prof = b->rs_profile;
-  if (prof && b->rs_stamps.bytes < sizeof(unsigned long long) * 4 * b->rs_grid)
-    MJ_CUDA(b->rs_stamps.alloc(sizeof(unsigned long long) * 4 * b->rs_grid));
+  if (prof && b->rs_stamps.bytes < sizeof(unsigned long long) * 4 * b->rs_resident)
+    MJ_CUDA(b->rs_stamps.alloc(sizeof(unsigned long long) * 4 * b->rs_resident));
   auto launch = [&](int par, cudaStream_t st) {
-    return rs_launch(b, v, b->rs_grid, prm, b->rs_chunks, b->rs_segs, b->rs_n_chunks, par, st,
-                     prof ? b->rs_stamps.as<unsigned long long>() : (unsigned long long*)nullptr);
+    return rs_launch(b, v, prm.rec_out ? rs_rec_grid(b) : b->rs_grid, prm, b->rs_chunks, b->rs_segs, b->rs_n_chunks,
+                     par, st, prof ? b->rs_stamps.as<unsigned long long>() : (unsigned long long*)nullptr);
   };
   int done = 0;
   if (use_graph && !diag && !prof && nsteps >= kGraphStepsRs) {
@@ -585,7 +600,11 @@ int lfb_fused_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, b
     }
   }
   for (; done < nsteps; done++) {
-    if (diag) lfb_receivers(b, b->cur(), nsteps, done, s);
+    // column `done` of the traces is the state before this step: the first by a kernel of its own, each other by the
+    // step before it, which reads that state
+    if (diag && done == 0) lfb_receivers(b, b->cur(), nsteps, 0, s);
+    prm.rec_stride = nsteps;
+    prm.rec_out = diag && done + 1 < nsteps ? b->traces_d.as<double>() + done + 1 : nullptr;
     const int rc = launch(b->step & 1, s);
     if (rc) return rc;
     b->cur_is_a = !b->cur_is_a;
@@ -655,12 +674,17 @@ int lfb_fused_step_en(mj_lfb* b, float* u0, float* u1, float* out, const float* 
 int lfb_fused_check(mj_lfb* b, cudaStream_t s) { return rs_check_err(b, s); }
 
 // One ordinary step of the one-kernel form (the integrator's own states and
-// step counter); copy: where a second copy of the new state goes, or nullptr.
-int lfb_fused_step(mj_lfb* b, cudaStream_t s, float* copy) {
+// step counter); copy: where a second copy of the new state goes, or nullptr;
+// rec: where the receivers' values of U^{n+1} go (a column of an array of
+// rec_stride columns).
+int lfb_fused_step(mj_lfb* b, cudaStream_t s, float* copy, double* rec, int rec_stride) {
   const RsVariant& v = rs_variants()[b->rs_variant];
   RsParams prm = rs_params(b, v);
   prm.ucopy = copy;
-  return rs_launch(b, v, b->rs_grid, prm, b->rs_chunks, b->rs_segs, b->rs_n_chunks, b->step & 1, s);
+  prm.rec_out = rec;
+  prm.rec_stride = rec_stride;
+  return rs_launch(b, v, rec ? rs_rec_grid(b) : b->rs_grid, prm, b->rs_chunks, b->rs_segs, b->rs_n_chunks, b->step & 1,
+                   s);
 }
 
 // Phase times (ms) of the last profiled step: element phase (last CTA,

@@ -38,6 +38,12 @@ struct RsParams {
   const double* gcoef;
   int n_pulse, S, n_tiles;
   int step;            // the step's pulse index, or -1: ctr[par], and ctr[1-par] = ctr[par] + 1 after it
+  // receivers of U^{n+1}, or rec_out = nullptr: out[(k*S + s)*rec_stride] =
+  // sum_t rec_w[k][t] U^{n+1}[rec_idx[k][t]][s]
+  const int* rec_idx;
+  const double* rec_w;
+  double* rec_out;
+  int n_rec, n_rec_w, rec_stride;
   unsigned char zmap[kMaxNK * kMaxNK];  // z-line (j*n + i) of each thread slot of an element (rs_zline_order)
 };
 
@@ -224,6 +230,48 @@ __device__ __forceinline__ void mul_v(float (&acc)[V], float c, const float (&x)
   }
 }
 
+
+// Receivers of U^{n+1} (RsParams) in a step's phase 1, after this CTA's tiles:
+// k_receivers_rhs as (receiver, L right-hand sides) jobs, the FP64 sums in the
+// same order, through the CTA's phase-1 shared memory (AREA bytes at smem, at
+// rest).  The CTAs with the fewest tiles take the first jobs.  A kernel of its
+// own cost 15 us per step whatever the mesh (a chain of 125 FP64 additions at
+// Q4 after two dependent gathers), as much as a small mesh's step, where half
+// of the CTAs wait for the last tiles.
+template <int T, int AREA>
+__device__ __forceinline__ void rs_receivers(const RsParams& p, const float* __restrict__ u, unsigned char* smem) {
+  const int S = p.S, L = S % 32 == 0 ? 32 : S % 16 == 0 ? 16 : 8, per = S / L, n_w = p.n_rec_w;
+  static_assert(T >= 32 && AREA >= 34 * 8, "a row of right-hand sides, a chunk of one weight");
+  constexpr int kChunk = AREA / 8 / 34 < 128 ? AREA / 8 / 34 : 128;
+  double* sv = reinterpret_cast<double*>(smem);
+  double* sw = sv + kChunk * 32;
+  int* si = reinterpret_cast<int*>(sw + kChunk);
+  const int lane = threadIdx.x % L, row = threadIdx.x / L, rows = T / L;
+  for (int job = gridDim.x - 1 - blockIdx.x; job < p.n_rec * per; job += gridDim.x) {
+    const int k = job / per, s = (job - k * per) * L + lane;
+    double acc = 0.0;
+    for (int t0 = 0; t0 < n_w; t0 += kChunk) {
+      const int m = min(kChunk, n_w - t0);
+      const size_t at = (size_t)k * n_w + t0;
+      __syncthreads();  // the tiles, or the previous chunk, are done with the memory
+      for (int a = threadIdx.x; a < m; a += T) {
+        sw[a] = __ldg(p.rec_w + at + a);
+        si[a] = __ldg(p.rec_idx + at + a);
+      }
+      __syncthreads();
+      if (row < rows) {
+#pragma unroll 8
+        for (int a = row; a < m; a += rows) sv[a * L + lane] = double(__ldg(u + (size_t)si[a] * S + s));
+      }
+      __syncthreads();
+      if (row == 0) {
+#pragma unroll 16
+        for (int a = 0; a < m; a++) acc += sw[a] * sv[a * L + lane];
+      }
+    }
+    if (row == 0) p.rec_out[((size_t)k * S + s) * p.rec_stride] = acc;
+  }
+}
 
 template <int N, int E, int LB, int V>
 struct RsPlan {
@@ -425,6 +473,9 @@ __global__ void __launch_bounds__(RsPlan<N, E, LB, V>::T, rs_min_ctas(RsPlan<N, 
     }
   }
 
+  if constexpr (!EN) {
+    if (p.rec_out) rs_receivers<P::T, P::kArea>(p, nxt, smem);
+  }
   fence_proxy_async_global();  // this thread's R stores before the bulk copies of phase 2
   if (stamps && t == 0) stamps[4 * blockIdx.x + 1] = global_ns();
   if (!grid_barrier(sync, err)) return;
