@@ -504,6 +504,7 @@ __global__ void __launch_bounds__(RpPlan<N, E, LB, V>::T, RpPlan<N, E, LB, V>::k
   if (!grid_barrier(sync, err)) return;
   if (stamps && t == 0) stamps[4 * blockIdx.x + 2] = global_ns();
 
+  if constexpr (EN) asm volatile("griddepcontrol.launch_dependents;");  // the adjoint's injection may start
   // ---- phase 2
   rp_dof_phase<P::T, P::kHalf>(p, x, smem, &bar[2], cur, nxt, par, err);
   if (stamps) {

@@ -481,6 +481,7 @@ __global__ void __launch_bounds__(RsPlan<N, E, LB, V>::T, rs_min_ctas(RsPlan<N, 
   if (!grid_barrier(sync, err)) return;
   if (stamps && t == 0) stamps[4 * blockIdx.x + 2] = global_ns();
 
+  if constexpr (EN) asm volatile("griddepcontrol.launch_dependents;");  // the adjoint's injection may start
   // ---- phase 2
   float* __restrict__ dst = p.uout ? p.uout : cur;
   const int step = p.step >= 0 ? p.step : p.ctr[par];
