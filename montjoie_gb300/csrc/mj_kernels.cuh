@@ -354,6 +354,7 @@ struct StreamDiag {
   const DiagDev* dd;
   DiagDev direct;
   int col;
+  int defer;  // the last part (stream_diag_tail) is k_stream_diag_tail's
 };
 
 struct StreamChunk {
@@ -369,30 +370,11 @@ __device__ __forceinline__ float stream_norm_term(float w, float u, float acc) {
   return __fmaf_rn(__fmul_rn(w, u), u, acc);
 }
 
-// End of a fused-diagnostics launch over the streaming chunks (grid G):
-// block tree of the threads' sums, one partial per CTA; the last CTA to
-// finish adds the partials in a fixed order and samples the receivers from
-// the finished state u.
+// Last part of the fused diagnostics, by one CTA of kStreamThreads: the G
+// partials added in a fixed order, and the receivers of the finished state u.
 template <typename Real>
-__device__ __forceinline__ void stream_diag_finish(double nacc, const StreamDiag& dg, const Real* u, int G) {
-  __shared__ double sh[kStreamThreads / 32];
-  __shared__ bool last;
+__device__ __forceinline__ void stream_diag_tail(const StreamDiag& dg, const Real* u, int G) {
   const int t = threadIdx.x;
-  for (int o = 16; o > 0; o >>= 1) nacc += __shfl_down_sync(0xffffffffu, nacc, o);
-  if ((t & 31) == 0) sh[t >> 5] = nacc;
-  __syncthreads();  // also: every thread's state writes are done
-  if (t < 32) {
-    double a = t < kStreamThreads / 32 ? sh[t] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if (t == 0) {
-      dg.partial[blockIdx.x] = a;
-      __threadfence();
-      last = atomicAdd(dg.done, 1u) == (unsigned)G - 1u;
-    }
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
   const DiagDev where = dg.dd ? *dg.dd : dg.direct;
   const int col = where.col + dg.col;
   const int warp = t >> 5, lane = t & 31;
@@ -434,6 +416,45 @@ __device__ __forceinline__ void stream_diag_finish(double nacc, const StreamDiag
         if (lane == 0) where.traces[(size_t)r * where.stride + col] = acc;
       }
   }
+}
+
+// The last part as a kernel of its own, beside the next step in a captured
+// graph: in the step's last CTA it keeps the next step waiting for about 6 us
+// (a fence, an atomic, the partials and two dependent gathers per receiver),
+// at 16^3 Q4 in FP64 almost as long as the gather itself (a step there: 33.4 ->
+// 27.0 us; 64^3 Q4 in FP32 307 -> 302 us).
+template <typename Real>
+__global__ void __launch_bounds__(kStreamThreads) k_stream_diag_tail(const Real* u, int G, StreamDiag dg) {
+  stream_diag_tail(dg, u, G);
+}
+
+// End of a fused-diagnostics launch over the streaming chunks (grid G):
+// block tree of the threads' sums, one partial per CTA; without defer, the
+// last CTA to finish does the last part.
+template <typename Real>
+__device__ __forceinline__ void stream_diag_finish(double nacc, const StreamDiag& dg, const Real* u, int G) {
+  __shared__ double sh[kStreamThreads / 32];
+  __shared__ bool last;
+  const int t = threadIdx.x;
+  for (int o = 16; o > 0; o >>= 1) nacc += __shfl_down_sync(0xffffffffu, nacc, o);
+  if ((t & 31) == 0) sh[t >> 5] = nacc;
+  __syncthreads();  // also: every thread's state writes are done
+  if (t < 32) {
+    double a = t < kStreamThreads / 32 ? sh[t] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (t == 0) {
+      dg.partial[blockIdx.x] = a;
+      if (!dg.defer) {
+        __threadfence();
+        last = atomicAdd(dg.done, 1u) == (unsigned)G - 1u;
+      }
+    }
+  }
+  if (dg.defer) return;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  stream_diag_tail(dg, u, G);
   if (t == 0) *dg.done = 0u;
 }
 

@@ -147,7 +147,9 @@ int autotune_k1(mj_op* op) {
   double best = 1e300;
   int bestE = -1, bestGrid = 1;
   bool bestVec = false, bestWarp = false, bestPacked = false, bestFs = false, bestFx = false, bestLn = false;
-  const bool time_it = (long long)op->n_elt * op->Q >= 2000000;
+  // fixed point is timed on small meshes too: its few candidates tie in the score below, and 16^3 Q4 takes 19.0 us with
+  // 5 elements per tile, 20.8 with 4, 10^3 Q8 39.9 with 3, 43.4 with 1
+  const bool time_it = op->fac_fx.ptr || (long long)op->n_elt * op->Q >= 2000000;
   // layouts: 0 compact, 1 vector lines, 2 one element per warp, 3 the same
   // with packed connectivity, 4 compact with one factor stage (2-4: FP32), 5 fixed point (FP64: always where the
   // derivative matrix is in its range; the FP64-pipe kernel took 2.1 (Q1) to 4.4 (Q6) times as long on large meshes,
@@ -854,7 +856,7 @@ int lf_stream_setup(mj_lf* lf, bool* fits = nullptr) {
   }
   MJ_CHECK_ARG(ctas >= 1, "streaming gather cannot be resident");
   lf->stream_grid_ = std::max(1, std::min(lf->n_stream_chunks, ctas * sm_count()));
-  MJ_CUDA(lf->stream_partial.alloc(sizeof(double) * lf->stream_grid_));
+  MJ_CUDA(lf->stream_partial.alloc(2 * sizeof(double) * lf->stream_grid_));  // two: a step's and the one's before it
   return MJ_OK;
 }
 
@@ -1248,6 +1250,23 @@ int lf_step(mj_lf* lf, const StreamDiag* dg = nullptr) {
 // kGraphSteps at the end of the graph).
 template <typename Real>
 int lf_capture(mj_lf* lf, bool prof, cudaGraphExec_t* out, bool diag = false) {
+  // Fused diagnostics: their last part is a branch beside the next step.  Step
+  // k + 2 writes over the state it reads and the partials it adds, and waits.
+  struct Branch {
+    cudaStream_t s = nullptr;
+    cudaEvent_t stepped = nullptr, tail[2] = {nullptr, nullptr};
+    ~Branch() {
+      for (cudaEvent_t e : {stepped, tail[0], tail[1]})
+        if (e) cudaEventDestroy(e);
+      if (s) cudaStreamDestroy(s);
+    }
+  } br;
+  const bool fused = diag && lf_fused_diag(lf);
+  if (fused) {
+    MJ_CUDA(cudaStreamCreateWithFlags(&br.s, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&br.stepped, &br.tail[0], &br.tail[1]})
+      MJ_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
   cudaStream_t cs;
   MJ_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaGraph_t g;
@@ -1260,15 +1279,24 @@ int lf_capture(mj_lf* lf, bool prof, cudaGraphExec_t* out, bool diag = false) {
   for (int k = 0; k < kGraphSteps; k++) {
     void* cur = a ? lf->ua.ptr : lf->ub.ptr;
     void* nxt = a ? lf->ub.ptr : lf->ua.ptr;
-    if (diag && lf_fused_diag(lf)) {  // the step writes its new iterate's column (k + 2)
-      const StreamDiag dg = lf_stream_diag(lf, lf->diag_where.as<DiagDev>(), DiagDev{}, k + 2);
+    if (fused) {  // the step writes its new iterate's column (k + 2)
+      StreamDiag dg = lf_stream_diag(lf, lf->diag_where.as<DiagDev>(), DiagDev{}, k + 2);
+      dg.defer = 1;
+      dg.partial += (k & 1) * lf->stream_grid_;
+      if (k >= 2) cudaStreamWaitEvent(cs, br.tail[k & 1], 0);
       lf_step_launch<Real>(lf, cur, nxt, k & 1, cs, prof, &dg);
+      cudaEventRecord(br.stepped, cs);
+      cudaStreamWaitEvent(br.s, br.stepped, 0);
+      k_stream_diag_tail<Real><<<1, kStreamThreads, 0, br.s>>>(static_cast<const Real*>(cur), lf->stream_grid_, dg);
+      cudaEventRecord(br.tail[k & 1], br.s);
     } else {
       if (diag) lf_diag_launch<Real>(lf, cur, nullptr, nullptr, 0, k, lf->diag_where.as<DiagDev>(), cs);
       lf_step_launch<Real>(lf, cur, nxt, k & 1, cs, prof);
     }
     a = !a;
   }
+  if (fused)
+    for (cudaEvent_t e : br.tail) cudaStreamWaitEvent(cs, e, 0);
   if (diag) {
     k_diag_advance<<<1, 1, 0, cs>>>(lf->diag_where.as<DiagDev>(), kGraphSteps);
     count_launch();
@@ -1362,7 +1390,7 @@ int lf_advance_impl(mj_lf* lf, int nsteps, double* norms, double* traces, int st
     count_launch();
     while (nsteps - s0 >= kGraphSteps) {
       MJ_CUDA(cudaGraphLaunch(lf->graph_diag, lf->stream));
-      count_launch((uint64_t)kGraphSteps * (lf_kernels_per_step(lf) + (fused ? 0 : 1)) + 1);
+      count_launch((uint64_t)kGraphSteps * (lf_kernels_per_step(lf) + 1) + 1);
       s0 += kGraphSteps;
       lf->step += kGraphSteps;
     }
