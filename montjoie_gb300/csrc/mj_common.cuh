@@ -113,4 +113,27 @@ int sm_count();
 // through.
 int take_kernel_error(void* dev_flag, cudaStream_t s, const char* what, int* host);
 
+// Launch of a kernel that begins with dependent_wait(): it may be launched
+// while the kernel before it on the stream is ending, which hides the launch
+// and the start of its CTAs; it reads and writes nothing before that kernel
+// has ended and its stores are visible.  A step of two such kernels gains
+// about 0.8 us: 2^3 Q4 in FP32 5.5 -> 4.7 us, 32^3 Q4 41.0 -> 40.2, Q8 32^3
+// 232.6 -> 230.8.  (They do not let the next kernel start any earlier than at
+// their end: its waiting CTAs would take the room of other streams' kernels.)
+template <class... P, class... A>
+void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+__device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace mj

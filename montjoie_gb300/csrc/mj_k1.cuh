@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(E* N* N)
     k_local_stiffness(const Real* __restrict__ x, const int* __restrict__ nodle_e,
                       const Real* __restrict__ fac_e, Real* __restrict__ R, const int* __restrict__ slot_e,
                       int n_tiles, int* __restrict__ err) {
+  dependent_wait();
   using P = K1Plan<Real, N, E, 1, VEC>;
   constexpr int NN = P::NN, Qp = P::Qp;
   const Real* __restrict__ Gm = GConst<Real>::get(N);
@@ -416,6 +417,7 @@ __global__ void __launch_bounds__(E* N* N)
     k_local_stiffness_fs(const Real* __restrict__ x, const int* __restrict__ nodle_e,
                          const Real* __restrict__ fac_e, Real* __restrict__ R, const int* __restrict__ slot_e,
                          int n_tiles, int* __restrict__ err) {
+  dependent_wait();
   using P = K1PlanFS<Real, N, E>;
   constexpr int NN = P::NN, Q = P::Q, Qp = P::Qp;
   const Real* __restrict__ Gm = GConst<Real>::get(N);
@@ -600,6 +602,7 @@ __global__ void __launch_bounds__(E * 32)
     k_local_stiffness_w(const Real* __restrict__ x, const int* __restrict__ nodle_e,
                         const Real* __restrict__ fac_e, Real* __restrict__ R, const int* __restrict__ slot_e,
                         int n_tiles, int* __restrict__ err) {
+  dependent_wait();
   // PK: nodle_e is the packed connectivity and slot_e the CSR offsets ptr
   static_assert(N * N <= 32, "one element per warp");
   using P = K1Plan<Real, N, E, 1, false>;

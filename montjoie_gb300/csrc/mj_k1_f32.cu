@@ -34,7 +34,7 @@ template <int E, bool PK>
 void launch_w_one(int grid, const void* x, const int* nodle_e, const void* fac_e, void* R, const int* slot_e,
                   int n_tiles, int* err, cudaStream_t s) {
   using P = K1Plan<float, 5, E, 1, false>;
-  k_local_stiffness_w<float, 5, E, kSpinLimit, PK><<<grid, E * 32, P::total, s>>>(
+  launch_dependent(k_local_stiffness_w<float, 5, E, kSpinLimit, PK>, grid, E * 32, P::total, s,
       static_cast<const float*>(x), nodle_e, static_cast<const float*>(fac_e), static_cast<float*>(R), slot_e,
       n_tiles, err);
 }

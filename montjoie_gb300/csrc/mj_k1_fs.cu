@@ -32,7 +32,7 @@ template <int N, int E>
 void launch_fs_one(int grid, const void* x, const int* nodle_e, const void* fac_e, void* R, const int* slot_e,
                    int n_tiles, int* err, cudaStream_t s) {
   using P = K1PlanFS<float, N, E>;
-  k_local_stiffness_fs<float, N, E><<<grid, P::threads, P::total, s>>>(
+  launch_dependent(k_local_stiffness_fs<float, N, E>, grid, P::threads, P::total, s,
       static_cast<const float*>(x), nodle_e, static_cast<const float*>(fac_e), static_cast<float*>(R), slot_e,
       n_tiles, err);
 }

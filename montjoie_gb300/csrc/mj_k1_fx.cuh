@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
                          const int2* __restrict__ fac_fx, const int* __restrict__ fac_exp,
                          const double* __restrict__ fac_e, double* __restrict__ R, const int* __restrict__ slot_e,
                          int n_tiles, int* __restrict__ err) {
+  dependent_wait();
   using P = FxPlan<N, E>;
   constexpr int NN = P::NN, Qp = P::Qp, RS = P::RS, W = P::W;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -526,7 +527,8 @@ template <bool SYM>
 void launch_fx(mj_op* op, const void* x, cudaStream_t s) {
 #define MJ_X(NV, EV)                                                                                          \
   if (op->n == NV && op->E == EV) {                                                                           \
-    k_local_stiffness_fx<NV, EV, SYM><<<op->grid_k1, FxPlan<NV, EV>::threads, FxPlan<NV, EV>::total, s>>>(    \
+    launch_dependent(                                                                                         \
+        k_local_stiffness_fx<NV, EV, SYM>, op->grid_k1, FxPlan<NV, EV>::threads, FxPlan<NV, EV>::total, s,    \
         static_cast<const double*>(x), op->nodle_e.as<int>(), op->fac_fx.as<int2>(), op->fac_exp.as<int>(),   \
         op->fac_e.as<double>(), op->R.as<double>(), op->slot_e.as<int>(), op->n_tiles, op->err.as<int>());    \
     return;                                                                                                   \

@@ -35,9 +35,8 @@ template <int N, int E, bool VEC>
 void launch_one(int grid, const void* x, const int* nodle_e, const void* fac_e, void* R, const int* slot_e,
                 int n_tiles, int* err, cudaStream_t s) {
   using P = K1Plan<Real, N, E, 1, VEC>;
-  k_local_stiffness<Real, N, E, VEC><<<grid, P::threads, P::total, s>>>(static_cast<const Real*>(x), nodle_e,
-                                                                        static_cast<const Real*>(fac_e),
-                                                                        static_cast<Real*>(R), slot_e, n_tiles, err);
+  launch_dependent(k_local_stiffness<Real, N, E, VEC>, grid, P::threads, P::total, s, static_cast<const Real*>(x),
+                   nodle_e, static_cast<const Real*>(fac_e), static_cast<Real*>(R), slot_e, n_tiles, err);
 }
 
 // (n, E) table: keep in step with k1_tile_candidates.

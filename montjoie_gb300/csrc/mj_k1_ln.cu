@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(E* N* N, LnPlan<N, E>::ctas)
     k_local_stiffness_ln(const float* __restrict__ x, const int* __restrict__ nodle_e,
                          const float* __restrict__ fac_e, float* __restrict__ R, const int* __restrict__ slot_e,
                          int n_tiles, int* __restrict__ err) {
+  dependent_wait();
   using P = LnPlan<N, E>;
   constexpr int NN = P::NN, Qp = P::Qp, RS = P::RS, W = P::W;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -268,7 +269,7 @@ void k1_launch_ln_f32(int n, int E, int grid, const void* x, const int* nodle_e,
                       const int* slot_e, int n_tiles, int* err, cudaStream_t s) {
 #define MJ_X(NV, EV)                                                                                             \
   if (n == NV && E == EV) {                                                                                      \
-    k_local_stiffness_ln<NV, EV><<<grid, LnPlan<NV, EV>::threads, LnPlan<NV, EV>::total, s>>>(                   \
+    launch_dependent(k_local_stiffness_ln<NV, EV>, grid, LnPlan<NV, EV>::threads, LnPlan<NV, EV>::total, s,                   \
         static_cast<const float*>(x), nodle_e, static_cast<const float*>(fac_e), static_cast<float*>(R), slot_e, \
         n_tiles, err);                                                                                           \
     return;                                                                                                      \

@@ -471,6 +471,7 @@ __global__ void __launch_bounds__(kStreamThreads, 8)  // 8 CTAs per SM: 32 regis
                              const unsigned* __restrict__ mask, const int* __restrict__ sidx,
                              const float* __restrict__ sval, int nsrc, const double* __restrict__ pulse, int n_pulse,
                              const double* __restrict__ inv_mass, double dt2, int* __restrict__ err, StreamDiag dg) {
+  dependent_wait();
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kStreamNB * kStreamBuf);
   const int t = threadIdx.x, G = gridDim.x;
@@ -593,6 +594,7 @@ __global__ void __launch_bounds__(kStreamThreads, 7)
                                const unsigned char* __restrict__ lists, const unsigned* __restrict__ mask,
                                const int* __restrict__ sidx, const double* __restrict__ sval, int nsrc,
                                const double* __restrict__ pulse, int n_pulse, int* __restrict__ err, StreamDiag dg) {
+  dependent_wait();
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kStreamNB * kStream64Buf);
   const int t = threadIdx.x, G = gridDim.x;
@@ -730,6 +732,7 @@ __global__ void __launch_bounds__(kStreamThreads, 8)
                        float* __restrict__ u0, const float* __restrict__ u1, const float* __restrict__ m,
                        float* __restrict__ w, float* __restrict__ z, const StreamChunk* __restrict__ chunks,
                        int n_chunks, float dt2, int* __restrict__ err) {
+  dependent_wait();
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kStreamNB * kStreamBuf);
   const int t = threadIdx.x, G = gridDim.x;

@@ -1107,13 +1107,13 @@ void lf_step4_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_
   if (prof) cudaEventRecord(lf->ev[lf->ev_used + 1], s);
   if (!EXACT && lf->stream_grid_ > 0) {  // FP32: the streaming forms
     const float* Rf = op->R.as<float>();
-    k_gather_o4_stream<0><<<lf->stream_grid_, kStreamThreads, kStreamSmem, s>>>(
+    launch_dependent(k_gather_o4_stream<0>, lf->stream_grid_, kStreamThreads, kStreamSmem, s,
         Rf, op->ptr.as<int>(), lf->ctr.as<int>(), qc, lf->pulse_d.as<double>(), lf->n_pulse,
         lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<float>(), lf->n_src_sorted, nullptr,
         nullptr, lf->minv.as<float>(), lf->w4.as<float>(), lf->z4.as<float>(), lf->stream_chunks.as<StreamChunk>(),
         lf->n_stream_chunks, float(dt2), op->err.as<int>());
     launch_k1<Real>(op, lf->z4.ptr, s);
-    k_gather_o4_stream<1><<<lf->stream_grid_, kStreamThreads, kStreamSmem, s>>>(
+    launch_dependent(k_gather_o4_stream<1>, lf->stream_grid_, kStreamThreads, kStreamSmem, s,
         Rf, op->ptr.as<int>(), lf->ctr.as<int>(), qc, lf->pulse3_d.as<double>(), lf->n_pulse3,
         lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<float>(), lf->n_src_sorted,
         static_cast<float*>(cur), static_cast<const float*>(next), lf->minv.as<float>(), lf->w4.as<float>(), nullptr,
@@ -1159,7 +1159,7 @@ void lf_step_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_t
   const double dt2 = lf->dt * lf->dt;
   if (lf->stream_gather && op->precision == MJ_FP32) {
     auto k2 = dg ? k_gather_leapfrog_stream<true> : k_gather_leapfrog_stream<false>;
-    k2<<<lf->stream_grid_, kStreamThreads, kStreamSmem, s>>>(
+    launch_dependent(k2, lf->stream_grid_, kStreamThreads, kStreamSmem, s,
         op->R.as<float>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, static_cast<float*>(cur),
         static_cast<const float*>(next), lf->minv.as<float>(), lf->stream_chunks.as<StreamChunk>(),
         lf->n_stream_chunks, lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<float>(),
@@ -1174,7 +1174,7 @@ void lf_step_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_t
   }
   if (op->precision == MJ_FP64 && lf->stream64) {
     auto k2 = dg ? k_gather_leapfrog_stream64<true> : k_gather_leapfrog_stream64<false>;
-    k2<<<lf->stream_grid_, kStreamThreads, kStream64Smem, s>>>(
+    launch_dependent(k2, lf->stream_grid_, kStreamThreads, kStream64Smem, s,
         op->R.as<double>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, static_cast<double*>(cur),
         static_cast<const double*>(next), lf->m64.as<double>(), lf->stream_chunks.as<StreamChunk>(),
         lf->n_stream_chunks, lf->stream_lists.as<unsigned char>(), lf->src_mask.as<unsigned>(),
