@@ -113,6 +113,7 @@ __device__ __forceinline__ void contrib_sums_block(const Real* __restrict__ R, c
 template <typename Real>
 __global__ void k_gather_mltadd(const Real* __restrict__ R, const int* __restrict__ ptr, Real alpha, Real beta,
                                 Real* __restrict__ y, int n_dof) {
+  dependent_wait();
   constexpr int V = kGatherV;
   for (int base = blockIdx.x * blockDim.x * V; base < n_dof; base += gridDim.x * blockDim.x * V) {
     int dv[V];
@@ -242,6 +243,7 @@ __global__ void k_gather_o4a(const Real* __restrict__ R, const int* __restrict__
                              const unsigned* __restrict__ mask, const int* __restrict__ sidx,
                              const Real* __restrict__ sval, int nsrc, const Real* __restrict__ minv, Real dt2,
                              Real* __restrict__ w, Real* __restrict__ z, int n_dof) {
+  dependent_wait();
   const int step = ctr[qc];
   const double p = step < n_pulse ? pulse[step] : 0.0;
   constexpr int V = kGatherV;
@@ -287,6 +289,7 @@ __global__ void k_gather_o4b(const Real* __restrict__ R, const int* __restrict__
                              const int* __restrict__ sidx, const Real* __restrict__ sval, int nsrc,
                              const Real* __restrict__ w, Real* __restrict__ u0, const Real* __restrict__ u1,
                              const Real* __restrict__ mass, const Real* __restrict__ minv, Real dt2, int n_dof) {
+  dependent_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) ctr[1 - qc] = ctr[qc] + 1;
   const int step = ctr[qc];
   const double p3 = step < n_pulse3 ? pulse3[step] : 0.0;

@@ -279,8 +279,8 @@ namespace {
 template <typename Real>
 int mltadd_impl(mj_op* op, double alpha, const void* x, double beta, void* y, cudaStream_t s) {
   launch_k1<Real>(op, x, s);
-  k_gather_mltadd<Real><<<stream_grid(op->n_dof), 256, 0, s>>>(op->R.as<Real>(), op->ptr.as<int>(), Real(alpha),
-                                                                Real(beta), static_cast<Real*>(y), op->n_dof);
+  launch_dependent(k_gather_mltadd<Real>, stream_grid(op->n_dof), kGatherThreads, 0, s, op->R.as<Real>(),
+                   op->ptr.as<int>(), Real(alpha), Real(beta), static_cast<Real*>(y), op->n_dof);
   count_launch();
   MJ_CUDA(cudaGetLastError());
   return MJ_OK;
@@ -1119,12 +1119,14 @@ void lf_step4_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_
         static_cast<float*>(cur), static_cast<const float*>(next), lf->minv.as<float>(), lf->w4.as<float>(), nullptr,
         lf->stream_chunks.as<StreamChunk>(), lf->n_stream_chunks, float(dt2), op->err.as<int>());
   } else {
-    k_gather_o4a<Real, EXACT><<<stream_grid(n), 256, 0, s>>>(
+    launch_dependent(
+        k_gather_o4a<Real, EXACT>, stream_grid(n), kGatherThreads, 0, s,
         op->R.as<Real>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, lf->pulse_d.as<double>(), lf->n_pulse,
         lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<Real>(), lf->n_src_sorted,
         lf->minv.as<Real>(), dt2, lf->w4.as<Real>(), lf->z4.as<Real>(), n);
     launch_k1<Real>(op, lf->z4.ptr, s);
-    k_gather_o4b<Real, EXACT><<<stream_grid(n), 256, 0, s>>>(
+    launch_dependent(
+        k_gather_o4b<Real, EXACT>, stream_grid(n), kGatherThreads, 0, s,
         op->R.as<Real>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, lf->pulse3_d.as<double>(), lf->n_pulse3,
         lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<Real>(), lf->n_src_sorted,
         lf->w4.as<Real>(), static_cast<Real*>(cur), static_cast<const Real*>(next),
