@@ -345,7 +345,8 @@ int mj_lfb_set_fused(mj_lfb* b, int enable);
 int mj_lfb_step_info(const mj_lfb* b, int* fused, int* threads, int* grid, int* n_candidates, double* candidate_ms);
 
 /* Forces the one-kernel step's variant instead of the timed choice:
- * tile_elems elements per tile; lanes thread lanes per z-line of an element
+ * tile_elems elements per tile; lanes thread lanes per z-line of an element,
+ * or per xy-plane in the variants that keep planes in registers
  * (lanes x sources_per_thread right-hand sides per pass); sources_per_thread
  * right-hand sides held by each thread.  Every variant gives the same states
  * bit for bit.  MJ_ERR_ARG when no such variant exists for the order or the
@@ -418,7 +419,10 @@ int mj_mb_set_config(mj_mb* mb, int threads);
 /* A batch of several orders also holds one sub-batch per order, each running
  * the kernel instance of its order alone; a step can then be one cooperative
  * launch per order (in increasing order) instead of one launch of the
- * all-orders kernel.  The first advance times this grouped form beside the
+ * all-orders kernel; groups on other kernels than the cooperative one step on
+ * streams of their own, joined to the batch's at the end of the advance, and
+ * an advance of a few steps takes the all-orders kernel where the groups'
+ * state copies would cost more than they gain.  The first advance times this grouped form beside the
  * two configurations of the all-orders kernel (runs restored afterwards) and
  * keeps the fastest.  Within the grouped form each group is timed both ways:
  * its batch kernel, or its runs' own step kernels (those of mj_lf_advance)
