@@ -147,9 +147,11 @@ int autotune_k1(mj_op* op) {
   double best = 1e300;
   int bestE = -1, bestGrid = 1;
   bool bestVec = false, bestWarp = false, bestPacked = false, bestFs = false, bestFx = false, bestLn = false;
-  // fixed point is timed on small meshes too: its few candidates tie in the score below, and 16^3 Q4 takes 19.0 us with
-  // 5 elements per tile, 20.8 with 4, 10^3 Q8 39.9 with 3, 43.4 with 1
-  const bool time_it = op->fac_fx.ptr || (long long)op->n_elt * op->Q >= 2000000;
+  // fixed point is timed on smaller meshes too: its few candidates tie in the score below, and 16^3 Q4 takes 19.0 us
+  // with 5 elements per tile, 20.8 with 4, 10^3 Q8 39.9 with 3, 43.4 with 1.  Below 100,000 points (8^3 Q4: 10.1
+  // against 10.6 us) the timing, 0.3 ms, would lengthen the set-up for nothing.
+  const long long points = (long long)op->n_elt * op->Q;
+  const bool time_it = points >= (op->fac_fx.ptr ? 100000 : 2000000);
   // layouts: 0 compact, 1 vector lines, 2 one element per warp, 3 the same
   // with packed connectivity, 4 compact with one factor stage (2-4: FP32), 5 fixed point (FP64: always where the
   // derivative matrix is in its range; the FP64-pipe kernel took 2.1 (Q1) to 4.4 (Q6) times as long on large meshes,
