@@ -69,16 +69,13 @@ size_t energy_smem(int S) {
 template <int N, int E, int L>
 int energy_prepare_one(int S, int* ctas) {
   using P = K1Plan<float, N, E, L>;
-  int dev = 0, optin = 0;
-  MJ_CUDA(cudaGetDevice(&dev));
-  MJ_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const size_t bytes = energy_smem<N, E, L>(S);
-  if (bytes > (size_t)optin) {
+  size_t limit = 0;
+  MJ_CUDA(allow_dynamic_smem(k_local_stiffness_rhs<N, E, L, true>, &limit));
+  if (bytes > limit) {
     set_error("adjoint gradient kernel: too many sources for its shared memory");
     return MJ_ERR_ARG;
   }
-  MJ_CUDA(cudaFuncSetAttribute(k_local_stiffness_rhs<N, E, L, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)bytes));
   MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, k_local_stiffness_rhs<N, E, L, true>, P::threads,
                                                         bytes));
   if (*ctas < 1) {

@@ -107,6 +107,23 @@ void gl_derivative_matrix(int r, const double* pts, double* g);
 
 int sm_count();
 
+// Lets a kernel be launched with any dynamic shared memory the device has room
+// for beside its static one, *limit bytes.  A kernel whose size depends on the
+// integrator (the EN steps: on S) takes this and not its own size: the
+// attribute belongs to the kernel, and a second integrator of a smaller size
+// would lower it under the first one's launches.
+template <class... P>
+cudaError_t allow_dynamic_smem(void (*kernel)(P...), size_t* limit) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (!e) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (!e) e = cudaFuncGetAttributes(&a, kernel);
+  if (e) return e;
+  *limit = (size_t)optin - a.sharedSizeBytes;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*limit);
+}
+
 // Reads a kernel's device error flag after the work on `s`; when it is set,
 // clears it (so the next call starts clean), records "<what>: <message>" and
 // returns MJ_ERR_CUDA.  Synchronises `s`.  host: a page-locked int to read it

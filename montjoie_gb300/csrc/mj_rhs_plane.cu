@@ -17,12 +17,10 @@ size_t rp_smem(int base, int E, int S, int n, bool en) {
 template <int N, int E, int LB, int V, bool EN>
 int prepare(int S, int* ctas) {
   using P = RpPlan<N, E, LB, V>;
-  int dev = 0, optin = 0;
-  MJ_CUDA(cudaGetDevice(&dev));
-  MJ_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const size_t smem = rp_smem(P::kSmem, E, S, N, EN);
-  if (smem > (size_t)optin) return MJ_OK;
-  MJ_CUDA(cudaFuncSetAttribute(k_rhs_plane<N, E, LB, V, EN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  size_t limit = 0;
+  MJ_CUDA(allow_dynamic_smem(k_rhs_plane<N, E, LB, V, EN>, &limit));
+  if (smem > limit) return MJ_OK;
   MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, k_rhs_plane<N, E, LB, V, EN>, P::T, smem));
   return MJ_OK;
 }

@@ -17,16 +17,13 @@ size_t en_smem(int base, int E, int S, int n) { return (size_t)base + (size_t)E 
 
 int rs_en_prepare(int n, int E, int LB, int V, int S, int* ctas) {
   *ctas = 0;
-  int dev = 0, optin = 0;
-  MJ_CUDA(cudaGetDevice(&dev));
-  MJ_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
 #define MJ_X(N_, E_, LB_, V_)                                                                                     \
   if (n == N_ && E == E_ && LB == LB_ && V == V_) {                                                               \
     using P = RsPlan<N_, E_, LB_, V_>;                                                                            \
     const size_t smem = en_smem(P::kSmem, E_, S, N_);                                                             \
-    if (smem > (size_t)optin) return MJ_OK;                                                                       \
-    MJ_CUDA(cudaFuncSetAttribute(k_rhs_step<N_, E_, LB_, V_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                 (int)smem));                                                                     \
+    size_t limit = 0;                                                                                             \
+    MJ_CUDA(allow_dynamic_smem(k_rhs_step<N_, E_, LB_, V_, true>, &limit));                                      \
+    if (smem > limit) return MJ_OK;                                                                               \
     MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, k_rhs_step<N_, E_, LB_, V_, true>, P::T, smem)); \
     return MJ_OK;                                                                                                 \
   }

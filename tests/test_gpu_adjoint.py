@@ -183,3 +183,24 @@ def test_every_step_variant_gives_the_same_gradient():
             m.close()
             assert J == J0, (E, LB, V, kw)
             assert np.array_equal(g, g0), (E, LB, V, kw)
+
+
+@pytest.mark.parametrize("variant", [(4, 8, 1), (2, 2, 4), None])
+def test_models_of_different_source_counts_side_by_side(variant):
+    """An 8-source and a 24-source model on the same kernels (plane form, z-line form, two-kernel form): the shared
+    memory that a gradient step needs grows with the sources, and neither model takes it from the other."""
+    models, first = [], []
+    for S in (24, 8):
+        case = build_case(S=S, nsteps=24)
+        m = make_model(case)
+        if variant:
+            m.batch.set_step_variant(*variant)
+        else:
+            m.batch.set_fused(False)
+        models.append((m, case))
+        first.append(m.loss_and_grad(case["c0"], case["data"]))
+    for (m, case), (J, g) in zip(models, first):
+        J2, g2 = m.loss_and_grad(case["c0"], case["data"])
+        assert J2 == J and np.array_equal(g2, g)
+    for m, _ in models:
+        m.close()
