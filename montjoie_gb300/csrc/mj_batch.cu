@@ -446,6 +446,7 @@ int mj_lfb_create(mj_op* op, const mj_lfb_desc* d, mj_lfb** out) {
   MJ_CUDA(b->inv_mass64.alloc(sizeof(double) * n));
   MJ_CUDA(b->pulse.alloc(sizeof(double) * std::max(1, d->n_pulse)));
   MJ_CUDA(b->ctr.alloc(sizeof(int) * 2));
+  MJ_CUDA(b->h_status.alloc(sizeof(int)));
   MJ_CUDA(b->ua.alloc(sizeof(float) * rows));
   MJ_CUDA(b->ub.alloc(sizeof(float) * rows));
   MJ_CUDA(cudaMemcpy(b->src_idx.ptr, si.data(), sizeof(int) * si.size(), cudaMemcpyHostToDevice));
@@ -583,7 +584,7 @@ int mj_lfb_advance(mj_lfb* b, int nsteps, double* traces, int trace_stride, int 
   MJ_CUDA(cudaGetLastError());
   if (diag)
     if (int rc = lfb_copy_traces(b, nsteps, traces, trace_stride, s)) return rc;
-  return take_kernel_error(b->op->err.ptr, s, "mj_lfb_advance", b->op->h_status.as<int>());
+  return take_kernel_error(b->op->err.ptr, s, "mj_lfb_advance", b->h_status.as<int>());
 }
 
 int mj_lfb_get_state(mj_lfb* b, double* u_n, double* u_np1) {
@@ -1187,7 +1188,7 @@ int mj_adj_backward(mj_adj* a, const double* residual, const double* coef, doubl
   std::vector<double> g(op->n_elt_pad);
   MJ_CUDA(cudaMemcpyAsync(g.data(), a->grad.ptr, sizeof(double) * g.size(), cudaMemcpyDeviceToHost, s));
   {
-    const int rc = take_kernel_error(op->err.ptr, s, "mj_adj_backward", op->h_status.as<int>());
+    const int rc = take_kernel_error(op->err.ptr, s, "mj_adj_backward", b->h_status.as<int>());
     if (rc) return rc;
   }
   for (int e = 0; e < op->n_elt; e++) grad[e] = g[e];

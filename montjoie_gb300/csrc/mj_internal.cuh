@@ -32,7 +32,7 @@ struct mj_op {
   std::vector<int> h_ptr;               // CSR of incidences per dof (host copy)
   double gradphi[mj::kMaxN * mj::kMaxN];
   mj::DevBuf xbuf, ybuf, stage;         // staging for host-vector MltAdd
-  mj::PinBuf h_status;                  // where kernel error flags are read (page-locked)
+  mj::PinBuf h_status;                  // where the operator's own calls read the error flag (page-locked)
   cudaStream_t stream = nullptr;
   std::vector<double> tune_ms;          // autotuner timings of the candidates (diagnostic)
   std::vector<int> tune_E, tune_vec;
@@ -58,7 +58,9 @@ struct mj_lf {
   mj::DevBuf ua, ub;         // state: U^n (cur) and U^{n+1} (next)
   mj::DevBuf du0, stage;     // staging
   mj::DevBuf partial, diag_d, flag;  // diag_d: norms, then the receivers' rows
-  mj::PinBuf h_diag;         // page-locked copy of small diagnostics, and the flag
+  // page-locked: non-finite flag, kernel error flag (ints), then a copy of small diagnostics.  Every integrator reads
+  // its flags through a word of its own: those of one operator may be advanced from several threads.
+  mj::PinBuf h_diag;
   mj::DevBuf diag_done, diag_where;  // fused diagnostics: finished-block counter, DiagDev of graph replays
   mj::DevBuf stream_partial;         // per-CTA norm partials of the streaming gather's diagnostics
   mj::DevBuf pulse_d, ctr;   // pulse of every step and the two step counters
@@ -114,6 +116,7 @@ struct mj_lfb {
   mj::DevBuf src_idx, src_val, src_rhs, m, inv_mass64, pulse, ctr;
   int n_src = 0;
   mj::DevBuf ua, ub, stage, rec_idx, rec_w, traces_d;
+  mj::PinBuf h_status;  // where kernel error flags are read (page-locked)
   int n_pulse = 0, n_rec = 0, n_rec_w = 0;
   int step = 0;
   bool cur_is_a = true, initialised = false;

@@ -129,6 +129,7 @@ struct UnionGroup {
 struct mj_mb {
   std::vector<mj_lf*> runs;
   DevBuf sync, err;
+  PinBuf h_status;  // where kernel error flags are read (page-locked)
   MeshTable table;  // kernel parameter
   std::vector<std::unique_ptr<DevBuf>> keep;  // per-run source masks and sorted sources
   std::vector<MeshDev> h_mesh;
@@ -483,9 +484,9 @@ int mb_check_err(mj_mb* mb, cudaStream_t s) {
     else if (rc) return rc;
     if (g->seq)  // runs stepped with their own kernels report through their operators
       for (mj_lf* lf : g->runs)
-        if (take_kernel_error(lf->op->err.ptr, s, "mj_mb_advance", lf->op->h_status.as<int>())) herr = 1;
+        if (take_kernel_error(lf->op->err.ptr, s, "mj_mb_advance", mb->h_status.as<int>())) herr = 1;
   }
-  if (mb->uni && take_kernel_error(mb->uni->op->err.ptr, s, "mj_mb_advance", mb->uni->op->h_status.as<int>())) herr = 1;
+  if (mb->uni && take_kernel_error(mb->uni->op->err.ptr, s, "mj_mb_advance", mb->h_status.as<int>())) herr = 1;
   int own = 0;
   MJ_CUDA(cudaMemcpyAsync(&own, mb->err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
   MJ_CUDA(cudaStreamSynchronize(s));
@@ -699,6 +700,7 @@ int mb_create(int n_runs, mj_lf* const* runs, bool split, std::unique_ptr<mj_mb>
     if (!rc) rc = mb_build_lists<128>(mb.get(), src_dofs, mb->cfg[1]);
     if (rc) return rc;
   }
+  MJ_CUDA(mb->h_status.alloc(sizeof(int)));
   MJ_CUDA(mb->sync.alloc(sizeof(SyncState)));
   MJ_CUDA(cudaMemset(mb->sync.ptr, 0, sizeof(SyncState)));
   MJ_CUDA(mb->err.alloc(sizeof(int)));

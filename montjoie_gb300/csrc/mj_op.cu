@@ -1425,7 +1425,7 @@ int lf_advance_impl(mj_lf* lf, int nsteps, double* norms, double* traces, int st
       MJ_CUDA(cudaMemcpy2DAsync(traces, sizeof(double) * stride, td, sizeof(double) * cols, sizeof(double) * cols,
                                 lf->n_rec, cudaMemcpyDeviceToHost, s));
   }
-  const int kernel_rc = take_kernel_error(lf->op->err.ptr, s, "mj_lf_advance", lf->op->h_status.as<int>());
+  const int kernel_rc = take_kernel_error(lf->op->err.ptr, s, "mj_lf_advance", hflag + 1);
   if (small) {
     if (nd) std::copy(hdata, hdata + cols, norms);
     const double* rows = hdata + (nd ? cols : 0);

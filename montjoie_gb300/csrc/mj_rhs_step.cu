@@ -371,7 +371,7 @@ int rs_rec_grid(const mj_lfb* b) {
 }
 
 int rs_check_err(mj_lfb* b, cudaStream_t s) {
-  int* herr = b->op->h_status.as<int>();
+  int* herr = b->h_status.as<int>();
   MJ_CUDA(cudaMemcpyAsync(herr, b->rs_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
   MJ_CUDA(cudaStreamSynchronize(s));
   if (*herr) {
