@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "mj_common.cuh"
@@ -61,6 +62,7 @@ struct mj_lf {
   // page-locked: non-finite flag, kernel error flag (ints), then a copy of small diagnostics.  Every integrator reads
   // its flags through a word of its own: those of one operator may be advanced from several threads.
   mj::PinBuf h_diag;
+  std::mutex stage_mutex;    // a cast into `stage` and the copy out of it are queued together (mj_lf_get_state)
   mj::DevBuf diag_done, diag_where;  // fused diagnostics: finished-block counter, DiagDev of graph replays
   mj::DevBuf stream_partial;         // per-CTA norm partials of the streaming gather's diagnostics
   mj::DevBuf pulse_d, ctr;   // pulse of every step and the two step counters

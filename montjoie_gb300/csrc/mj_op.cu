@@ -1501,6 +1501,7 @@ int mj_lf_get_state(mj_lf* lf, double* u_n, double* u_np1) {
     return MJ_ERR_STATE;
   }
   DevBuf& stage = lf->stage;
+  std::lock_guard<std::mutex> lock(lf->stage_mutex);
   int rc;
   if (u_n && (rc = download_vec(lf->op, lf->cur(), u_n, stage, lf->stream))) return rc;
   if (u_np1 && (rc = download_vec(lf->op, lf->next(), u_np1, stage, lf->stream))) return rc;

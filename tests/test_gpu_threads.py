@@ -1,4 +1,4 @@
-"""Integrators used from several host threads: each reads its own error word."""
+"""Integrators used from several host threads: each reads its own error word and stages its own copies."""
 import threading
 
 import numpy as np
@@ -6,7 +6,7 @@ import pytest
 
 from conftest import load_golden
 from montjoie_gb300 import _lib
-from montjoie_gb300.leapfrog import BatchLeapFrog
+from montjoie_gb300.leapfrog import BatchLeapFrog, LeapFrogIterator
 from montjoie_gb300.operator import FemMatrixFreeOperator
 
 pytestmark = pytest.mark.gpu
@@ -60,3 +60,24 @@ def test_a_failing_batch_beside_a_good_one():
         bad.close()
         good.close()
         op.close()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_state_read_by_several_threads(precision):
+    g = load_golden("cube4_q4")
+    n = g["massD"].size
+    op = FemMatrixFreeOperator(4, g["nodle"], g["bh"], n, precision, gradphi=g["gradphi"])
+    lf = LeapFrogIterator(op, float(g["dt"]), g["massD"])
+    lf.SetInitialConditionS(np.random.default_rng(0).uniform(-1, 1, n))
+    lf.Advance(7)
+    want = lf.GetState()
+    assert not np.array_equal(*want)
+
+    def read():
+        for _ in range(200):
+            for a, b in zip(lf.GetState(), want):
+                assert np.array_equal(a, b)
+
+    _in_threads(read, read, read)
+    lf.close()
+    op.close()
