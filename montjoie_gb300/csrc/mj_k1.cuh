@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(E* N* N)
     ph ^= 1u;
     const int* nd = s_nod(0) + pe;
 #pragma unroll
-    for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+    for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
   }
   for (int it = 0; tile < n_tiles; tile += g, ++it) {
     const int s = it & 1;
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(E* N* N)
       ph ^= 1u << so;
       const int* nd = s_nod(so) + pe;
 #pragma unroll
-      for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+      for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
     }
 
     const int* st = slot_e + ((size_t)tile * E + el) * Qp + ij;
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(E* N* N)
     ph ^= 1u;
     const int* nd = s_nod(0) + pe;
 #pragma unroll
-    for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+    for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
   }
   for (int it = 0; tile < n_tiles; tile += g, ++it) {
     const int s = it & 1;
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(E* N* N)
       ph ^= 1u << so;
       const int* nd = s_nod(so) + pe;
 #pragma unroll
-      for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+      for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
     }
 
     const int* st = slot_e + ((size_t)tile * E + el) * Qp + ij;
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(E * 32)
       for (int k = 0; k < N; k++) {
         const int w = nd[k * NN];
         const int d = PK ? (w & ((1 << kPkDofBits) - 1)) : w;
-        u[k] = __ldg(x + d);
+        u[k] = ld_fresh(x + d);
         if constexpr (PK) slot[k] = __ldg(slot_e + d) + (int)((unsigned)w >> kPkDofBits);
       }
     }
@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(E * 32)
         for (int k = 0; k < N; k++) {
           const int w = nd[k * NN];
           const int d = PK ? (w & ((1 << kPkDofBits) - 1)) : w;
-          u[k] = __ldg(x + d);
+          u[k] = ld_fresh(x + d);
           if constexpr (PK) nslot[k] = __ldg(slot_e + d) + (int)((unsigned)w >> kPkDofBits);
         }
       }

@@ -226,7 +226,7 @@ __device__ __noinline__ void fx_tile_fp64(const double* __restrict__ x, const in
   const int base = el * P::W, lx = base + j * RS, ly = base + i;
   double u[N], vz[N];
   for (int k = 0; k < N; k++) {
-    u[k] = x[nod[el * Qp + k * NN + ij]];
+    u[k] = ld_fresh(x + nod[el * Qp + k * NN + ij]);
     su[lx + k * N * RS + i] = u[k];
   }
   __syncthreads();
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     ph ^= 1u;
     const int* nd = s_nod(0) + pe;
 #pragma unroll
-    for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+    for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
     line_max(0);
   }
   __syncthreads();
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
       if (!lost) {
         const int* nd = s_nod(so) + pe;
 #pragma unroll
-        for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+        for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
       }
     }
     long long wz[N];

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(E* N* N, LnPlan<N, E>::ctas)
     ph ^= 1u;
     const int* nd = s_nod(0) + pe;
 #pragma unroll
-    for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+    for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
   }
   bool lost = false;  // the wait for this tile's Nodle (done during the previous tile) ran out
   for (int it = 0; tile < n_tiles; tile += g, ++it) {
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(E* N* N, LnPlan<N, E>::ctas)
       if (!lost) {
         const int* nd = s_nod(so) + pe;
 #pragma unroll
-        for (int k = 0; k < N; k++) u[k] = __ldg(x + nd[k * NN]);
+        for (int k = 0; k < N; k++) u[k] = ld_fresh(x + nd[k * NN]);
       }
     }
     const int* st = slot_e + ((size_t)tile * E + el) * Qp + ij;

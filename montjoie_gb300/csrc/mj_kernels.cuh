@@ -27,12 +27,12 @@ __device__ __forceinline__ void contrib_sums_global(const Real* __restrict__ R, 
     qb[v] = on[v] ? __ldg(ptr + d[v] + 1) : 0;
   }
 #pragma unroll
-  for (int v = 0; v < V; v++) first[v] = qa[v] < qb[v] ? __ldg(R + qa[v]) : Real(0);
+  for (int v = 0; v < V; v++) first[v] = qa[v] < qb[v] ? ld_fresh(R + qa[v]) : Real(0);
 #pragma unroll
   for (int v = 0; v < V; v++) {
     s[v] = Real(0);
     if (qa[v] < qb[v]) s[v] += first[v];
-    for (int q = qa[v] + 1; q < qb[v]; q++) s[v] += __ldg(R + q);
+    for (int q = qa[v] + 1; q < qb[v]; q++) s[v] += ld_fresh(R + q);
   }
 }
 
@@ -72,7 +72,7 @@ __device__ __forceinline__ void contrib_sums_block(const Real* __restrict__ R, c
     }
 #pragma unroll
     for (int v = 0; v < V; v++) {
-      s[v] = deg[v] ? __ldg(R + first[v * T + t]) : 0.0;
+      s[v] = deg[v] ? ld_fresh(R + first[v * T + t]) : 0.0;
       rank[v] = deg[v] >= 2 ? atomicAdd(&count[min(deg[v], D - 1)], 1) : 0;
     }
     __syncthreads();
@@ -94,7 +94,7 @@ __device__ __forceinline__ void contrib_sums_block(const Real* __restrict__ R, c
       const int l = list[i], n = degree[l];
       const double* q = R + first[l];
       double a = acc[l];
-      for (int k = 1; k < n; k++) a += __ldg(q + k);
+      for (int k = 1; k < n; k++) a += ld_fresh(q + k);
       acc[l] = a;
     }
     __syncthreads();
