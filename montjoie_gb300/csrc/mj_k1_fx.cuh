@@ -25,9 +25,36 @@
 //   g = sum G u     <= 2^61    h < 2^60, m < 2^62.8
 //   v = sum B' g    <= 2^60    h < 2^59, m < 2^62.4
 //   y = 3 sums G' v <= 2^62.6  h < 2^60, m < 2^62.8
-// so no accumulator overflows for any input in range.  Measured against
-// extended precision, the products are closer than the FP64 kernel's for
-// smooth, random and steep fields at every order (1e-17 to 1e-15 relative L2).
+// so no accumulator overflows for any input in range.
+//
+// Which elements.  With one scale per element a value 2^-k below the largest
+// keeps 60 - k bits where FP64 keeps 53, and the matrix spends several of the
+// 7 to spare (its entries span 2^4.7 at Q4, 2^7 at Q8).  FP64's own error at a
+// point hangs on the largest |u| on the three lines through it, each weighted
+// by its direction's factor; here the fluxes' unit, which follows the
+// element's largest gradient, decides.  So an element is computed here only if
+// that maximum is nowhere more than 2^max(1, sv + X) below the element's
+// largest |u|: sv, the bits by which the gradients are below their bound, is
+// high (5 to 13) for smooth fields and 1 to 3 for spikes; X = fx_contrast.
+// Within this the product is as close to the exact one as FP64's (restated in
+// exact integers, 177,000 elements with random, smooth and line-, edge- and
+// face-dominated fields, cubic, stretched, curved and skewed: 34 further off in
+// relative L2, by at most 3.1 times, nearly all on stretched elements; largest
+// error of an entry over its absolute sum in units of 2^-53, in 99.9% of the
+// elements and at most: Q4 3.2 and 11, FP64 6.4; Q8 13 and 20, FP64 11; the
+// bound of FP64 arithmetic is 16 and 24).  Without it a field that peaks at a
+// vertex lost up to 87 times in L2.
+// All other elements (spikes, the numerical tail ahead of a front; factors that
+// vary by more than 2.5 along an element, which is known when they are
+// converted) take the FP64 arithmetic of k_local_stiffness on their own
+// threads, beside the others of the tile (fx_exact_*), and so does an element
+// out of range (a NaN or infinity in u or B, or scales whose result would leave
+// the normal range).  The choice hangs on the element alone, not on the tile it
+// is in.  Of smooth waves 2.5 elements long or more, fewer than 0.04% of the
+// elements take it.  The FP64 pipe takes 16 clocks per warp instruction, so one
+// such element keeps its tile for 7 us at Q4 and 22 us at Q8, and a field of
+// spikes takes what the FP64-pipe kernel does (16^3 Q4 57 and 61 us per
+// product, 15x13x11 Q8 260 and 237).
 //
 // Measured (us per launch, FP64-pipe kernel at its best tile -> this kernel):
 // Q4 16^3 60 -> 20, 64^3 2300 -> 598; Q8 15x13x11-sized 359 -> 94, 32^3 3150
@@ -37,10 +64,6 @@
 // half of its rate.  Without the lo*lo term it takes 15% less and errs up to
 // 3 times more than the FP64 kernel on steep fields; with the mirror symmetry
 // it takes 25% less than in the general form.
-//
-// A tile with an element out of range (a NaN or infinity in u or B, or scales
-// whose result would leave the normal range) takes the FP64 arithmetic of
-// k_local_stiffness instead (fx_tile_fp64), so such values propagate as there.
 //
 // Layout: E elements per CTA, E*n*n threads.  A thread owns a z-line in the
 // gather, the z-contractions, the factor products and the result, and an
@@ -68,7 +91,9 @@
 namespace mj {
 namespace {
 
-constexpr int kFxBad = INT_MIN;  // fac_exp of an element whose factors are not finite
+// fac_exp of an element: the scale kb of its factors << 12 | s_z << 8 | s_y << 4 | s_x, s_d the factors' weight of
+// direction d against the largest, as a power of two downwards; kFxBad: not finite or too uneven.
+constexpr int kFxBad = INT_MIN;
 
 // Coefficients of the line transforms of every order as (lo, hi, lo >> 17),
 // and their scales.  [n][0]: gradient, y_l = sum_a G[a][l] r_a; [n][1]:
@@ -81,7 +106,12 @@ __constant__ int c_fx_exp[kMaxNK + 1];  // sum of both scales
 // Exponent of the similarity scaling at node i of n (see above).
 __host__ __device__ constexpr int fx_c(int n, int i) {
   const int d = i < n - 1 - i ? i : n - 1 - i;  // distance from the nearer end
-  return d == 0 ? (n == 2 ? 0 : n == 3 ? 1 : 2) : d == 1 && n >= 6 ? 1 : 0;
+  return d == 0 ? (n == 2 ? 0 : n <= 6 ? 2 : 3) : d == 1 && n >= 6 ? 1 : 0;
+}
+
+// X of the contrast rule (see above).
+__host__ __device__ constexpr int fx_contrast(int n) {
+  return n <= 4 ? 3 - n : n == 5 ? -1 : n <= 7 ? -2 : -3;
 }
 
 __device__ __forceinline__ int2 fx_limbs(long long v) {
@@ -204,7 +234,7 @@ struct FxPlan {
   static constexpr size_t fac_bytes = sizeof(int2) * 6 * E * Qp;
   static constexpr size_t nod_bytes = sizeof(int) * E * Qp;
   static constexpr size_t work_bytes = ((sizeof(long long) * 3 * E * W + 15) / 16) * 16;
-  static constexpr size_t max_bytes = ((sizeof(unsigned) * 3 * E + 15) / 16) * 16;
+  static constexpr size_t max_bytes = ((sizeof(unsigned) * 4 * E + 15) / 16) * 16;
   static constexpr size_t max_at = fac_bytes + 2 * nod_bytes + work_bytes;
   static constexpr size_t total = max_at + max_bytes + 3 * sizeof(uint64_t);
   static constexpr int threads = E * NN;
@@ -213,52 +243,117 @@ struct FxPlan {
   static_assert(fac_bytes % 16 == 0 && nod_bytes % 16 == 0, "bulk copies");
 };
 
-// The tile in FP64: the arithmetic of k_local_stiffness<double> (compact).
-// Every thread of the CTA calls it; work arrays are free on entry and exit.
+// An element in FP64, the arithmetic of k_local_stiffness<double> (compact) in
+// the three phases of the tile, by the element's threads; su, sa, sb: its work
+// arrays, u staged in su.  ij: the thread's z-line.  Three points at a time: a
+// tile waits for its elements here, and one point is a chain of up to 3 n
+// dependent FP64 operations.
+// Gradients along x and y of the thread's points into sa and sb.
 template <int N, int E>
-__device__ __noinline__ void fx_tile_fp64(const double* __restrict__ x, const int* nod, const double* __restrict__ fac,
-                                          double* __restrict__ R, const int* __restrict__ slot, double* su, double* sa,
-                                          double* sb) {
-  using P = FxPlan<N, E>;
-  constexpr int NN = P::NN, Qp = P::Qp, RS = P::RS;
+__device__ __noinline__ void fx_exact_gradient(const double* su, double* sa, double* sb, int ij) {
+  constexpr int RS = FxPlan<N, E>::RS;
   const double* __restrict__ G = c_gmat64[N];
-  const int el = threadIdx.x / NN, ij = threadIdx.x - el * NN, j = ij / N, i = ij - j * N;
-  const int base = el * P::W, lx = base + j * RS, ly = base + i;
-  double u[N], vz[N];
+  const int j = ij / N, i = ij - j * N;
+#pragma unroll 3
   for (int k = 0; k < N; k++) {
-    u[k] = ld_fresh(x + nod[el * Qp + k * NN + ij]);
-    su[lx + k * N * RS + i] = u[k];
-  }
-  __syncthreads();
-  const double* f = fac + (size_t)el * 6 * Qp + ij;
+    const double *rx = su + (k * N + j) * RS, *ry = su + k * N * RS + i;
+    double gx = 0, gy = 0;
 #pragma unroll
-  for (int k = 0; k < N; k++) {
-    double gx = 0, gy = 0, gz = 0;
-#pragma unroll 1
     for (int a = 0; a < N; a++) {
-      gx += G[a * N + i] * su[lx + k * N * RS + a];
-      gy += G[a * N + j] * su[ly + k * N * RS + a * RS];
+      gx += G[a * N + i] * rx[a];
+      gy += G[a * N + j] * ry[a * RS];
     }
+    sa[(k * N + j) * RS + i] = gx;
+    sb[(k * N + j) * RS + i] = gy;
+  }
+}
+
+// Fluxes of the thread's points, over their gradients and (along z) over u.
+template <int N, int E>
+__device__ __noinline__ void fx_exact_flux(double* su, double* sa, double* sb, const double* __restrict__ fac, int ij) {
+  constexpr int NN = N * N, Qp = FxPlan<N, E>::Qp, RS = FxPlan<N, E>::RS;
+  const double* __restrict__ G = c_gmat64[N];
+  const int at = ij / N * RS + ij % N;
+  double u[N];
+#pragma unroll
+  for (int a = 0; a < N; a++) u[a] = su[at + a * N * RS];
+#pragma unroll 3
+  for (int k = 0; k < N; k++) {
+    const double* f = fac + k * NN + ij;
+    const double bxx = f[0], bxy = f[Qp], bxz = f[2 * Qp], byy = f[3 * Qp], byz = f[4 * Qp], bzz = f[5 * Qp];
+    const double gx = sa[at + k * N * RS], gy = sb[at + k * N * RS];
+    double gz = 0;
 #pragma unroll
     for (int a = 0; a < N; a++) gz += G[a * N + k] * u[a];
-    const double* fk = f + k * NN;
-    const double bxx = fk[0], bxy = fk[Qp], bxz = fk[2 * Qp], byy = fk[3 * Qp], byz = fk[4 * Qp], bzz = fk[5 * Qp];
-    sa[lx + k * N * RS + i] = fac_dot(bxx, gx, bxy, gy, bxz, gz);
-    sb[lx + k * N * RS + i] = fac_dot(bxy, gx, byy, gy, byz, gz);
-    vz[k] = fac_dot(bxz, gx, byz, gy, bzz, gz);
+    sa[at + k * N * RS] = fac_dot(bxx, gx, bxy, gy, bxz, gz);
+    sb[at + k * N * RS] = fac_dot(bxy, gx, byy, gy, byz, gz);
+    su[at + k * N * RS] = fac_dot(bxz, gx, byz, gy, bzz, gz);
   }
-  __syncthreads();
-#pragma unroll
+}
+
+// Divergence at the thread's points into R.
+template <int N, int E>
+__device__ __noinline__ void fx_exact_divergence(const double* su, const double* sa, const double* sb,
+                                                 double* __restrict__ R, const int* __restrict__ slot, int ij) {
+  constexpr int NN = N * N, RS = FxPlan<N, E>::RS;
+  const double* __restrict__ G = c_gmat64[N];
+  const int j = ij / N, i = ij - j * N;
+#pragma unroll 3
   for (int k = 0; k < N; k++) {
+    const double *rx = sa + (k * N + j) * RS, *ry = sb + k * N * RS + i, *rz = su + j * RS + i;
     double y = 0;
 #pragma unroll
     for (int a = 0; a < N; a++) {
-      y += G[i * N + a] * sa[lx + k * N * RS + a];
-      y += G[j * N + a] * sb[ly + k * N * RS + a * RS];
-      y += G[k * N + a] * vz[a];
+      y += G[i * N + a] * rx[a];
+      y += G[j * N + a] * ry[a * RS];
+      y += G[k * N + a] * rz[a * N * RS];
     }
-    R[slot[el * Qp + k * NN + ij]] = y;
+    R[slot[k * NN + ij]] = y;
   }
+}
+
+// The contrast rule for the elements of a tile with a thread that is bad (its
+// element is out of range) or whose z-line lies low; every thread of the CTA
+// calls it, u staged as integers in s_u; scratch: 2 N^2 words per element.
+// um: the element's largest |u| (high word), shift: the exponent of the rule.
+// True: this thread's element is computed in FP64.
+template <int N, int E>
+__device__ __noinline__ bool fx_choose(const long long* s_u, unsigned* scratch, int* s_mode, bool bad, bool low,
+                                       unsigned um, int xp, int shift, int ij) {
+  using P = FxPlan<N, E>;
+  constexpr int NN = P::NN, RS = P::RS, W = P::W;
+  const int el = threadIdx.x / NN, j = ij / N, i = ij - j * N;
+  if (bad || low) atomicOr(&s_mode[el], bad ? 2 : 1);
+  __syncthreads();
+  const bool look = s_mode[el] == 1;
+  unsigned* line = scratch + el * 2 * NN;  // largest |u| of the x-lines, then of the y-lines
+  unsigned zm = 0u;
+  auto mag = [&](int at) {
+    const int hi = (int)(s_u[el * W + at] >> 32);
+    return (unsigned)(hi ^ (hi >> 31));
+  };
+  if (look) {
+    unsigned xm = 0u, ym = 0u;
+#pragma unroll 1
+    for (int a = 0; a < N; a++) {
+      xm = max(xm, mag(ij * RS + a));
+      ym = max(ym, mag((ij / N * N + a) * RS + ij % N));
+      zm = max(zm, mag((a * N + j) * RS + i));
+    }
+    line[ij] = xm >> (xp & 15);
+    line[NN + ij] = ym >> (xp >> 4 & 15);
+    zm >>= xp >> 8 & 15;
+  }
+  __syncthreads();
+  if (look) {
+    const unsigned least = (((um & 0xfffffu) | 0x100000u) << (kFxBitsU - 52)) >> shift;
+    bool out = false;
+#pragma unroll 1
+    for (int k = 0; k < N; k++) out |= max(max(line[k * N + j], line[NN + k * N + i]), zm) < least;
+    if (out) atomicOr(&s_mode[el], 2);
+  }
+  __syncthreads();
+  return s_mode[el] & 2;
 }
 
 template <int N, int E, bool SYM>
@@ -278,6 +373,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
   long long* s_b = s_a + E * W;
   unsigned* s_max = reinterpret_cast<unsigned*>(smem + P::max_at);  // [2][E]: largest |u| (high word) of the tile's and
   unsigned* s_gmax = s_max + 2 * E;                                 // the next tile's elements; [E]: largest |g|
+  int* s_mode = reinterpret_cast<int*>(s_max + 3 * E);  // [E]: bit 0: a z-line lies low, bit 1: the element in FP64
   // bar[0], bar[1]: the Nodle stages; bar[2]: the factor stage
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + P::max_at + P::max_bytes);
 
@@ -297,7 +393,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     mbar_init(&bar[2], 1);
     fence_mbar_init();
   }
-  for (int q = t; q < 3 * E; q += P::threads) s_max[q] = 0u;
+  for (int q = t; q < 4 * E; q += P::threads) s_max[q] = 0u;
   __syncthreads();
   auto issue_nod = [&](int st, int tile) {
     if (t == 0 && tile < n_tiles) {
@@ -320,13 +416,14 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
   issue_nod(1, tile + g);
   uint32_t ph = 0u;  // bits 0, 1: parity of the next completion of Nodle stage 0, 1; bit 2: of the factor stage
   double u[N];
-  // largest high word of |u| over the thread's line (nonzero for any nonzero u), into the element's maximum
+  unsigned zm = 0u;
+  // zm: largest high word of |u| over the thread's line (nonzero for any nonzero u); into the element's maximum
   auto line_max = [&](int par) {
-    unsigned m = 0u;
+    zm = 0u;
 #pragma unroll
     for (int k = 0; k < N; k++)
-      m = max(m, ((unsigned)__double2hiint(u[k]) & 0x7fffffffu) | (__double2loint(u[k]) != 0 ? 1u : 0u));
-    atomicMax(&s_max[par * E + el], m);
+      zm = max(zm, ((unsigned)__double2hiint(u[k]) & 0x7fffffffu) | (__double2loint(u[k]) != 0 ? 1u : 0u));
+    atomicMax(&s_max[par * E + el], zm);
   };
   if (tile < n_tiles) {
     const bool ok = mbar_wait_bounded(&bar[0], 0u);
@@ -351,11 +448,13 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     const int s = it & 1;
     // the element's scales: u 2^ku, B 2^kb, result 2^eo
     const unsigned um = s_max[s * E + el];
-    const int kb = __ldg(fac_exp + (size_t)tile * E + el);
+    const int xp = __ldg(fac_exp + (size_t)tile * E + el);
     const int eu = (int)(um >> 20) - 1023;
     const int ku = um ? kFxBitsU - eu : 0;
-    const int eo = kFxYBias - ku - (kb == kFxBad ? 0 : kb) - kg;
-    const bool bad = kb == kFxBad || (um && (eu > 1023 || eu < -900 || eo < -950 || eo > 1000));
+    const int eo = kFxYBias - ku - (xp == kFxBad ? 0 : xp >> 12) - kg;
+    const bool bad = xp == kFxBad || (um && (eu > 1023 || eu < -900 || eo < -950 || eo > 1000));
+    // this thread's z-line below the element's largest |u|, weighted, in units of 2^-20 of a power of two
+    const int below = (int)min(um - zm + ((xp >> 8 & 15u) << 20), 0x7fffffffu);
     long long uz[N];
     {
       const double sc = __hiloint2double((1023 + (bad ? 0 : ku)) << 20, 0);
@@ -365,10 +464,9 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
         s_u[lz + k * N * RS] = uz[k];
       }
     }
-    const bool fp64 = __syncthreads_or(bad);  // also: u staged, the maxima read
-    if (t < E) s_max[s * E + t] = 0u;
+    __syncthreads();  // u staged, the maxima read
     long long gz[N];
-    if (!fp64) {
+    {
       long long r[N], y[N];
 #pragma unroll
       for (int a = 0; a < N; a++) r[a] = s_u[lx + a];
@@ -409,7 +507,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     long long vz[N];
     // |g| < 2^(64 - lz) with lz >= 2 leading zeros: |v| < 2^62 2^(64 - lz) / 2^(64 - sv) <= 2^60
     const int sv = min(31, __clz((int)s_gmax[el]) - 2);
-    if (!fp64) {
+    {
       const int2* f = s_fac + el * 6 * Qp + ij;
 #pragma unroll
       for (int k = 0; k < N; k++) {
@@ -427,12 +525,26 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
         s_b[lz + k * N * RS] = b.norm(sv);
         vz[k] = c.norm(sv);
       }
-    } else {
-      fx_tile_fp64<N, E>(x, s_nod(s), fac_e + (size_t)tile * E * 6 * Qp, R, slot_e + (size_t)tile * E * Qp,
-                         reinterpret_cast<double*>(s_u), reinterpret_cast<double*>(s_a),
-                         reinterpret_cast<double*>(s_b));
     }
-    __syncthreads();  // the factor stage is free, the fluxes are staged
+    bool exact = false;  // this thread's element in FP64
+    const int shift = max(1, sv + fx_contrast(N));
+    if (__syncthreads_or(bad || below > shift << 20)) {  // also: the factor stage is free, the fluxes are staged
+      double *su = reinterpret_cast<double*>(s_u + el * W), *sa = reinterpret_cast<double*>(s_a + el * W);
+      double* sb = reinterpret_cast<double*>(s_b + el * W);
+      const size_t e = (size_t)tile * E + el;
+      exact = fx_choose<N, E>(s_u, reinterpret_cast<unsigned*>(s_fac), s_mode, bad, below > shift << 20,
+                              s_max[s * E + el], __ldg(fac_exp + e), shift, ij);
+      if (exact)
+#pragma unroll
+        for (int k = 0; k < N; k++) s_u[lz + k * N * RS] = __double_as_longlong(u[k]);
+      __syncthreads();
+      if (t < E) s_mode[t] = 0;
+      if (exact) fx_exact_gradient<N, E>(su, sa, sb, ij);
+      __syncthreads();
+      if (exact) fx_exact_flux<N, E>(su, sa, sb, fac_e + e * 6 * Qp, ij);
+      __syncthreads();
+    }
+    if (t < E) s_max[s * E + t] = 0u;
     if (t < E) s_gmax[t] = 0u;
     if (t == 0) fence_proxy_async();
     issue_fac(tile + g);  // the next tile's factors, during this divergence
@@ -451,7 +563,10 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
       }
     }
     long long wz[N];
-    if (!fp64) {
+    if (exact) {
+      fx_exact_divergence<N, E>(reinterpret_cast<double*>(s_u + el * W), reinterpret_cast<double*>(s_a + el * W),
+                                reinterpret_cast<double*>(s_b + el * W), R, slot_e + ((size_t)tile * E + el) * Qp, ij);
+    } else {
       long long r[N], y[N];
 #pragma unroll
       for (int a = 0; a < N; a++) r[a] = s_a[lx + a];
@@ -476,7 +591,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     }
     if (t == 0) fence_proxy_async();
     issue_nod(s, tile + 2 * g);
-    if (!fp64) {
+    if (!exact) {
       const int ex = 1023 + (um ? eo - sv : 9) - fx_c(N, i) - fx_c(N, j);
       const int* st = slot_e + ((size_t)tile * E + el) * Qp + ij;
 #pragma unroll

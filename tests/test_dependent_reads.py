@@ -22,7 +22,7 @@ def test_no_read_only_loads_of_what_the_kernel_before_writes():
     for path in glob.glob(os.path.join(ROOT, "montjoie_gb300", "csrc", "mj_k*")):
         for head, body in _functions(re.sub(r"//.*", "", open(path).read())):
             dependent = "dependent_wait();" in body
-            if dependent or re.search(r"contrib_sums_(global|block)\(|fx_tile_fp64\(", head):
+            if dependent or re.search(r"contrib_sums_(global|block)\(", head):
                 dependents += dependent
                 readers += "ld_fresh(" in body
                 assert not re.search(r"__ldg\(\s*[xR]\b", body), (path, head)
