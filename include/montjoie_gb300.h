@@ -182,6 +182,11 @@ uint64_t mj_kernel_launches(void);
  * were captured with. */
 int mj_debug_set_wait_limits(long long mbar_polls, long long barrier_polls, long long barrier_ns);
 
+/* Test hook, no reference counterpart: from now on device allocations of the
+ * library that would take it more than more_bytes beyond what it holds fail
+ * as if the device were full (negative: no limit).  Process-wide. */
+int mj_debug_set_memory_limit(long long more_bytes);
+
 /* ---- leap-frog time loop -------------------------------------------- */
 
 typedef struct {

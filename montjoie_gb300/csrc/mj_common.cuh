@@ -50,6 +50,13 @@ inline void count_launch(uint64_t n = 1) { launch_counter().fetch_add(n, std::me
     }                                      \
   } while (0)
 
+// Device memory that the library holds, and the most it may hold (a test's
+// limit; none by default).
+struct DeviceMemory {
+  std::atomic<size_t> held{0}, limit{SIZE_MAX};
+};
+DeviceMemory& device_memory();
+
 // Device buffer owned by the library (cudaMalloc/cudaFree).
 struct DevBuf {
   void* ptr = nullptr;
@@ -59,15 +66,26 @@ struct DevBuf {
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (ptr) cudaFree(ptr);
+    if (ptr) {
+      cudaFree(ptr);
+      device_memory().held -= bytes;
+    }
     ptr = nullptr;
     bytes = 0;
   }
   cudaError_t alloc(size_t b) {
     release();
-    bytes = b;
     if (b == 0) return cudaSuccess;
-    return cudaMalloc(&ptr, b);
+    DeviceMemory& m = device_memory();
+    if (m.held + b > m.limit) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMalloc(&ptr, b);
+    if (e) {
+      ptr = nullptr;
+      return e;
+    }
+    bytes = b;
+    m.held += b;
+    return cudaSuccess;
   }
   template <class T>
   T* as() const { return static_cast<T*>(ptr); }

@@ -49,7 +49,7 @@ struct mj_lf {
   double dt = 0;
   int n_dof = 0;
   mj::DevBuf src_idx, src_val;  // sparse source (value in op precision)
-  mj::DevBuf mass, minv;     // op precision (FP64: D and 1/D; FP32: unused / dt^2/D)
+  mj::DevBuf mass, minv;     // op precision (FP64: D, and 1/D in inv_mass64; FP32: unused / dt^2/D)
   mj::DevBuf inv_mass64;     // FP64 1/D for the initial step
   mj::DevBuf norm_w;         // FP64 weights, or empty
   mj::DevBuf norm_w32;       // the same rounded to FP32 (FP32 integrators), or empty
@@ -97,6 +97,9 @@ struct mj_lf {
   mj::DevBuf stream_chunks;
   mj::DevBuf m64, stream_lists;  // FP64: dt^2/D, and each chunk's dofs with several contributions
   int n_stream_chunks = 0, stream_grid_ = 0;
+  // 1/D (FP64) or dt^2/D (FP32) in the operator's precision
+  template <class Real>
+  const Real* minv_as() const { return static_cast<const Real*>(minv.ptr ? minv.ptr : inv_mass64.ptr); }
   ~mj_lf() {
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
     if (graph) cudaGraphExecDestroy(graph);

@@ -23,6 +23,11 @@ thread_local std::string g_last_error;
 
 void set_error(const std::string& msg) { g_last_error = msg; }
 
+DeviceMemory& device_memory() {
+  static DeviceMemory* m = new DeviceMemory;  // outlives buffers freed at exit
+  return *m;
+}
+
 std::atomic<uint64_t>& launch_counter() {
   static std::atomic<uint64_t> c{0};
   return c;
@@ -435,12 +440,20 @@ int op_finish(mj_op* op) {
   int rc = op->precision == MJ_FP64 ? k1_set_gmat_f64(op->n, op->gradphi) : k1_set_gmat_f32(op->n, op->gradphi);
   if (rc) return rc;
   if (op->precision == MJ_FP64 && k1_fx_supports(op->n, op->gradphi, &op->fx_sym)) {
-    rc = k1_set_gmat_fx(op->n, op->gradphi, op->fx_sym);
-    if (rc) return rc;
-    MJ_CUDA(op->fac_fx.alloc(op->fac_e.bytes));
-    MJ_CUDA(op->fac_exp.alloc(sizeof(int) * op->n_elt_pad));
-    rc = k1_fixed_factors(op, op->stream);
-    if (rc) return rc;
+    // the factors a second time, as limbs (48 bytes per point); where they do not fit the FP64-pipe kernel runs from
+    // fac_e alone.  Room for the vectors of a product or a run on this operator is left: 8 of n_dof doubles.
+    DevBuf room;
+    if (room.alloc(8 * sizeof(double) * (size_t)op->n_dof) == cudaSuccess &&
+        op->fac_fx.alloc(op->fac_e.bytes) == cudaSuccess &&
+        op->fac_exp.alloc(sizeof(int) * op->n_elt_pad) == cudaSuccess) {
+      rc = k1_set_gmat_fx(op->n, op->gradphi, op->fx_sym);
+      if (!rc) rc = k1_fixed_factors(op, op->stream);
+      if (rc) return rc;
+    } else {
+      cudaGetLastError();  // out of memory is not an error here
+      op->fac_fx.release();
+      op->fac_exp.release();
+    }
   }
   return autotune_k1(op);
 }
@@ -742,6 +755,12 @@ int mj_op_mltadd(mj_op* op, double alpha, const double* x, double beta, double* 
   return take_kernel_error(op->err.ptr, s, "mj_op_mltadd", op->h_status.as<int>());
 }
 
+int mj_debug_set_memory_limit(long long more_bytes) {
+  DeviceMemory& m = device_memory();
+  m.limit = more_bytes < 0 ? SIZE_MAX : m.held + (size_t)more_bytes;
+  return MJ_OK;
+}
+
 int mj_debug_set_wait_limits(long long mbar_polls, long long barrier_polls, long long barrier_ns) {
   mj::k1_waits_run_out() = mbar_polls == 0;
   mj::WaitLimits w;
@@ -910,9 +929,7 @@ int mj_lf_create(mj_op* op, const mj_lf_desc* desc, mj_lf** out) {
     if (desc->n_src)
       MJ_CUDA(cudaMemcpy(lf->src_val.ptr, desc->src_val, sizeof(double) * desc->n_src, cudaMemcpyHostToDevice));
     MJ_CUDA(lf->mass.alloc(sizeof(double) * n));
-    MJ_CUDA(lf->minv.alloc(sizeof(double) * n));
     MJ_CUDA(cudaMemcpy(lf->mass.ptr, desc->mass, sizeof(double) * n, cudaMemcpyHostToDevice));
-    MJ_CUDA(cudaMemcpy(lf->minv.ptr, lf->inv_mass64.ptr, sizeof(double) * n, cudaMemcpyDeviceToDevice));
   } else {
     std::vector<float> sv(std::max(1, desc->n_src)), m(n);
     for (int s = 0; s < desc->n_src; s++) sv[s] = (float)desc->src_val[s];
@@ -970,20 +987,30 @@ int mj_lf_create(mj_op* op, const mj_lf_desc* desc, mj_lf** out) {
   } else {
     // the streaming form when 1/D is the reciprocal of D (a caller's own array may be something else);
     // m64 padded by 4 entries like the states (16-byte rounded bulk copies)
-    DevBuf other;
-    int h_other = 0;
-    MJ_CUDA(other.alloc(sizeof(int)));
-    MJ_CUDA(cudaMemset(other.ptr, 0, sizeof(int)));
-    MJ_CUDA(lf->m64.alloc(sizeof(double) * (n + 4)));
-    MJ_CUDA(cudaMemset(lf->m64.ptr, 0, sizeof(double) * (n + 4)));
-    k_dt2_over_mass<<<stream_grid(n), 256>>>(lf->inv_mass64.as<double>(), lf->mass.as<double>(), desc->dt * desc->dt,
-                                             lf->m64.as<double>(), n, other.as<int>());
-    count_launch();
-    MJ_CUDA(cudaMemcpy(&h_other, other.ptr, sizeof(int), cudaMemcpyDeviceToHost));
-    if (!h_other) {
-      int rc = lf_sorted_sources(lf.get());
-      if (!rc) rc = lf_stream_setup(lf.get(), &lf->stream64);
-      if (rc) return rc;
+    auto stream64 = [&]() -> int {
+      DevBuf other;
+      int h_other = 0;
+      MJ_CUDA(other.alloc(sizeof(int)));
+      MJ_CUDA(cudaMemset(other.ptr, 0, sizeof(int)));
+      MJ_CUDA(lf->m64.alloc(sizeof(double) * (n + 4)));
+      MJ_CUDA(cudaMemset(lf->m64.ptr, 0, sizeof(double) * (n + 4)));
+      k_dt2_over_mass<<<stream_grid(n), 256>>>(lf->inv_mass64.as<double>(), lf->mass.as<double>(),
+                                               desc->dt * desc->dt, lf->m64.as<double>(), n, other.as<int>());
+      count_launch();
+      MJ_CUDA(cudaMemcpy(&h_other, other.ptr, sizeof(int), cudaMemcpyDeviceToHost));
+      if (h_other) return MJ_OK;
+      if (int rc = lf_sorted_sources(lf.get())) return rc;
+      return lf_stream_setup(lf.get(), &lf->stream64);
+    };
+    const int rc = stream64();
+    if (rc && rc != MJ_ERR_NOMEM) return rc;
+    if (rc || !lf->stream64) {  // its arrays do not fit or serve nothing: the gather and source kernels need none
+      cudaGetLastError();
+      lf->stream64 = false;
+      lf->stream_grid_ = 0;
+      for (DevBuf* b : {&lf->m64, &lf->stream_lists, &lf->stream_chunks, &lf->stream_partial, &lf->src_mask,
+                        &lf->src_sidx, &lf->src_sval})
+        b->release();
     }
   }
   *out = lf.release();
@@ -1125,14 +1152,14 @@ void lf_step4_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_
         k_gather_o4a<Real, EXACT>, stream_grid(n), kGatherThreads, 0, s,
         op->R.as<Real>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, lf->pulse_d.as<double>(), lf->n_pulse,
         lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<Real>(), lf->n_src_sorted,
-        lf->minv.as<Real>(), dt2, lf->w4.as<Real>(), lf->z4.as<Real>(), n);
+        lf->minv_as<Real>(), dt2, lf->w4.as<Real>(), lf->z4.as<Real>(), n);
     launch_k1<Real>(op, lf->z4.ptr, s);
     launch_dependent(
         k_gather_o4b<Real, EXACT>, stream_grid(n), kGatherThreads, 0, s,
         op->R.as<Real>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, lf->pulse3_d.as<double>(), lf->n_pulse3,
         lf->src_mask.as<unsigned>(), lf->src_sidx.as<int>(), lf->src_sval.as<Real>(), lf->n_src_sorted,
         lf->w4.as<Real>(), static_cast<Real*>(cur), static_cast<const Real*>(next),
-        EXACT ? lf->mass.as<Real>() : nullptr, lf->minv.as<Real>(), dt2, n);
+        EXACT ? lf->mass.as<Real>() : nullptr, lf->minv_as<Real>(), dt2, n);
   }
   count_launch(2);
   if (prof) {
@@ -1194,11 +1221,11 @@ void lf_step_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_t
   if (op->precision == MJ_FP64) {
     k_gather_leapfrog<Real, true><<<stream_grid(n), 256, 0, s>>>(
         op->R.as<Real>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, static_cast<Real*>(cur),
-        static_cast<const Real*>(next), lf->mass.as<Real>(), lf->minv.as<Real>(), Real(dt2), n);
+        static_cast<const Real*>(next), lf->mass.as<Real>(), lf->minv_as<Real>(), Real(dt2), n);
   } else {
     k_gather_leapfrog<Real, false><<<stream_grid(n), 256, 0, s>>>(
         op->R.as<Real>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, static_cast<Real*>(cur),
-        static_cast<const Real*>(next), nullptr, lf->minv.as<Real>(), Real(dt2), n);
+        static_cast<const Real*>(next), nullptr, lf->minv_as<Real>(), Real(dt2), n);
   }
   if (lf->n_src) {
     k_source<Real><<<(lf->n_src + 255) / 256, 256, 0, s>>>(lf->src_idx.as<int>(), lf->src_val.as<Real>(), lf->n_src,
