@@ -426,10 +426,11 @@ int mj_mb_set_config(mj_mb* mb, int threads);
  * launch per order (in increasing order) instead of one launch of the
  * all-orders kernel; groups on other kernels than the cooperative one step on
  * streams of their own, joined to the batch's at the end of the advance, and
- * an advance of a few steps takes the all-orders kernel where the groups'
- * state copies would cost more than they gain.  The first advance times this grouped form beside the
- * two configurations of the all-orders kernel (runs restored afterwards) and
- * keeps the fastest.  Within the grouped form each group is timed both ways:
+ * an advance of a few steps takes the runs' own kernels in place of the
+ * unions (below) where the state copies would cost more than they gain: the
+ * bits are the same, however a run is split into advances.  The first advance
+ * times this grouped form beside the two configurations of the all-orders
+ * kernel (runs restored afterwards) and keeps the fastest.  Within the grouped form each group is timed both ways:
  * its batch kernel, or its runs' own step kernels (those of mj_lf_advance)
  * one run after the other, and keeps the faster (large meshes of high order
  * run well on their own kernels, many small ones batched).  Reports whether

@@ -114,6 +114,19 @@ static __global__ void k_union_states(const __grid_constant__ UnionStates runs, 
   }
 }
 
+// The error flags of a batch's kernels (kernel parameter): the batch's, its
+// groups' and their unions' (at most 2 + 2 x 8), and its runs'.
+constexpr int kMaxFlags = 96;
+struct ErrorFlags {
+  int* f[kMaxFlags];
+  int n = 0;
+};
+static_assert(kMaxRuns + 18 <= kMaxFlags, "every flag of a batch");
+
+static __global__ void k_read_flags(const __grid_constant__ ErrorFlags t, int* __restrict__ out) {
+  if ((int)threadIdx.x < t.n) out[threadIdx.x] = *t.f[threadIdx.x];
+}
+
 // A group's runs stepped as one union operator (lf_union_create).
 struct UnionGroup {
   std::unique_ptr<mj_op> op;
@@ -129,7 +142,8 @@ struct UnionGroup {
 struct mj_mb {
   std::vector<mj_lf*> runs;
   DevBuf sync, err;
-  PinBuf h_status;  // where kernel error flags are read (page-locked)
+  DevBuf flags;     // copy of every error flag of the batch
+  PinBuf h_status;  // where it is read (page-locked)
   MeshTable table;  // kernel parameter
   std::vector<std::unique_ptr<DevBuf>> keep;  // per-run source masks and sorted sources
   std::vector<MeshDev> h_mesh;
@@ -159,8 +173,11 @@ struct mj_mb {
   std::unique_ptr<UnionGroup> uni;
   bool force_union = false;  // mj_mb_set_config(-2)
   // What an advance of the timed form costs besides its steps: the union
-  // copies in and out (0 in a form without; < 0: forced, not timed).
-  double copy_ms = -1;
+  // copies in and out (0 in a form without; < 0: forced, not timed).  own_ms:
+  // a step of it where every union's runs take their own kernels instead,
+  // which give the same bits and need no copies; own_now: this advance does.
+  double copy_ms = -1, own_ms = 0;
+  bool own_now = false;
   // Grouped by order: a stream per group beside the batch's own, and the
   // events that fork and join them.
   std::vector<cudaStream_t> side;
@@ -246,12 +263,13 @@ int mb_launch(mj_mb* mb, int which, int k, int i, cudaStream_t s) {
     }
     return MJ_OK;
   }
-  if (which == 3) return mb_launch_union(mb, k, i, s);
+  if (which == 3) return mb->own_now ? mb_launch_seq(mb, k, s) : mb_launch_union(mb, k, i, s);
   return which == 0 ? mb_launch_t<256>(mb, mb->cfg[0], k, s) : mb_launch_t<128>(mb, mb->cfg[1], k, s);
 }
 
 // Kernel launches of one step in the batch's chosen form.
 uint64_t mb_launches_per_step(const mj_mb* mb) {
+  if (mb->use == 3 && mb->own_now) return 2 * mb->runs.size();
   if (mb->use == 3) return 3;  // element kernel, streaming gather, sources
   if (mb->use != 2) return 1;
   uint64_t n = 0;
@@ -327,6 +345,7 @@ int union_copy(mj_mb* mb, bool in, int steps, cudaStream_t s) {
 
 // union_copy for every union the batch's chosen form steps.
 int mb_union_copy(mj_mb* mb, bool in, int steps, cudaStream_t s) {
+  if (mb->own_now) return MJ_OK;
   if (mb->use == 3) return union_copy(mb, in, steps, s);
   if (mb->use == 2)
     for (auto& g : mb->groups)
@@ -476,28 +495,40 @@ int mb_offset(const mj_mb* mb) {
   return off < 0 ? 0 : off;
 }
 
+// Error flags of a batch: its own kernel's, its union's, and those of runs
+// stepped with their own kernels, which report through their operators.
+void mb_flags(const mj_mb* mb, ErrorFlags& t) {
+  t.f[t.n++] = mb->err.as<int>();
+  if (mb->uni) t.f[t.n++] = mb->uni->op->err.as<int>();
+  if (mb->seq || (mb->use == 3 && mb->own_now))
+    for (mj_lf* lf : mb->runs) t.f[t.n++] = lf->op->err.as<int>();
+  for (auto& g : mb->groups) mb_flags(g.get(), t);
+}
+
+// The flags come back in one copy and one wait: a copy and a wait for each
+// took 10 us, 100 us of an advance of ten runs.
 int mb_check_err(mj_mb* mb, cudaStream_t s) {
-  int herr = 0;
-  for (auto& g : mb->groups) {
-    const int rc = mb_check_err(g.get(), s);
-    if (rc == MJ_ERR_STATE) herr = 1;
-    else if (rc) return rc;
-    if (g->seq)  // runs stepped with their own kernels report through their operators
-      for (mj_lf* lf : g->runs)
-        if (take_kernel_error(lf->op->err.ptr, s, "mj_mb_advance", mb->h_status.as<int>())) herr = 1;
-  }
-  if (mb->uni && take_kernel_error(mb->uni->op->err.ptr, s, "mj_mb_advance", mb->h_status.as<int>())) herr = 1;
-  int own = 0;
-  MJ_CUDA(cudaMemcpyAsync(&own, mb->err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+  ErrorFlags t;
+  mb_flags(mb, t);
+  k_read_flags<<<1, kMaxFlags, 0, s>>>(t, mb->flags.as<int>());
+  count_launch();
+  int* h = mb->h_status.as<int>();
+  MJ_CUDA(cudaMemcpyAsync(h, mb->flags.ptr, sizeof(int) * t.n, cudaMemcpyDeviceToHost, s));
   MJ_CUDA(cudaStreamSynchronize(s));
-  herr |= own;
-  if (herr) {
-    cudaMemset(mb->err.ptr, 0, sizeof(int));
-    cudaMemset(mb->sync.ptr, 0, sizeof(SyncState));
-    set_error("mj_mb_advance: a bounded wait timed out (batch state is invalid)");
-    return MJ_ERR_STATE;
-  }
-  return MJ_OK;
+  bool bad = false;
+  for (int k = 0; k < t.n; k++) bad = bad || h[k];
+  if (!bad) return MJ_OK;
+  for (int k = 0; k < t.n; k++) cudaMemset(t.f[k], 0, sizeof(int));
+  cudaMemset(mb->sync.ptr, 0, sizeof(SyncState));
+  for (auto& g : mb->groups) cudaMemset(g->sync.ptr, 0, sizeof(SyncState));
+  set_error("mj_mb_advance: a bounded wait timed out (batch state is invalid)");
+  return MJ_ERR_STATE;
+}
+
+// own_now of the batch and its groups.
+void mb_set_own(mj_mb* mb, bool on) {
+  mb->own_now = on;
+  for (auto& g : mb->groups) g->own_now = on;
 }
 
 // Times the batch's forms on the batch itself (3 steps each after one
@@ -525,7 +556,7 @@ int mb_autotune(mj_mb* mb, int off, cudaStream_t s) {
   MJ_CUDA(cudaEventCreate(&e1));
   const uint64_t before = launch_counter().load();
   int best = 0;
-  double copy_ms[4] = {0, 0, 0, 0};
+  double copy_ms[4] = {0, 0, 0, 0}, own_ms[4] = {0, 0, 0, 0};
   std::vector<int> forms = {0, 1};
   if (!mb->groups.empty()) forms.push_back(2);
   if (mb->uni) forms.push_back(3);
@@ -559,15 +590,24 @@ int mb_autotune(mj_mb* mb, int off, cudaStream_t s) {
     if (!rc) rc = mb_check_err(mb, s);
     float ms = 0.f;
     if (!rc) rc = cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
-    if (c >= 2) {  // its copies, out and in again
+    if (c >= 2) {  // its copies, out and in again, and its steps without them
+      float cms = 0.f;
       if (!rc) rc = cudaEventRecord(e0, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
       if (!rc) rc = mb_union_copy(mb, false, 4, s);
       if (!rc) rc = mb_union_copy(mb, true, 0, s);
       if (!rc) rc = cudaEventRecord(e1, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
       if (!rc) rc = cudaStreamSynchronize(s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
-      float cms = 0.f;
       if (!rc) rc = cudaEventElapsedTime(&cms, e0, e1) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
       copy_ms[c] = cms;
+      mb_set_own(mb, true);
+      if (!rc) rc = mb_steps(mb, off, 0, 1, s);
+      if (!rc) rc = cudaEventRecord(e0, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+      if (!rc) rc = mb_steps(mb, off, 1, 3, s);
+      if (!rc) rc = cudaEventRecord(e1, s) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+      if (!rc) rc = mb_check_err(mb, s);
+      mb_set_own(mb, false);
+      if (!rc) rc = cudaEventElapsedTime(&cms, e0, e1) == cudaSuccess ? MJ_OK : MJ_ERR_CUDA;
+      own_ms[c] = cms / 3.0;
     }
     if (rc) {
       mb->use = -1;
@@ -592,6 +632,7 @@ int mb_autotune(mj_mb* mb, int off, cudaStream_t s) {
   MJ_CUDA(cudaStreamSynchronize(s));
   mb->use = best;
   mb->copy_ms = copy_ms[best];
+  mb->own_ms = own_ms[best];
   return MJ_OK;
 }
 
@@ -700,7 +741,8 @@ int mb_create(int n_runs, mj_lf* const* runs, bool split, std::unique_ptr<mj_mb>
     if (!rc) rc = mb_build_lists<128>(mb.get(), src_dofs, mb->cfg[1]);
     if (rc) return rc;
   }
-  MJ_CUDA(mb->h_status.alloc(sizeof(int)));
+  MJ_CUDA(mb->flags.alloc(sizeof(int) * kMaxFlags));
+  MJ_CUDA(mb->h_status.alloc(sizeof(int) * kMaxFlags));
   MJ_CUDA(mb->sync.alloc(sizeof(SyncState)));
   MJ_CUDA(cudaMemset(mb->sync.ptr, 0, sizeof(SyncState)));
   MJ_CUDA(mb->err.alloc(sizeof(int)));
@@ -776,19 +818,16 @@ int mj_mb_advance(mj_mb* mb, int nsteps, int use_graph) {
         const int rc = mb_autotune(g.get(), off, s);
         if (rc) return rc;
       }
-  // An advance of a few steps does not pay for a union's copies: one kernel
-  // of all its meshes then (the forms' FP32 states agree to rounding, and
-  // timing chooses between them anyway).  10 meshes, one step: 172 us, with
-  // the copies 234.
-  struct Form {  // this call's form; the batch keeps its own
+  // An advance of a few steps does not pay for a union's copies: its runs
+  // take their own kernels then, whose bits are the union's: how a run is
+  // split into advances does not change its bits.  10 meshes, one step: 104 us;
+  // 225 in the one-kernel form with an error check per run.
+  struct Own {
     mj_mb* mb;
-    int use;
-    ~Form() { mb->use = use; }
-  } kept{mb, mb->use};
-  if (mb->use >= 2 && mb->copy_ms >= 0 && nsteps < kGraphStepsMb && !mb->profile) {
-    const int one = mb->tune_ms[0] <= mb->tune_ms[1] ? 0 : 1;
-    if (nsteps * mb->tune_ms[one] < mb->copy_ms + nsteps * mb->tune_ms[mb->use]) mb->use = one;
-  }
+    ~Own() { mb_set_own(mb, false); }
+  } kept{mb};
+  mb_set_own(mb, mb->use >= 2 && mb->copy_ms >= 0 && nsteps < kGraphStepsMb && !mb->profile &&
+                     nsteps * mb->own_ms < mb->copy_ms + nsteps * mb->tune_ms[mb->use]);
   if (int rc = mb_union_copy(mb, true, 0, s)) return rc;
   mb->last_graph = false;
   int done = 0;

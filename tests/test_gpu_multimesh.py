@@ -227,3 +227,36 @@ def test_short_and_long_advances_mix(steps):
     for op, lf in batch_runs + single_runs:
         lf.close()
         op.close()
+
+
+def test_splitting_an_advance_does_not_change_the_states():
+    """A tuned batch gives the same bits whether it advances 25 steps at once or one, two or three at a time."""
+    from montjoie_gb300 import mesh as M
+    from montjoie_gb300.leapfrog import MeshBatch
+    from montjoie_gb300.problem import AcousticProblem
+    runs = []
+    for k, (order, cells) in enumerate([(2, 30), (3, 20), (4, 16), (6, 10), (8, 8), (2, 18), (3, 14), (4, 20), (6, 12)]):
+        m = M.perturbed_cube(cells, seed=k, amplitude=0.05, kind="random", c_mode="element")
+        s = M.AcousticSetup(order=order, dt=0.2 / cells / order ** 2, nsteps=60, src_radius=0.3)
+        pb = AcousticProblem(m, s)
+        op = pb.operator("fp32")
+        runs.append((op, pb.integrator(op, diagnostics=False)))
+    mb = MeshBatch([lf for _, lf in runs])
+
+    def advance(*lengths):
+        for op, lf in runs:
+            lf.SetInitialConditionS(np.zeros(op.n_dof))
+        for n in lengths:
+            mb.advance(n)
+        return [lf.GetState() for _, lf in runs]
+
+    advance(25)  # the forms are timed here
+    want = advance(25)
+    assert all(np.abs(u).max() > 0 for u, _ in want)
+    for lengths in ([1] * 25, [3, 2] * 5, [19, 6], [20, 5]):
+        for (a, b), (u, v) in zip(advance(*lengths), want):
+            assert np.array_equal(a, u) and np.array_equal(b, v), lengths
+    mb.close()
+    for op, lf in runs:
+        lf.close()
+        op.close()
