@@ -153,9 +153,10 @@ int mj_op_tuning(const mj_op* op, int* tile_elems, int* vector_lines, int* grid,
 /* Forces the element-kernel variant instead of the autotuner's choice:
  * tile_elems elements per CTA and the work layout (vector_lines: 0 compact,
  * 1 vector lines, 2 one element per warp, 3 the same with packed
- * connectivity, 4 compact with one factor stage; 1 to 4 are FP32 only, 2 and
- * 3 exist for order 4, 3 for meshes of fewer than 2^27 dofs each shared by
- * at most 32 elements);
+ * connectivity, 4 compact with one factor stage, 5 fixed point, 6 line owner;
+ * 1 to 4 and 6 are FP32 only, 2 and 3 exist for order 4, 3 for meshes of fewer
+ * than 2^27 dofs each shared by at most 32 elements, 5 for FP64 operators that
+ * hold its factors, 6 for orders 7 and 8);
  * MJ_ERR_ARG when no such variant exists for the order.  Integrators bound to the operator
  * keep captured CUDA graphs of the old variant until re-created. */
 int mj_op_set_variant(mj_op* op, int tile_elems, int vector_lines);

@@ -701,17 +701,22 @@ int mj_op_tuning(const mj_op* op, int* tile_elems, int* vector_lines, int* grid,
 
 int mj_op_set_variant(mj_op* op, int tile_elems, int vector_lines) {
   MJ_CHECK_ARG(op, "mj_op_set_variant: null operator");
-  MJ_CHECK_ARG(vector_lines >= 0 && vector_lines <= 4, "mj_op_set_variant: layout must be 0, 1, 2, 3 or 4");
+  MJ_CHECK_ARG(vector_lines >= 0 && vector_lines <= 6, "mj_op_set_variant: layout must be 0 to 6");
   MJ_CHECK_ARG(vector_lines != 3 || op->nodle_pk.ptr, "mj_op_set_variant: no packed connectivity for this operator");
   const bool warp = vector_lines == 2 || vector_lines == 3, vec = vector_lines == 1, packed = vector_lines == 3;
-  const bool fs = vector_lines == 4;
-  const std::vector<int> cands = warp ? k1_warp_tile_candidates(op->n) : k1_tile_candidates(op->n);
+  const bool fs = vector_lines == 4, fx = vector_lines == 5, ln = vector_lines == 6;
+  MJ_CHECK_ARG(!fx || op->fac_fx.ptr, "mj_op_set_variant: the operator has no fixed-point kernel");
+  const std::vector<int> cands = warp ? k1_warp_tile_candidates(op->n)
+                                 : ln ? k1_ln_tile_candidates(op->n)
+                                      : k1_tile_candidates(op->n);
   MJ_CHECK_ARG(std::find(cands.begin(), cands.end(), tile_elems) != cands.end(),
                "mj_op_set_variant: no element kernel with this tile size and layout for this order");
-  MJ_CHECK_ARG(vector_lines == 0 || op->precision == MJ_FP32,
-               "mj_op_set_variant: the vector-line, warp and one-factor-stage layouts are FP32 only");
+  MJ_CHECK_ARG(vector_lines == 0 || fx || op->precision == MJ_FP32,
+               "mj_op_set_variant: the vector-line, warp, one-factor-stage and line-owner layouts are FP32 only");
   int ctas = 0;
-  const int rc = warp ? k1_prepare_w_f32(op->n, tile_elems, packed, &ctas)
+  const int rc = fx   ? k1_prepare_fx(op, tile_elems, &ctas)
+                 : ln ? k1_prepare_ln_f32(op->n, tile_elems, &ctas)
+                 : warp ? k1_prepare_w_f32(op->n, tile_elems, packed, &ctas)
                  : fs ? k1_prepare_fs_f32(op->n, tile_elems, &ctas)
                       : op->precision == MJ_FP64 ? k1_prepare_f64(op->n, tile_elems, false, &ctas)
                                                  : k1_prepare_f32(op->n, tile_elems, vec, &ctas);
@@ -721,7 +726,8 @@ int mj_op_set_variant(mj_op* op, int tile_elems, int vector_lines) {
   op->warp = warp;
   op->packed = packed;
   op->fs = fs;
-  op->fx = op->ln = false;
+  op->fx = fx;
+  op->ln = ln;
   op->n_tiles = op->n_elt_pad / tile_elems;
   op->grid_k1 = std::max(1, std::min(op->n_tiles, ctas * sm_count()));
   return MJ_OK;

@@ -132,7 +132,7 @@ class FemMatrixFreeOperator:
         """Forces the element-kernel variant (otherwise chosen by the autotuner):
         layout 0 / False compact, 1 / True vector lines, 2 one element per warp,
         3 one element per warp reading the packed connectivity, 4 compact with
-        one factor stage."""
+        one factor stage, 5 fixed point (FP64), 6 line owner (orders 7, 8)."""
         _lib.check(_lib.load().mj_op_set_variant(self._h, int(tile_elems), int(layout)))
 
     def device_bytes(self) -> int:
