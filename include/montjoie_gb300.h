@@ -172,11 +172,13 @@ uint64_t mj_kernel_launches(void);
  * own copies in flight land, and the entry point returns MJ_ERR_CUDA (element
  * kernels) or MJ_ERR_STATE (cooperative steps) with a message; the state is
  * then invalid but the next call starts clean.  This call lets a test make
- * waits run out: mbar_polls = 0 switches two element-kernel variants (FP32
- * one element per warp, order 4, 2 elements per CTA; FP64 compact, order 4,
- * 4 elements per CTA; see mj_op_set_variant) to instances compiled with a
- * bulk-copy wait limit of 0 (the bound is a compile-time constant in the
- * kernels), any other value switches them back; barrier_polls and
+ * waits run out: mbar_polls = 0 switches some variants (FP32 one element per
+ * warp, order 4, 2 elements per CTA; FP64 compact, order 4, 4 elements per CTA;
+ * fixed point, order 4, 5 elements; line owner, order 7, 2 elements, see
+ * mj_op_set_variant; the FP64 streaming gather; the many-source step's plane
+ * variant 4, 8, 1 of order 4, see mj_lfb_set_step_variant) to instances
+ * compiled with a bulk-copy wait limit of 0 (the bound is a compile-time
+ * constant in the kernels), any other value switches them back; barrier_polls and
  * barrier_ns lower the grid barrier's limits (0: give up after the first
  * poll; values above the defaults are clamped to them; negative values
  * restore them).  Process-wide; captured CUDA graphs keep the kernels they

@@ -212,10 +212,14 @@ int k1_prepare_fx_gen(int n, int E, int* ctas_per_sm);
 void k1_launch_fx(mj_op* op, const void* x, cudaStream_t s);
 void k1_launch_fx_gen(mj_op* op, const void* x, cudaStream_t s);
 
-// Test instances of two variants compiled with a bulk-copy wait limit of 0
+// Test instances of some variants compiled with a bulk-copy wait limit of 0
 // (the test hook of mj_debug_set_wait_limits): FP32 one element per warp with
-// n = 5, E = 2, and FP64 compact with n = 5, E = 4.  Return false (nothing
-// launched) for any other variant.
+// n = 5, E = 2, FP64 compact with n = 5, E = 4, fixed point with n = 5, E = 5
+// and line owner with n = 8, E = 2.  Return false (nothing launched) for any
+// other variant.
+bool k1_launch_fx_waits_out(mj_op* op, const void* x, cudaStream_t s);
+bool k1_launch_ln_f32_waits_out(int n, int E, int grid, const void* x, const int* nodle_e, const void* fac_e, void* R,
+                                const int* slot_e, int n_tiles, int* err, cudaStream_t s);
 bool k1_launch_w_f32_waits_out(int n, int E, int grid, const void* x, const int* nodle_e, const void* fac_e,
                                void* R, const int* slot_e, int n_tiles, int* err, cudaStream_t s);
 bool k1_launch_f64_waits_out(int n, int E, int grid, const void* x, const int* nodle_e, const void* fac_e,

@@ -113,6 +113,18 @@ int k1_set_gmat_fx(int n, const double* g, bool sym) {
 int k1_prepare_fx(const mj_op* op, int E, int* ctas) {
   return op->fx_sym ? k1_prepare_fx_sym(op->n, E, ctas) : k1_prepare_fx_gen(op->n, E, ctas);
 }
+// The instance with a bulk-copy wait limit of 0: order 4, 5 elements per CTA.
+bool k1_launch_fx_waits_out(mj_op* op, const void* x, cudaStream_t s) {
+  if (op->n != 5 || op->E != 5 || !op->fx_sym) return false;
+  using P = FxPlan<5, 5>;
+  auto* k = k_local_stiffness_fx<5, 5, true, 0>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::total) != cudaSuccess) return false;
+  k<<<op->grid_k1, P::threads, P::total, s>>>(static_cast<const double*>(x), op->nodle_e.as<int>(),
+                                              op->fac_fx.as<int2>(), op->fac_exp.as<int>(), op->fac_e.as<double>(),
+                                              op->R.as<double>(), op->slot_e.as<int>(), op->n_tiles,
+                                              op->err.as<int>());
+  return true;
+}
 void k1_launch_fx(mj_op* op, const void* x, cudaStream_t s) {
   if (op->fx_sym) k1_launch_fx_sym(op, x, s);
   else k1_launch_fx_gen(op, x, s);

@@ -356,7 +356,7 @@ __device__ __noinline__ bool fx_choose(const long long* s_u, unsigned* scratch, 
   return s_mode[el] & 2;
 }
 
-template <int N, int E, bool SYM>
+template <int N, int E, bool SYM, long SPIN = kSpinLimit>
 __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     k_local_stiffness_fx(const double* __restrict__ x, const int* __restrict__ nodle_e,
                          const int2* __restrict__ fac_fx, const int* __restrict__ fac_exp,
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     atomicMax(&s_max[par * E + el], zm);
   };
   if (tile < n_tiles) {
-    const bool ok = mbar_wait_bounded(&bar[0], 0u);
+    const bool ok = mbar_wait_bounded<SPIN>(&bar[0], 0u);
     if (__syncthreads_or(!ok)) {
       if (t == 0) {  // report; every copy issued above may still be in flight
         atomicExch(err, 1);
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
       atomicMax(&s_gmax[el], gm);
     }
     {  // this tile's factors (the vote is also the barrier after the gradients)
-      const bool ok = mbar_wait_bounded(&bar[2], (ph >> 2) & 1u);
+      const bool ok = mbar_wait_bounded<SPIN>(&bar[2], (ph >> 2) & 1u);
       if (__syncthreads_or(!ok)) {
         if (t == 0) {  // report; this tile's factors and the next tile's Nodle may be in flight
           atomicExch(err, 1);
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     bool lost = false;
     if (nt < n_tiles) {
       const int so = s ^ 1;
-      lost = !mbar_wait_bounded(&bar[so], (ph >> so) & 1u);
+      lost = !mbar_wait_bounded<SPIN>(&bar[so], (ph >> so) & 1u);
       ph ^= 1u << so;
       if (!lost) {
         const int* nd = s_nod(so) + pe;

@@ -52,7 +52,7 @@ __device__ __forceinline__ void grad_line(const float (&r)[N], float (&y)[N]) {
   }
 }
 
-template <int N, int E>
+template <int N, int E, long SPIN = kSpinLimit>
 __global__ void __launch_bounds__(E* N* N, LnPlan<N, E>::ctas)
     k_local_stiffness_ln(const float* __restrict__ x, const int* __restrict__ nodle_e,
                          const float* __restrict__ fac_e, float* __restrict__ R, const int* __restrict__ slot_e,
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(E* N* N, LnPlan<N, E>::ctas)
   uint32_t ph = 0u;  // bits 0, 1: parity of the next completion of Nodle stage 0, 1; bit 2: of the factor stage
   float u[N];
   if (tile < n_tiles) {
-    const bool ok = mbar_wait_bounded(&bar[0], 0u);
+    const bool ok = mbar_wait_bounded<SPIN>(&bar[0], 0u);
     if (__syncthreads_or(!ok)) {
       if (t == 0) {  // report; every copy issued above may still be in flight
         atomicExch(err, 1);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(E* N* N, LnPlan<N, E>::ctas)
       grad_line<N>(u, z);
     }
     {  // this tile's factors (the vote is also the barrier after the gradients)
-      const bool ok = mbar_wait_bounded(&bar[2], (ph >> 2) & 1u);
+      const bool ok = mbar_wait_bounded<SPIN>(&bar[2], (ph >> 2) & 1u);
       if (__syncthreads_or(!ok)) {
         if (t == 0) {  // report; this tile's factors and the Nodle of the next two tiles may be in flight
           atomicExch(err, 1);
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(E* N* N, LnPlan<N, E>::ctas)
     const int nt = tile + g;
     if (nt < n_tiles) {
       const int so = s ^ 1;
-      lost = !mbar_wait_bounded(&bar[so], (ph >> so) & 1u);
+      lost = !mbar_wait_bounded<SPIN>(&bar[so], (ph >> so) & 1u);
       ph ^= 1u << so;
       if (!lost) {
         const int* nd = s_nod(so) + pe;
@@ -263,6 +263,18 @@ int k1_prepare_ln_f32(int n, int E, int* ctas) {
 #undef MJ_X
   set_error("no line-owner element kernel variant for this order and tile size");
   return MJ_ERR_ARG;
+}
+
+// The instance with a bulk-copy wait limit of 0: order 7, 2 elements per CTA.
+bool k1_launch_ln_f32_waits_out(int n, int E, int grid, const void* x, const int* nodle_e, const void* fac_e, void* R,
+                                const int* slot_e, int n_tiles, int* err, cudaStream_t s) {
+  if (n != 8 || E != 2) return false;
+  using P = LnPlan<8, 2>;
+  auto* k = k_local_stiffness_ln<8, 2, 0>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::total) != cudaSuccess) return false;
+  k<<<grid, P::threads, P::total, s>>>(static_cast<const float*>(x), nodle_e, static_cast<const float*>(fac_e),
+                                       static_cast<float*>(R), slot_e, n_tiles, err);
+  return true;
 }
 
 void k1_launch_ln_f32(int n, int E, int grid, const void* x, const int* nodle_e, const void* fac_e, void* R,

@@ -655,7 +655,7 @@ static_assert(kStream64P % 16 == 0 && kStream64L % 16 == 0 && kStream64R % 16 ==
               "aligned buffer segments");
 static_assert(kStream64Dofs == kStreamThreads, "one dof per thread");
 
-template <bool DIAG>
+template <bool DIAG, long SPIN = kSpinLimit>
 __global__ void __launch_bounds__(kStreamThreads, 7)
     k_gather_leapfrog_stream64(const double* __restrict__ R, const int* __restrict__ ptr, int* __restrict__ ctr,
                                int qc, double* __restrict__ u0, const double* __restrict__ u1,
@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(kStreamThreads, 7)
   double nacc = 0.0;  // DIAG: this thread's sum of w u^2
   for (int c = blockIdx.x; c < n_chunks; c += G, b = (b + 1 == kStreamNB ? 0 : b + 1)) {
     const StreamChunk ch = chunks[c];
-    const bool ok = mbar_wait_bounded(&bar[b], (ph >> b) & 1u);
+    const bool ok = mbar_wait_bounded<SPIN>(&bar[b], (ph >> b) & 1u);
     if (__syncthreads_or(!ok)) {
       // report, wait (bounded) for this CTA's copies still in flight, and
       // still take part in the diagnostics' finished-CTA count

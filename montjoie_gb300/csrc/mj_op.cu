@@ -87,7 +87,10 @@ void launch_k1(mj_op* op, const void* x, cudaStream_t s) {
     const bool done =
         op->warp ? k1_launch_w_f32_waits_out(op->n, op->E, op->grid_k1, x, op->nodle_e.as<int>(), op->fac_e.ptr,
                                             op->R.ptr, op->slot_e.as<int>(), op->n_tiles, op->err.as<int>(), s)
-        : op->precision == MJ_FP64 && !op->vec && !op->fx
+        : op->fx ? k1_launch_fx_waits_out(op, x, s)
+        : op->ln ? k1_launch_ln_f32_waits_out(op->n, op->E, op->grid_k1, x, op->nodle_e.as<int>(), op->fac_e.ptr,
+                                              op->R.ptr, op->slot_e.as<int>(), op->n_tiles, op->err.as<int>(), s)
+        : op->precision == MJ_FP64 && !op->vec
             ? k1_launch_f64_waits_out(op->n, op->E, op->grid_k1, x, op->nodle_e.as<int>(), op->fac_e.ptr, op->R.ptr,
                                       op->slot_e.as<int>(), op->n_tiles, op->err.as<int>(), s)
             : false;
@@ -871,8 +874,9 @@ int lf_stream_setup(mj_lf* lf, bool* fits = nullptr) {
   }
   int ctas = 0;
   if (f64) {
-    MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    MJ_CUDA(cudaFuncSetAttribute(k_gather_leapfrog_stream64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    for (auto* k : {k_gather_leapfrog_stream64<false>, k_gather_leapfrog_stream64<true>,
+                    k_gather_leapfrog_stream64<false, 0>, k_gather_leapfrog_stream64<true, 0>})
+      MJ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     MJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_gather_leapfrog_stream64<true>, kStreamThreads,
                                                           smem));
   } else {
@@ -1211,6 +1215,7 @@ void lf_step_launch(mj_lf* lf, void* cur, const void* next, int qc, cudaStream_t
   }
   if (op->precision == MJ_FP64 && lf->stream64) {
     auto k2 = dg ? k_gather_leapfrog_stream64<true> : k_gather_leapfrog_stream64<false>;
+    if (k1_waits_run_out()) k2 = dg ? k_gather_leapfrog_stream64<true, 0> : k_gather_leapfrog_stream64<false, 0>;
     launch_dependent(k2, lf->stream_grid_, kStreamThreads, kStream64Smem, s,
         op->R.as<double>(), op->ptr.as<int>(), lf->ctr.as<int>(), qc, static_cast<double*>(cur),
         static_cast<const double*>(next), lf->m64.as<double>(), lf->stream_chunks.as<StreamChunk>(),

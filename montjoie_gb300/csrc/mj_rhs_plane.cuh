@@ -98,7 +98,7 @@ __device__ __forceinline__ void fma_g(float (&acc)[V], int idx, const float (&x)
 
 // Phase 2: sums, update and sources of this CTA's chunks, through two buffers
 // of HALF bytes at smem and the two unused mbarriers at bar.
-template <int T, int HALF>
+template <int T, int HALF, long SPIN>
 __device__ __forceinline__ void rp_dof_phase(const RsParams& p, const RpParams& x, unsigned char* smem,
                                              uint64_t* bar, float* __restrict__ cur,
                                              const float* __restrict__ nxt, int par, int* err) {
@@ -153,7 +153,7 @@ __device__ __forceinline__ void rp_dof_phase(const RsParams& p, const RpParams& 
   for (int c = blockIdx.x, it = 0; c < x.n_chunks; c += G, ++it) {
     const int b = it & 1;
     const RpChunk ch = x.chunks[c];
-    const bool ok = mbar_wait_bounded(&bar[b], (ph2 >> b) & 1u);
+    const bool ok = mbar_wait_bounded<SPIN>(&bar[b], (ph2 >> b) & 1u);
     if (__syncthreads_or(!ok)) {
       if (t == 0) {  // report; buffer b and, if issued, buffer b^1 may have copies in flight
         atomicExch(err, 1);
@@ -229,7 +229,7 @@ __device__ __forceinline__ void rp_dof_phase(const RsParams& p, const RpParams& 
   }
 }
 
-template <int N, int E, int LB, int V, bool EN>
+template <int N, int E, int LB, int V, bool EN, long SPIN = kSpinLimit>
 __global__ void __launch_bounds__(RpPlan<N, E, LB, V>::T, RpPlan<N, E, LB, V>::kCtas)
     k_rhs_plane(const RsParams p, const RpParams x, SyncState* sync, int par, int* err,
                 unsigned long long* __restrict__ stamps) {
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(RpPlan<N, E, LB, V>::T, RpPlan<N, E, LB, V>::k
   uint32_t ph = 0u;
   for (int tile = blockIdx.x, it = 0; tile < p.n_tiles; tile += G, ++it) {
     const int s = it & 1;
-    const bool ok = mbar_wait_bounded(&bar[s], (ph >> s) & 1u);
+    const bool ok = mbar_wait_bounded<SPIN>(&bar[s], (ph >> s) & 1u);
     if (__syncthreads_or(!ok)) {
       if (t == 0) {  // report; only stage s can have copies in flight here
         atomicExch(err, 1);
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(RpPlan<N, E, LB, V>::T, RpPlan<N, E, LB, V>::k
 
   if constexpr (EN) asm volatile("griddepcontrol.launch_dependents;");  // the adjoint's injection may start
   // ---- phase 2
-  rp_dof_phase<P::T, P::kHalf>(p, x, smem, &bar[2], cur, nxt, par, err);
+  rp_dof_phase<P::T, P::kHalf, SPIN>(p, x, smem, &bar[2], cur, nxt, par, err);
   if (stamps) {
     __syncthreads();
     if (t == 0) stamps[4 * blockIdx.x + 3] = global_ns();

@@ -7,8 +7,10 @@
 // reports the failure with a message.
 // - mbarrier waits poll at most kSpinLimit times, a compile-time bound (a
 //   limit read from memory changes the register allocation of the element
-//   kernels and slows them); the test hook instead switches two element-kernel
-//   variants to instances compiled with a limit of 0 (mj_k1_f32.cu, mj_k1_f64.cu).
+//   kernels and slows them); the test hook instead switches some variants to
+//   instances compiled with a limit of 0 (element kernels: mj_k1_f32.cu,
+//   mj_k1_f64.cu, mj_k1_fx.cu, mj_k1_ln.cu; the FP64 streaming gather; the plane
+//   form of the many-source step: mj_rhs_plane.cu).
 // - The grid barrier's limits live in constant memory, one copy per
 //   translation unit that launches cooperative kernels; each unit registers a
 //   setter at load so that mj_debug_set_wait_limits can lower them all.
