@@ -135,16 +135,12 @@ __device__ __forceinline__ void rp_dof_phase(const RsParams& p, const RpParams& 
     issue_chunk(blockIdx.x, 0);
     issue_chunk(blockIdx.x + G, 1);
   }
-  // sources at interior dofs: phase 1 has stored their update without them
+  // sources at interior dofs, one per (dof, right-hand side): phase 1 has stored their update without them
   if (pulse_on) {
     for (int e = blockIdx.x * T + t; e < x.n_fix; e += G * T) {
       const int d = __ldg(x.fix + 2 * e), r = __ldg(x.fix + 2 * e + 1);
-      if (e > 0 && __ldg(x.fix + 2 * e - 2) == d && __ldg(x.fix + 2 * e - 1) == r)
-        continue;  // the first of its run adds them all
       float un = dst[(size_t)d * S + r];
-      const float md = __ldg(p.m + d);
-      for (int q = e; q < x.n_fix && __ldg(x.fix + 2 * q) == d && __ldg(x.fix + 2 * q + 1) == r; q++)
-        un += md * pf * __ldg(x.fix_val + q);
+      un += __ldg(p.m + d) * pf * __ldg(x.fix_val + e);
       dst[(size_t)d * S + r] = un;
       if (p.ucopy) p.ucopy[(size_t)d * S + r] = un;
     }
