@@ -46,15 +46,13 @@
 // vertex lost up to 87 times in L2.
 // All other elements (spikes, the numerical tail ahead of a front; factors that
 // vary by more than 2.5 along an element, which is known when they are
-// converted) take the FP64 arithmetic of k_local_stiffness on their own
-// threads, beside the others of the tile (fx_exact_*), and so does an element
-// out of range (a NaN or infinity in u or B, or scales whose result would leave
+// converted) take the FP64 arithmetic of k_local_stiffness beside the others of
+// the tile (fx_exact), and so does an element out of range (a NaN or infinity in u or B, or scales whose result would leave
 // the normal range).  The choice hangs on the element alone, not on the tile it
 // is in.  Of smooth waves 2.5 elements long or more, fewer than 0.04% of the
-// elements take it.  The FP64 pipe takes 16 clocks per warp instruction, so one
-// such element keeps its tile for 7 us at Q4 and 22 us at Q8, and a field of
-// spikes takes what the FP64-pipe kernel does (16^3 Q4 57 and 61 us per
-// product, 15x13x11 Q8 260 and 237).
+// elements take it.  One such element keeps its tile for 2 us at Q4 and 13 us
+// at Q8; a field of spikes everywhere takes about what the FP64-pipe kernel does
+// (16^3 Q4 58 and 61 us per product, 15x13x11 Q8 268 and 237).
 //
 // Measured (us per launch, FP64-pipe kernel at its best tile -> this kernel):
 // Q4 16^3 60 -> 20, 64^3 2300 -> 598; Q8 15x13x11-sized 359 -> 94, 32^3 3150
@@ -243,64 +241,52 @@ struct FxPlan {
   static_assert(fac_bytes % 16 == 0 && nod_bytes % 16 == 0, "bulk copies");
 };
 
-// An element in FP64, the arithmetic of k_local_stiffness<double> (compact) in
-// the three phases of the tile, by the element's threads; su, sa, sb: its work
-// arrays, u staged in su.  ij: the thread's z-line.  Three points at a time: a
-// tile waits for its elements here, and one point is a chain of up to 3 n
-// dependent FP64 operations.
-// Gradients along x and y of the thread's points into sa and sb.
+// The chosen elements of a tile (s_mode bit 1) in FP64, the arithmetic of
+// k_local_stiffness<double> (compact), their u staged as doubles in s_u;
+// scratch: the factor stage, free.  The whole CTA works on their points,
+// whichever threads own them: the FP64 pipe takes 16 clocks per warp
+// instruction whatever its active lanes, so the points are dealt densely (by
+// their element's own threads, 25 or 81 in 2 or 4 warps, one element of a tile
+// took 7 us at Q4 and 22 at Q8).
 template <int N, int E>
-__device__ __noinline__ void fx_exact_gradient(const double* su, double* sa, double* sb, int ij) {
-  constexpr int RS = FxPlan<N, E>::RS;
+__device__ __noinline__ void fx_exact(const double* s_u, double* s_a, double* s_b, const int* s_mode, double* scratch,
+                                      const double* __restrict__ fac, double* __restrict__ R,
+                                      const int* __restrict__ slot) {
+  using P = FxPlan<N, E>;
+  constexpr int NN = P::NN, Q = N * NN, Qp = P::Qp, RS = P::RS, W = P::W;
+  static_assert(sizeof(double) * E * W + sizeof(int) * E <= P::fac_bytes, "z-fluxes and the list fit the factor stage");
   const double* __restrict__ G = c_gmat64[N];
-  const int j = ij / N, i = ij - j * N;
-#pragma unroll 3
-  for (int k = 0; k < N; k++) {
-    const double *rx = su + (k * N + j) * RS, *ry = su + k * N * RS + i;
-    double gx = 0, gy = 0;
+  int* list = reinterpret_cast<int*>(scratch + E * W);
+  int count = 0;
+  for (int e = 0; e < E; e++)
+    if (s_mode[e] & 2) {
+      if (threadIdx.x == 0) list[count] = e;
+      count++;
+    }
+  __syncthreads();
+  for (int q = threadIdx.x; q < count * Q; q += P::threads) {
+    const int el = list[q / Q], p = q % Q, k = p / NN, ij = p % NN, j = ij / N, i = ij % N;
+    const double *rx = s_u + el * W + (k * N + j) * RS, *ry = s_u + el * W + k * N * RS + i;
+    const double* rz = s_u + el * W + j * RS + i;
+    double gx = 0, gy = 0, gz = 0;
 #pragma unroll
     for (int a = 0; a < N; a++) {
       gx += G[a * N + i] * rx[a];
       gy += G[a * N + j] * ry[a * RS];
+      gz += G[a * N + k] * rz[a * N * RS];
     }
-    sa[(k * N + j) * RS + i] = gx;
-    sb[(k * N + j) * RS + i] = gy;
-  }
-}
-
-// Fluxes of the thread's points, over their gradients and (along z) over u.
-template <int N, int E>
-__device__ __noinline__ void fx_exact_flux(double* su, double* sa, double* sb, const double* __restrict__ fac, int ij) {
-  constexpr int NN = N * N, Qp = FxPlan<N, E>::Qp, RS = FxPlan<N, E>::RS;
-  const double* __restrict__ G = c_gmat64[N];
-  const int at = ij / N * RS + ij % N;
-  double u[N];
-#pragma unroll
-  for (int a = 0; a < N; a++) u[a] = su[at + a * N * RS];
-#pragma unroll 3
-  for (int k = 0; k < N; k++) {
-    const double* f = fac + k * NN + ij;
+    const double* f = fac + (size_t)el * 6 * Qp + p;
     const double bxx = f[0], bxy = f[Qp], bxz = f[2 * Qp], byy = f[3 * Qp], byz = f[4 * Qp], bzz = f[5 * Qp];
-    const double gx = sa[at + k * N * RS], gy = sb[at + k * N * RS];
-    double gz = 0;
-#pragma unroll
-    for (int a = 0; a < N; a++) gz += G[a * N + k] * u[a];
-    sa[at + k * N * RS] = fac_dot(bxx, gx, bxy, gy, bxz, gz);
-    sb[at + k * N * RS] = fac_dot(bxy, gx, byy, gy, byz, gz);
-    su[at + k * N * RS] = fac_dot(bxz, gx, byz, gy, bzz, gz);
+    const int at = el * W + (k * N + j) * RS + i;
+    s_a[at] = fac_dot(bxx, gx, bxy, gy, bxz, gz);
+    s_b[at] = fac_dot(bxy, gx, byy, gy, byz, gz);
+    scratch[at] = fac_dot(bxz, gx, byz, gy, bzz, gz);
   }
-}
-
-// Divergence at the thread's points into R.
-template <int N, int E>
-__device__ __noinline__ void fx_exact_divergence(const double* su, const double* sa, const double* sb,
-                                                 double* __restrict__ R, const int* __restrict__ slot, int ij) {
-  constexpr int NN = N * N, RS = FxPlan<N, E>::RS;
-  const double* __restrict__ G = c_gmat64[N];
-  const int j = ij / N, i = ij - j * N;
-#pragma unroll 3
-  for (int k = 0; k < N; k++) {
-    const double *rx = sa + (k * N + j) * RS, *ry = sb + k * N * RS + i, *rz = su + j * RS + i;
+  __syncthreads();
+  for (int q = threadIdx.x; q < count * Q; q += P::threads) {
+    const int el = list[q / Q], p = q % Q, k = p / NN, ij = p % NN, j = ij / N, i = ij % N;
+    const double *rx = s_a + el * W + (k * N + j) * RS, *ry = s_b + el * W + k * N * RS + i;
+    const double* rz = scratch + el * W + j * RS + i;
     double y = 0;
 #pragma unroll
     for (int a = 0; a < N; a++) {
@@ -308,7 +294,7 @@ __device__ __noinline__ void fx_exact_divergence(const double* su, const double*
       y += G[j * N + a] * ry[a * RS];
       y += G[k * N + a] * rz[a * N * RS];
     }
-    R[slot[k * NN + ij]] = y;
+    R[slot[(size_t)el * Qp + p]] = y;
   }
 }
 
@@ -529,20 +515,19 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     bool exact = false;  // this thread's element in FP64
     const int shift = max(1, sv + fx_contrast(N));
     if (__syncthreads_or(bad || below > shift << 20)) {  // also: the factor stage is free, the fluxes are staged
-      double *su = reinterpret_cast<double*>(s_u + el * W), *sa = reinterpret_cast<double*>(s_a + el * W);
-      double* sb = reinterpret_cast<double*>(s_b + el * W);
-      const size_t e = (size_t)tile * E + el;
       exact = fx_choose<N, E>(s_u, reinterpret_cast<unsigned*>(s_fac), s_mode, bad, below > shift << 20,
-                              s_max[s * E + el], __ldg(fac_exp + e), shift, ij);
-      if (exact)
+                              s_max[s * E + el], __ldg(fac_exp + (size_t)tile * E + el), shift, ij);
+      if (__syncthreads_or(exact)) {
+        if (exact)
 #pragma unroll
-        for (int k = 0; k < N; k++) s_u[lz + k * N * RS] = __double_as_longlong(u[k]);
-      __syncthreads();
+          for (int k = 0; k < N; k++) s_u[lz + k * N * RS] = __double_as_longlong(u[k]);
+        __syncthreads();
+        fx_exact<N, E>(reinterpret_cast<double*>(s_u), reinterpret_cast<double*>(s_a), reinterpret_cast<double*>(s_b),
+                       s_mode, reinterpret_cast<double*>(s_fac), fac_e + (size_t)tile * E * 6 * Qp, R,
+                       slot_e + (size_t)tile * E * Qp);
+        __syncthreads();  // the factor stage and the work arrays are free
+      }
       if (t < E) s_mode[t] = 0;
-      if (exact) fx_exact_gradient<N, E>(su, sa, sb, ij);
-      __syncthreads();
-      if (exact) fx_exact_flux<N, E>(su, sa, sb, fac_e + e * 6 * Qp, ij);
-      __syncthreads();
     }
     if (t < E) s_max[s * E + t] = 0u;
     if (t < E) s_gmax[t] = 0u;
@@ -563,10 +548,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
       }
     }
     long long wz[N];
-    if (exact) {
-      fx_exact_divergence<N, E>(reinterpret_cast<double*>(s_u + el * W), reinterpret_cast<double*>(s_a + el * W),
-                                reinterpret_cast<double*>(s_b + el * W), R, slot_e + ((size_t)tile * E + el) * Qp, ij);
-    } else {
+    if (!exact) {
       long long r[N], y[N];
 #pragma unroll
       for (int a = 0; a < N; a++) r[a] = s_a[lx + a];
