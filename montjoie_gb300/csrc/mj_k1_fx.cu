@@ -82,6 +82,13 @@ double fx_beta(int n) {
   return 1.25 * (hi / lo) * (hi / lo);
 }
 
+__global__ void k_count_uneven(const int* __restrict__ fexp, int n_elt, int* __restrict__ count) {
+  int c = 0;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_elt; e += gridDim.x * blockDim.x) c += fexp[e] == kFxBad;
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+}
+
 }  // namespace
 
 // The matrix is one for the fixed-point forms: within 1% (of its largest
@@ -135,6 +142,18 @@ int k1_fixed_factors(mj_op* op, cudaStream_t s) {
       op->fac_e.as<double>(), op->fac_fx.as<int2>(), op->fac_exp.as<int>(), op->n_elt_pad, op->n, op->Qp, fx_beta(op->n));
   count_launch();
   MJ_CUDA(cudaGetLastError());
+  return MJ_OK;
+}
+
+int k1_fx_uneven(const mj_op* op, int* count, cudaStream_t s) {
+  DevBuf c;
+  MJ_CUDA(c.alloc(sizeof(int)));
+  MJ_CUDA(cudaMemsetAsync(c.ptr, 0, sizeof(int), s));
+  k_count_uneven<<<std::max(1, std::min((op->n_elt + 255) / 256, 4 * sm_count())), 256, 0, s>>>(
+      op->fac_exp.as<int>(), op->n_elt, c.as<int>());
+  count_launch();
+  MJ_CUDA(cudaMemcpyAsync(count, c.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MJ_CUDA(cudaStreamSynchronize(s));
   return MJ_OK;
 }
 
