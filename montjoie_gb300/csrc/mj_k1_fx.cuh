@@ -55,13 +55,13 @@
 // (16^3 Q4 58 and 61 us per product, 15x13x11 Q8 268 and 237).
 //
 // Measured (us per launch, FP64-pipe kernel at its best tile -> this kernel):
-// Q4 16^3 60 -> 20, 64^3 2300 -> 598; Q8 15x13x11-sized 359 -> 94, 32^3 3150
-// -> 763; Q6 40^3 2575 -> 590; Q1 64^3 94 -> 45.  What bounds it now (ncu, Q4
-// 40^3): the integer multiply pipe (about 60% busy) behind 16 to 20 warps per
-// SM, which shared memory (the factor stage) and registers allow; DRAM is at
-// half of its rate.  Without the lo*lo term it takes 15% less and errs up to
-// 3 times more than the FP64 kernel on steep fields; with the mirror symmetry
-// it takes 25% less than in the general form.
+// Q4 16^3 60 -> 16, 64^3 2300 -> 597; Q8 32^3 3150 -> 750; Q6 40^3 2575 -> 588;
+// Q1 64^3 94 -> 41.  What bounds it now (ncu, Q4 48^3): the integer multiply
+// pipe (60% busy) behind 16 to 20 warps per SM, which shared memory (the factor
+// stage) and registers allow; DRAM is at half of its rate.  Without the lo*lo
+// term it takes 15% less and errs up to 3 times more than the FP64 kernel on
+// steep fields; with the mirror symmetry it takes 25% less than in the general
+// form.
 //
 // Layout: E elements per CTA, E*n*n threads.  A thread owns a z-line in the
 // gather, the z-contractions, the factor products and the result, and an
@@ -223,6 +223,11 @@ __device__ __forceinline__ void fx_line(const long long (&r)[N], long long (&y)[
   }
 }
 
+// Least registers of a thread: at Q1 and Q2 shared memory admits so many CTAs
+// that the kernel would spill (us per launch at the registers of all the CTAs
+// -> these: Q1 100^3 172 -> 148, Q2 30^3 19.3 -> 17.9, 50^3 67.1 both).
+constexpr int fx_regs(int n, int E) { return n == 2 ? 80 : n == 3 ? (E <= 12 ? 96 : 72) : 48; }
+
 template <int N, int E>
 struct FxPlan {
   static constexpr int NN = N * N;
@@ -236,8 +241,10 @@ struct FxPlan {
   static constexpr size_t max_at = fac_bytes + 2 * nod_bytes + work_bytes;
   static constexpr size_t total = max_at + max_bytes + 3 * sizeof(uint64_t);
   static constexpr int threads = E * NN;
-  // CTAs per SM that shared memory admits (228 KB per SM, 1 KB of it per CTA): the register budget follows it
-  static constexpr int ctas = (int)(228 * 1024 / (total + 1024));
+  // CTAs per SM that shared memory (228 KB per SM, 1 KB of it per CTA) and fx_regs admit: the register budget
+  static constexpr int by_smem = (int)(228 * 1024 / (total + 1024));
+  static constexpr int by_regs = 65536 / ((threads + 31) / 32 * 32 * fx_regs(N, E));
+  static constexpr int ctas = by_smem < by_regs ? by_smem : by_regs;
   static_assert(fac_bytes % 16 == 0 && nod_bytes % 16 == 0, "bulk copies");
 };
 
