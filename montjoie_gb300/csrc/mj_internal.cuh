@@ -207,7 +207,6 @@ bool k1_fx_supports(int n, const double* g, bool* sym);
 int k1_set_gmat_fx(int n, const double* g, bool sym);
 int k1_set_gmat_fx_gen(int n, const double* g);
 int k1_fixed_factors(mj_op* op, cudaStream_t s);
-int k1_fx_uneven(const mj_op* op, int* count, cudaStream_t s);  // elements that the kernel computes in FP64 always
 int k1_prepare_fx(const mj_op* op, int E, int* ctas_per_sm);
 int k1_prepare_fx_gen(int n, int E, int* ctas_per_sm);
 void k1_launch_fx(mj_op* op, const void* x, cudaStream_t s);

@@ -12,8 +12,8 @@ namespace {
 // the contrast rule, the smallest with
 //   2^s_d beta x (the least, over the lines along d, of the line's largest B'_dd)
 //     >= the largest row sum;
-// kFxBad when a factor is not finite or B'_dd varies by more than 2 beta
-// between lines.  beta: 1.25 times what the quadrature weights alone make of
+// kFxBad when a factor is not finite, kFxUneven when B'_dd varies by more than
+// 2 beta between lines.  beta: 1.25 times what the quadrature weights alone make of
 // it.  One warp per element.
 __global__ void k_fixed_factors(const double* __restrict__ fac, int2* __restrict__ fx, int* __restrict__ fexp,
                                 int n_elt, int n, int Qp, double beta) {
@@ -59,14 +59,15 @@ __global__ void k_fixed_factors(const double* __restrict__ fac, int2* __restrict
   }
   if (lane) return;
   int out = kb * 4096;
+  bool even = true;
   if (m > 0.0)
     for (int d = 0; d < 3; d++) {
-      fin = fin && most[d] <= 2.0 * beta * least[d];
+      even = even && most[d] <= 2.0 * beta * least[d];
       int s = 0;
       while (s < 15 && scalbn(beta * least[d], s) < m) s++;
       out |= s << 4 * d;
     }
-  fexp[e] = fin ? out : kFxBad;
+  fexp[e] = !fin ? kFxBad : even ? out : kFxUneven;
 }
 
 // beta of k_fixed_factors: of the weights w 2^c, (largest / smallest)^2 over a
@@ -80,13 +81,6 @@ double fx_beta(int n) {
     hi = std::max(hi, v);
   }
   return 1.25 * (hi / lo) * (hi / lo);
-}
-
-__global__ void k_count_uneven(const int* __restrict__ fexp, int n_elt, int* __restrict__ count) {
-  int c = 0;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_elt; e += gridDim.x * blockDim.x) c += fexp[e] == kFxBad;
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
 
 }  // namespace
@@ -142,18 +136,6 @@ int k1_fixed_factors(mj_op* op, cudaStream_t s) {
       op->fac_e.as<double>(), op->fac_fx.as<int2>(), op->fac_exp.as<int>(), op->n_elt_pad, op->n, op->Qp, fx_beta(op->n));
   count_launch();
   MJ_CUDA(cudaGetLastError());
-  return MJ_OK;
-}
-
-int k1_fx_uneven(const mj_op* op, int* count, cudaStream_t s) {
-  DevBuf c;
-  MJ_CUDA(c.alloc(sizeof(int)));
-  MJ_CUDA(cudaMemsetAsync(c.ptr, 0, sizeof(int), s));
-  k_count_uneven<<<std::max(1, std::min((op->n_elt + 255) / 256, 4 * sm_count())), 256, 0, s>>>(
-      op->fac_exp.as<int>(), op->n_elt, c.as<int>());
-  count_launch();
-  MJ_CUDA(cudaMemcpyAsync(count, c.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
-  MJ_CUDA(cudaStreamSynchronize(s));
   return MJ_OK;
 }
 

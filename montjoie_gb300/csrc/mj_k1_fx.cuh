@@ -46,13 +46,17 @@
 // vertex lost up to 87 times in L2.
 // All other elements (spikes, the numerical tail ahead of a front; factors that
 // vary by more than 2.5 along an element, which is known when they are
-// converted) take the FP64 arithmetic of k_local_stiffness beside the others of
-// the tile (fx_exact), and so does an element out of range (a NaN or infinity in u or B, or scales whose result would leave
-// the normal range).  The choice hangs on the element alone, not on the tile it
+// converted) are computed beside the others of the tile: from Q3 up line by line
+// in integers, each line with a scale of its own (fx_lines), at Q1 and Q2 in the
+// FP64 arithmetic of k_local_stiffness (fx_exact).  An element out of range (a
+// NaN or infinity in u or B, or scales that may leave the normal range) always
+// takes the latter.  The choice hangs on the element alone, not on the tile it
 // is in.  Of smooth waves 2.5 elements long or more, fewer than 0.04% of the
-// elements take it.  One such element keeps its tile for 2 us at Q4 and 13 us
-// at Q8; a field of spikes everywhere takes about what the FP64-pipe kernel does
-// (16^3 Q4 58 and 61 us per product, 15x13x11 Q8 268 and 237).
+// elements are chosen.  One such element keeps its tile for 2 us at Q4 and 7 us
+// at Q8; spikes everywhere take 43 us per product at 16^3 Q4 (FP64-pipe kernel
+// 61, dense field 20), 186 at 15x13x11 Q8 (237, 65).  A run from rest has tails
+// in most elements until its waves fill the mesh: 64^3 Q4 1.95 ms per step in
+// its first hundreds of steps (FP64-pipe kernel 2.67, dense field 0.73).
 //
 // Measured (us per launch, FP64-pipe kernel at its best tile -> this kernel):
 // Q4 16^3 60 -> 16, 64^3 2300 -> 597; Q8 32^3 3150 -> 750; Q6 40^3 2575 -> 588;
@@ -90,8 +94,8 @@ namespace mj {
 namespace {
 
 // fac_exp of an element: the scale kb of its factors << 12 | s_z << 8 | s_y << 4 | s_x, s_d the factors' weight of
-// direction d against the largest, as a power of two downwards; kFxBad: not finite or too uneven.
-constexpr int kFxBad = INT_MIN;
+// direction d against the largest, as a power of two downwards; kFxBad: not finite; kFxUneven: too uneven for one scale.
+constexpr int kFxBad = INT_MIN, kFxUneven = INT_MIN + 1;
 
 // Coefficients of the line transforms of every order as (lo, hi, lo >> 17),
 // and their scales.  [n][0]: gradient, y_l = sum_a G[a][l] r_a; [n][1]:
@@ -99,7 +103,7 @@ constexpr int kFxBad = INT_MIN;
 // a < n/2, the middle coefficient at a = n/2 (n odd) and Mo_a at n-1-a;
 // general: the matrix.
 __constant__ int4 c_fx[kMaxNK + 1][2][kMaxNK * kMaxNK];
-__constant__ int c_fx_exp[kMaxNK + 1];  // sum of both scales
+__constant__ int2 c_fx_exp[kMaxNK + 1];  // both scales
 
 // Exponent of the similarity scaling at node i of n (see above).
 __host__ __device__ constexpr int fx_c(int n, int i) {
@@ -248,13 +252,13 @@ struct FxPlan {
   static_assert(fac_bytes % 16 == 0 && nod_bytes % 16 == 0, "bulk copies");
 };
 
-// The chosen elements of a tile (s_mode bit 1) in FP64, the arithmetic of
+// The elements of a tile out of range (s_mode 4) in FP64, the arithmetic of
 // k_local_stiffness<double> (compact), their u staged as doubles in s_u;
 // scratch: the factor stage, free.  The whole CTA works on their points,
 // whichever threads own them: the FP64 pipe takes 16 clocks per warp
 // instruction whatever its active lanes, so the points are dealt densely (by
 // their element's own threads, 25 or 81 in 2 or 4 warps, one element of a tile
-// took 7 us at Q4 and 22 at Q8).
+// took 7 us at Q4 and 22 at Q8, dealt so 2 and 13).
 template <int N, int E>
 __device__ __noinline__ void fx_exact(const double* s_u, double* s_a, double* s_b, const int* s_mode, double* scratch,
                                       const double* __restrict__ fac, double* __restrict__ R,
@@ -266,11 +270,12 @@ __device__ __noinline__ void fx_exact(const double* s_u, double* s_a, double* s_
   int* list = reinterpret_cast<int*>(scratch + E * W);
   int count = 0;
   for (int e = 0; e < E; e++)
-    if (s_mode[e] & 2) {
+    if (s_mode[e] & 4) {
       if (threadIdx.x == 0) list[count] = e;
       count++;
     }
   __syncthreads();
+  if (!count) return;
   for (int q = threadIdx.x; q < count * Q; q += P::threads) {
     const int el = list[q / Q], p = q % Q, k = p / NN, ij = p % NN, j = ij / N, i = ij % N;
     const double *rx = s_u + el * W + (k * N + j) * RS, *ry = s_u + el * W + k * N * RS + i;
@@ -305,18 +310,114 @@ __device__ __noinline__ void fx_exact(const double* s_u, double* s_a, double* s_
   }
 }
 
+// r 2^(59 - e + 1023 + c), truncated: e is at least r's biased exponent + c.
+__device__ __forceinline__ long long fx_from_double(double r, int c, int e) {
+  const int hi = __double2hiint(r);
+  const unsigned mh = (hi & 0xfffff) | ((hi & 0x7ff00000) ? 0x100000 : 0);
+  const unsigned long long m = ((unsigned long long)mh << 32 | (unsigned)__double2loint(r)) << (kFxBitsU - 52);
+  const long long v = (long long)(m >> min(e - c - max(hi >> 20 & 0x7ff, 1), 63));
+  return hi < 0 ? -v : v;
+}
+
+// y 2^s, rounded; below the normal range 0.
+__device__ __forceinline__ double fx_to_double(long long y, int s) {
+  const double d = __ll2double_rn(y);
+  const int hi = __double2hiint(d), t = (hi >> 20 & 0x7ff) + s;
+  if (y == 0 || t <= 0) return 0.0;
+  return t >= 2047 ? copysign(HUGE_VAL, d) : __hiloint2double(hi + s * (1 << 20), __double2loint(d));
+}
+
+// One line of doubles transformed in integers, scaled by its own largest value.
+template <int N, int KIND, bool SYM>
+__device__ __forceinline__ void fx_own_line(const double* in, double* out, int step) {
+  double r[N];
+  int e = 1;
+#pragma unroll
+  for (int a = 0; a < N; a++) {
+    r[a] = in[a * step];
+    e = max(e, max(__double2hiint(r[a]) >> 20 & 0x7ff, 1) + (KIND ? fx_c(N, a) : 0));
+  }
+  long long v[N], y[N];
+#pragma unroll
+  for (int a = 0; a < N; a++) v[a] = fx_from_double(r[a], KIND ? fx_c(N, a) : 0, e);
+  fx_line<N, KIND, SYM>(v, y);
+  const int s = 64 - (KIND ? kFxShY : kFxShG) - kFxBitsU + e - 1023 - (KIND ? c_fx_exp[N].y : c_fx_exp[N].x);
+#pragma unroll
+  for (int a = 0; a < N; a++) out[a * step] = fx_to_double(y[a], s - (KIND ? fx_c(N, a) : 0));
+}
+
+// Orders whose elements outside the contrast rule are transformed line by line:
+// 17 FP64 operations per point (the factor rows, six conversions, two sums)
+// where FP64 takes 6 n + 9.  At Q1 and Q2 that saves little or nothing, and
+// FP64's two or three terms round less than the stages do.
+template <int N>
+constexpr bool kFxLines = N >= 4;
+
+// The elements of a tile outside the contrast rule (s_mode 2 and not 4): their
+// line transforms in integers with a scale for every line, the gradients and
+// fluxes doubles in between, the factor rows in FP64.  Rounded once per stage
+// it needs no rule: over fields and factors that vary by up to 2^40 within an
+// element, entries are closer to the exact product than FP64's (largest error
+// over the absolute sum in units of 2^-53, 99% of 96,000 elements: Q1 2.7, FP64
+// 2.9; Q4 2.9 and 4.9; Q8 3.4 and 7.6), on the tails ahead of a front too (Q4
+// 2.0 and 3.3, Q8 2.1 and 4.8).  Arguments and work distribution as fx_exact.
+template <int N, int E, bool SYM>
+__device__ __noinline__ void fx_lines(const double* s_u, double* s_a, double* s_b, const int* s_mode, double* scratch,
+                                      const double* __restrict__ fac, double* __restrict__ R,
+                                      const int* __restrict__ slot) {
+  using P = FxPlan<N, E>;
+  constexpr int NN = P::NN, Q = N * NN, Qp = P::Qp, RS = P::RS, W = P::W;
+  int* list = reinterpret_cast<int*>(scratch + E * W);
+  int count = 0;
+  for (int e = 0; e < E; e++)
+    if ((s_mode[e] & 6) == 2) {
+      if (threadIdx.x == 0) list[count] = e;
+      count++;
+    }
+  __syncthreads();
+  if (!count) return;
+  for (int q = threadIdx.x; q < count * 3 * NN; q += P::threads) {
+    const int l = q % NN, d = q / NN % 3, el = list[q / (3 * NN)];
+    const int at = el * W + (d == 0 ? l * RS : d == 1 ? l / N * N * RS + l % N : l / N * RS + l % N);
+    fx_own_line<N, 0, SYM>(s_u + at, (d == 0 ? s_a : d == 1 ? s_b : scratch) + at,
+                           d == 0 ? 1 : d == 1 ? RS : N * RS);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < count * Q; q += P::threads) {
+    const int p = q % Q, el = list[q / Q], at = el * W + p / N * RS + p % N;
+    const double* f = fac + (size_t)el * 6 * Qp + p;
+    const double gx = s_a[at], gy = s_b[at], gz = scratch[at];
+    const double bxx = f[0], bxy = f[Qp], bxz = f[2 * Qp], byy = f[3 * Qp], byz = f[4 * Qp], bzz = f[5 * Qp];
+    s_a[at] = fac_dot(bxx, gx, bxy, gy, bxz, gz);
+    s_b[at] = fac_dot(bxy, gx, byy, gy, byz, gz);
+    scratch[at] = fac_dot(bxz, gx, byz, gy, bzz, gz);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < count * 3 * NN; q += P::threads) {
+    const int l = q % NN, d = q / NN % 3, el = list[q / (3 * NN)];
+    const int at = el * W + (d == 0 ? l * RS : d == 1 ? l / N * N * RS + l % N : l / N * RS + l % N);
+    double* v = (d == 0 ? s_a : d == 1 ? s_b : scratch) + at;
+    fx_own_line<N, 1, SYM>(v, v, d == 0 ? 1 : d == 1 ? RS : N * RS);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < count * Q; q += P::threads) {
+    const int p = q % Q, el = list[q / Q], at = el * W + p / N * RS + p % N;
+    R[slot[(size_t)el * Qp + p]] = s_a[at] + s_b[at] + scratch[at];
+  }
+}
+
 // The contrast rule for the elements of a tile with a thread that is bad (its
 // element is out of range) or whose z-line lies low; every thread of the CTA
 // calls it, u staged as integers in s_u; scratch: 2 N^2 words per element.
 // um: the element's largest |u| (high word), shift: the exponent of the rule.
-// True: this thread's element is computed in FP64.
+// s_mode: 2 not by one scale, 4 in FP64.  True: 2 for this thread's element.
 template <int N, int E>
 __device__ __noinline__ bool fx_choose(const long long* s_u, unsigned* scratch, int* s_mode, bool bad, bool low,
                                        unsigned um, int xp, int shift, int ij) {
   using P = FxPlan<N, E>;
   constexpr int NN = P::NN, RS = P::RS, W = P::W;
   const int el = threadIdx.x / NN, j = ij / N, i = ij - j * N;
-  if (bad || low) atomicOr(&s_mode[el], bad ? 2 : 1);
+  if (bad || low) atomicOr(&s_mode[el], bad ? 6 : xp == kFxUneven ? 2 : 1);
   __syncthreads();
   const bool look = s_mode[el] == 1;
   unsigned* line = scratch + el * 2 * NN;  // largest |u| of the x-lines, then of the y-lines
@@ -366,7 +467,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
   long long* s_b = s_a + E * W;
   unsigned* s_max = reinterpret_cast<unsigned*>(smem + P::max_at);  // [2][E]: largest |u| (high word) of the tile's and
   unsigned* s_gmax = s_max + 2 * E;                                 // the next tile's elements; [E]: largest |g|
-  int* s_mode = reinterpret_cast<int*>(s_max + 3 * E);  // [E]: bit 0: a z-line lies low, bit 1: the element in FP64
+  int* s_mode = reinterpret_cast<int*>(s_max + 3 * E);  // [E]: 1: a z-line lies low, 2: not by one scale, 4: in FP64
   // bar[0], bar[1]: the Nodle stages; bar[2]: the factor stage
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + P::max_at + P::max_bytes);
 
@@ -436,7 +537,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     line_max(0);
   }
   __syncthreads();
-  const int kg = c_fx_exp[N];
+  const int kg = c_fx_exp[N].x + c_fx_exp[N].y;
   for (int it = 0; tile < n_tiles; tile += g, ++it) {
     const int s = it & 1;
     // the element's scales: u 2^ku, B 2^kb, result 2^eo
@@ -444,10 +545,10 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     const int xp = __ldg(fac_exp + (size_t)tile * E + el);
     const int eu = (int)(um >> 20) - 1023;
     const int ku = um ? kFxBitsU - eu : 0;
-    const int eo = kFxYBias - ku - (xp == kFxBad ? 0 : xp >> 12) - kg;
+    const int eo = kFxYBias - ku - (xp <= kFxUneven ? 0 : xp >> 12) - kg;
     const bool bad = xp == kFxBad || (um && (eu > 1023 || eu < -900 || eo < -950 || eo > 1000));
     // this thread's z-line below the element's largest |u|, weighted, in units of 2^-20 of a power of two
-    const int below = (int)min(um - zm + ((xp >> 8 & 15u) << 20), 0x7fffffffu);
+    const int below = xp == kFxUneven ? INT_MAX : (int)min(um - zm + ((xp >> 8 & 15u) << 20), 0x7fffffffu);
     long long uz[N];
     {
       const double sc = __hiloint2double((1023 + (bad ? 0 : ku)) << 20, 0);
@@ -519,19 +620,31 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
         vz[k] = c.norm(sv);
       }
     }
-    bool exact = false;  // this thread's element in FP64
+    bool apart = false;  // this thread's element not by one scale
     const int shift = max(1, sv + fx_contrast(N));
     if (__syncthreads_or(bad || below > shift << 20)) {  // also: the factor stage is free, the fluxes are staged
-      exact = fx_choose<N, E>(s_u, reinterpret_cast<unsigned*>(s_fac), s_mode, bad, below > shift << 20,
+      apart = fx_choose<N, E>(s_u, reinterpret_cast<unsigned*>(s_fac), s_mode, bad, below > shift << 20,
                               s_max[s * E + el], __ldg(fac_exp + (size_t)tile * E + el), shift, ij);
-      if (__syncthreads_or(exact)) {
-        if (exact)
+      if (__syncthreads_or(apart)) {
+        if (apart) {
+          bool wide = !kFxLines<N> || eu > 900;  // gradients that may overflow, values that may leave the normal range
 #pragma unroll
-          for (int k = 0; k < N; k++) s_u[lz + k * N * RS] = __double_as_longlong(u[k]);
+          for (int k = 0; k < N; k++) {
+            s_u[lz + k * N * RS] = __double_as_longlong(u[k]);
+            wide |= u[k] != 0.0 && ((unsigned)__double2hiint(u[k]) & 0x7fffffffu) < ((1023u - 960u) << 20);
+          }
+          if (wide) atomicOr(&s_mode[el], 4);
+        }
         __syncthreads();
-        fx_exact<N, E>(reinterpret_cast<double*>(s_u), reinterpret_cast<double*>(s_a), reinterpret_cast<double*>(s_b),
-                       s_mode, reinterpret_cast<double*>(s_fac), fac_e + (size_t)tile * E * 6 * Qp, R,
-                       slot_e + (size_t)tile * E * Qp);
+        double *du = reinterpret_cast<double*>(s_u), *da = reinterpret_cast<double*>(s_a);
+        double *db = reinterpret_cast<double*>(s_b), *dz = reinterpret_cast<double*>(s_fac);
+        const double* f = fac_e + (size_t)tile * E * 6 * Qp;
+        const int* st = slot_e + (size_t)tile * E * Qp;
+        if constexpr (kFxLines<N>) {
+          fx_lines<N, E, SYM>(du, da, db, s_mode, dz, f, R, st);
+          __syncthreads();
+        }
+        fx_exact<N, E>(du, da, db, s_mode, dz, f, R, st);
         __syncthreads();  // the factor stage and the work arrays are free
       }
       if (t < E) s_mode[t] = 0;
@@ -555,7 +668,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
       }
     }
     long long wz[N];
-    if (!exact) {
+    if (!apart) {
       long long r[N], y[N];
 #pragma unroll
       for (int a = 0; a < N; a++) r[a] = s_a[lx + a];
@@ -580,7 +693,7 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
     }
     if (t == 0) fence_proxy_async();
     issue_nod(s, tile + 2 * g);
-    if (!exact) {
+    if (!apart) {
       const int ex = 1023 + (um ? eo - sv : 9) - fx_c(N, i) - fx_c(N, j);
       const int* st = slot_e + ((size_t)tile * E + el) * Qp + ij;
 #pragma unroll
@@ -650,7 +763,7 @@ int set_gmat_fx(int n, const double* g) {
     return kind ? std::ldexp(g[l * n + a], fx_c(n, l) - fx_c(n, a)) : g[a * n + l];
   };
   int4 v[2][kMaxNK * kMaxNK] = {};
-  int ksum = 0;
+  int k[2];
   for (int kind = 0; kind < 2; kind++) {
     double m = 0.0;  // largest sum of |coefficients|
     for (int l = 0; l < n; l++) {
@@ -659,7 +772,7 @@ int set_gmat_fx(int n, const double* g) {
       m = std::max(m, t);
     }
     const int kg = kFxBitsG - std::ilogb(m);
-    ksum += kg;
+    k[kind] = kg;
     auto M = [&](int a, int l) { return std::llrint(std::ldexp(coef(kind, a, l), kg)); };
     auto put = [&](int at, long long x) {
       const int lo = (int)(x & 0xffffffffLL);
@@ -681,7 +794,7 @@ int set_gmat_fx(int n, const double* g) {
   }
   const size_t per = sizeof(v);
   MJ_CUDA(cudaMemcpyToSymbol(c_fx, v, per, per * n));
-  MJ_CUDA(cudaMemcpyToSymbol(c_fx_exp, &ksum, sizeof(int), sizeof(int) * n));
+  MJ_CUDA(cudaMemcpyToSymbol(c_fx_exp, k, sizeof(int2), sizeof(int2) * n));
   MJ_CUDA(cudaMemcpyToSymbol(c_gmat64, g, sizeof(double) * n * n, sizeof(double) * kMaxNK * kMaxNK * n));
   return MJ_OK;
 }

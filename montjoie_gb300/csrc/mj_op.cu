@@ -446,20 +446,13 @@ int op_finish(mj_op* op) {
     // the factors a second time, as limbs (48 bytes per point); where they do not fit the FP64-pipe kernel runs from
     // fac_e alone.  Room for the vectors of a product or a run on this operator is left: 8 of n_dof doubles.
     DevBuf room;
-    bool use = false;
     if (room.alloc(8 * sizeof(double) * (size_t)op->n_dof) == cudaSuccess &&
         op->fac_fx.alloc(op->fac_e.bytes) == cudaSuccess &&
         op->fac_exp.alloc(sizeof(int) * op->n_elt_pad) == cudaSuccess) {
       rc = k1_set_gmat_fx(op->n, op->gradphi, op->fx_sym);
       if (!rc) rc = k1_fixed_factors(op, op->stream);
-      int uneven = 0;
-      if (!rc) rc = k1_fx_uneven(op, &uneven, op->stream);
       if (rc) return rc;
-      // elements with uneven factors go to FP64 in every product; with more than half of them the FP64-pipe kernel is
-      // the faster one (all of them: Q8 15x13x11 268 us per product against 237, 16^3 Q4 58 against 61)
-      use = 2 * uneven <= op->n_elt;
-    }
-    if (!use) {
+    } else {
       cudaGetLastError();  // out of memory is not an error here
       op->fac_fx.release();
       op->fac_exp.release();

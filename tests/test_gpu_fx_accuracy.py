@@ -130,21 +130,3 @@ def test_an_element_does_not_see_the_others_of_its_tile(order):
     u[1, 0, 0, 0] = np.inf
     assert np.array_equal(e.apply(u)[~other], y[~other])
     e.op.close()
-
-
-@pytest.mark.parametrize("order", [2, 4, 8])
-def test_uneven_factors_take_the_fp64_kernel(order):
-    """Factors that vary by 2^9 within every element: no element is one for fixed point."""
-    e = _Elements(order)
-    at = [q for q, (a, _) in enumerate(e.names) if a == "uneven"]
-    e.B, e.u, e.names = e.B[at], e.u[at], [e.names[q] for q in at]
-    Q = (order + 1) ** 3
-    b = np.zeros((len(at), Q, 6))
-    b[:, e.local] = e.B.reshape(len(at), Q, 6)
-    e.op.close()
-    e.op = FemMatrixFreeOperator(order, np.arange(len(at) * Q, dtype=np.int32).reshape(-1, Q), b, len(at) * Q, "fp64",
-                                 gradphi=e.G)
-    assert e.op.tuning()["layout"] == "compact"
-    y = e.apply(e.u)
-    _check(order, e, y, y)
-    e.op.close()
