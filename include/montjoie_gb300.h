@@ -42,7 +42,9 @@ extern "C" {
 #define MJ_ERR_NOMEM 6       /* device allocation failed */
 
 /* ---- precision of an operator ---------------------------------------- */
-#define MJ_FP64 0   /* plain form: FP64 everywhere */
+#define MJ_FP64 0   /* plain form: FP64 state, factors, masses and results; the
+                       element product in FP64 or in 64-bit integers where
+                       these are as accurate (mj_op_tuning, layout 5) */
 #define MJ_FP32 1   /* chosen form: FP32 state, factors and contractions,
                        FP64 setup, mass inversion and diagnostics */
 
@@ -142,7 +144,10 @@ int mj_op_info(const mj_op* op, int* order, int* n_elt, int* n_dof, int* precisi
  * plus the rank and no slot array is read; 4 compact with one factor stage:
  * the next tile's factors are copied during the current tile's divergence,
  * so a CTA holds one factor block instead of two; 5 fixed point, the kernel of
- * MJ_FP64 operators: two-limb integer products instead of the FP64 pipe; 6
+ * MJ_FP64 operators with a Gauss-Lobatto derivative matrix and room for a second
+ * copy of the factors: two-limb integer products instead of the FP64 pipe, by
+ * one scale per element where its field allows that, else by one per line, or
+ * in FP64 (orders 1 and 2, values out of range); 6
  * line owner, FP32 orders 7 and 8: a thread computes whole lines of the
  * gradient), grid; and the timings (ms per launch,
  * or a negative occupancy score on meshes too small to time) of the
