@@ -201,7 +201,7 @@ void k1_launch_w_f32(int n, int E, bool packed, int grid, const void* x, const i
 // Fixed-point kernel of FP64 operators (mj_k1_fx.cuh), the same tile sizes,
 // in two forms: the derivative matrix exactly antisymmetric under the mirror
 // (_sym, mj_k1_fx.cu) or any (_gen, mj_k1_fxg.cu).  supports: the matrix is
-// within its range; fixed_factors: fac_e into fac_fx / fac_exp (after every
+// a Gauss-Lobatto one to 1%; fixed_factors: fac_e into fac_fx / fac_exp (after every
 // change of fac_e).
 bool k1_fx_supports(int n, const double* g, bool* sym);
 int k1_set_gmat_fx(int n, const double* g, bool sym);

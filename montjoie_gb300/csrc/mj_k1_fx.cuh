@@ -27,12 +27,12 @@
 //   y = 3 sums G' v <= 2^62.6  h < 2^60, m < 2^62.8
 // so no accumulator overflows for any input in range.
 //
-// Which elements.  With one scale per element a value 2^-k below the largest
+// Which elements.  With its one scale per element a value 2^-k below the largest
 // keeps 60 - k bits where FP64 keeps 53, and the matrix spends several of the
 // 7 to spare (its entries span 2^4.7 at Q4, 2^7 at Q8).  FP64's own error at a
 // point hangs on the largest |u| on the three lines through it, each weighted
 // by its direction's factor; here the fluxes' unit, which follows the
-// element's largest gradient, decides.  So an element is computed here only if
+// element's largest gradient, decides.  So an element takes one scale only if
 // that maximum is nowhere more than 2^max(1, sv + X) below the element's
 // largest |u|: sv, the bits by which the gradients are below their bound, is
 // high (5 to 13) for smooth fields and 1 to 3 for spikes; X = fx_contrast.

@@ -162,7 +162,7 @@ int autotune_k1(mj_op* op) {
   const bool time_it = points >= (op->fac_fx.ptr ? 100000 : 2000000);
   // layouts: 0 compact, 1 vector lines, 2 one element per warp, 3 the same
   // with packed connectivity, 4 compact with one factor stage (2-4: FP32), 5 fixed point (FP64: always where the
-  // derivative matrix is in its range; the FP64-pipe kernel took 2.1 (Q1) to 4.4 (Q6) times as long on large meshes,
+  // operator holds the limbs; on dense fields the FP64-pipe kernel took 2.1 (Q1) to 4.4 (Q6) times as long on large meshes,
   // 1.4 to 3 times on meshes of 5,000 to 275,000 dofs, and as long on 125 dofs)
   std::vector<int> layouts = {op->fac_fx.ptr ? 5 : 0};
   if (op->precision == MJ_FP32) {
