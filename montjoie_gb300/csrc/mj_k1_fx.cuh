@@ -54,9 +54,11 @@
 // is in.  Of smooth waves 2.5 elements long or more, fewer than 0.04% of the
 // elements are chosen.  One such element keeps its tile for 2 us at Q4 and 7 us
 // at Q8; spikes everywhere take 43 us per product at 16^3 Q4 (FP64-pipe kernel
-// 61, dense field 20), 186 at 15x13x11 Q8 (237, 65).  A run from rest has tails
-// in most elements until its waves fill the mesh: 64^3 Q4 1.95 ms per step in
-// its first hundreds of steps (FP64-pipe kernel 2.67, dense field 0.73).
+// 61, dense field 20), 171 at 15x13x11 Q8 (237, 65).  A run from rest has tails
+// in most elements until its waves fill the mesh; in its first hundreds of steps
+// a step takes (us; FP64-pipe kernel, dense field) Q4 40^3 460 (610, 178), Q8
+// 15^3 264 (366, 102), Q6 24^3 370 (504, 154), Q3 45^3 313 (369, 126), Q2 60^3
+// 383 (319, 133), Q1 100^3 374 (354, 170).
 //
 // Measured (us per launch, FP64-pipe kernel at its best tile -> this kernel):
 // Q4 16^3 60 -> 16, 64^3 2300 -> 597; Q8 32^3 3150 -> 750; Q6 40^3 2575 -> 588;
@@ -325,6 +327,11 @@ __device__ __forceinline__ double fx_to_double(long long y, int s) {
   const int hi = __double2hiint(d), t = (hi >> 20 & 0x7ff) + s;
   if (y == 0 || t <= 0) return 0.0;
   return t >= 2047 ? copysign(HUGE_VAL, d) : __hiloint2double(hi + s * (1 << 20), __double2loint(d));
+}
+
+// A range of global memory (16-byte aligned, a multiple of 16 bytes) into L2.
+__device__ __forceinline__ void fx_prefetch(const void* p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
 // One line of doubles transformed in integers, scaled by its own largest value.
@@ -627,6 +634,10 @@ __global__ void __launch_bounds__(E* N* N, FxPlan<N, E>::ctas)
                               s_max[s * E + el], __ldg(fac_exp + (size_t)tile * E + el), shift, ij);
       if (__syncthreads_or(apart)) {
         if (apart) {
+          if (ij == 0) {  // read by plain loads in a moment (40^3 Q4 from rest 485 -> 460 us per step, Q8 15^3 290 -> 264)
+            fx_prefetch(fac_e + ((size_t)tile * E + el) * 6 * Qp, 6 * Qp * sizeof(double));
+            fx_prefetch(slot_e + ((size_t)tile * E + el) * Qp, Qp * sizeof(int));
+          }
           bool wide = !kFxLines<N> || eu > 900;  // gradients that may overflow, values that may leave the normal range
 #pragma unroll
           for (int k = 0; k < N; k++) {
